@@ -4,8 +4,8 @@ A batch of ridge-regularised LPs
 
     min c^T x + ridge ||x||^2   s.t.  rmin <= A x <= rmax,  cl <= x <= cu
 
-is run for K PDHG iterations with fixed steps (one CTA per instance, CUDA
-kernels behind ``igaos_pdhg_unrolled_forward``); the backward is the exact
+is run for K PDHG iterations with fixed steps (a thread-block cluster per
+instance, CUDA kernels behind ``igaos_pdhg_unrolled_forward``); the backward is the exact
 reverse mode of those K iterations (``igaos_pdhg_unrolled_backward``), with
 checkpoints every ``checkpoint`` iterations and replay in between. Outputs
 are x_K, y_K and obj = c^T x_K + ridge ||x_K||^2 per instance; gradients flow

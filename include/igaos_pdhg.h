@@ -464,7 +464,7 @@ int igaos_pdhg_evaluate_noalloc(int m, int n, const int* ap, const int* ai,
  * value arrays hold float (precision IGAOS_PDHG_FP32) or double
  * (IGAOS_PDHG_FP64). Work is enqueued on `stream`; nothing is allocated. */
 typedef struct igaos_pdhg_unrolled_layout {
-    int count;          /* instances (one CTA each) */
+    int count;          /* instances (one thread-block cluster each) */
     int precision;      /* IGAOS_PDHG_FP32 or IGAOS_PDHG_FP64 */
     int iterations;     /* K >= 1 */
     int checkpoint;     /* checkpoint interval >= 1 */
