@@ -40,15 +40,41 @@
 namespace igx {
 namespace {
 
-// threads per instance (one CTA): big instances are latency-bound per
-// iteration, so the whole CTA's width goes to one LP
+// Threads of a CTA, by class (below). The first kBT at most are workers: one
+// owns columns (rows) t, t + kBT, ...; with fewer threads than kBT every column
+// has its own, so the per-thread sums of the step's dot products, and their
+// merge over warps, do not depend on the class. Threads past kBT take part in
+// the products alone, and the last warp takes the step decisions.
 constexpr int kBT = 512;
 constexpr int kBW = kBT / 32;
+constexpr unsigned kFull = 0xffffffffu;
 
 struct BatchDesc {
-    int m, n, nnz, pad;
+    int m, n, nnz, mode;  // mode: where the instance is held (kHeld...)
+    long long pad_c, pad_r;  // staged entries of the sorted slices, columns and rows
     long long ap_off, cp_off, nz_off, row_off, col_off;
+    long long base_off;  // slice bases (in units of 32 entries): columns'
+                         // (slices + 1), then rows'
+    long long out_off;   // kHeldOut: staged entries in global memory
 };
+
+// kHeldOut: everything in global memory. kHeldMatrix: the matrix and the
+// gathered vectors in shared memory. kHeldAll: the iterates and the residual
+// data too.
+enum { kHeldOut = 0, kHeldMatrix = 1, kHeldAll = 2 };
+
+__host__ __device__ inline int slices_of(int rows) { return (rows + 31) / 32; }
+// staged values and 16-bit indices, x_bar, both slots of y, A~ x_bar, the
+// slices' bases and the rows' numbers
+__host__ __device__ inline size_t matrix_bytes(const BatchDesc& d) {
+    const size_t pad = (size_t)d.pad_c + d.pad_r;
+    return ((4 * pad + 4 * (size_t)d.n + 12 * (size_t)d.m +
+             4 * (size_t)(slices_of(d.n) + slices_of(d.m) + 2) + 2 * pad +
+             2 * ((size_t)d.n + d.m)) + 15) & ~(size_t)15;
+}
+__host__ __device__ inline size_t state_bytes(const BatchDesc& d) {
+    return 4 * (9 * (size_t)d.n + 7 * (size_t)d.m);
+}
 
 struct BatchOut {
     int status, handed;  // handed: stopped at handoff_at for the FP64 finish
@@ -66,8 +92,8 @@ __device__ __forceinline__ long long global_ns() {
 constexpr int kFacTab = 1 << 16;  // tabulated 1 - k^-0.3, 1 + k^-0.6
 
 struct BatchArgs {
-    int count;
-    const int* order;
+    int count;           // instances of this launch's class
+    const int* order;    // their indices, largest first
     unsigned int* queue;
     const BatchDesc* desc;
     const int *ap, *ai;
@@ -77,9 +103,14 @@ struct BatchArgs {
     int *cp, *ci, *cnt;
     float *cax, *sax, *scax;
     double* cax64;       // original values in CSC order, FP64
+    const int *order_c, *order_r;  // columns and rows by decreasing length
+    const int* bases;              // first staged entry of each slice of 32 of them
+    float* out_val;                // staged entries of kHeldOut instances
+    int* out_idx;
     float *dr, *dc, *sc, *scl, *scu, *srmin, *srmax, *yh32;
-    float *x[2], *xa[2], *xbar, *vt;
+    float *x[2], *xa[2], *xbar, *vt, *g[2], *ab;
     float *y[2], *ya[2], *axc[2], *mt;
+    double *rdr, *rdc;
     double *xh, *yh, *pesx, *pesy, *axh, *atyh;
     const float* fac;
     double tol;
@@ -93,56 +124,86 @@ struct BatchArgs {
     BatchOut* out;
 };
 
-struct BatchShared {
-    Acc<float> acc[kBW * 4];
-    double dred[kBW * 8];
-    float fmax_[kBW * 8];
-    int part[kBT];
-    int inst;
+// The step being attempted, written by the decision warp.
+struct BatchStep {
     float tau, sigma, w;
-    int parity, accept;
-    long long kdone;
+    int parity;   // slot of the accepted iterates
+    int check, done, restart, use_avg;
 };
 
-// ---- block-level helpers (every thread of the CTA calls them) -----------
-template <int NV>
-__device__ void bmerge(BatchShared& sh, Acc<float> (&v)[NV]) {
-    block_merge<float, NV, kBW>(v, sh.acc);
+struct BMetrics {
+    double pinf, dinf, gap, op, od, prow, err;
+    bool finite;
+};
+
+// Controller state used at checks only (the decision warp's first lane).
+struct BatchRare {
+    double epoch_kkt, prev_cand;
+    long long epoch_start, restarts;
+    int status, asked, handed, have_pe;
+    BMetrics last, now[2];
+};
+
+struct BatchShared {
+    BatchRare rare;
+    Acc<float> acc[kBW * 3];
+    double dred[kBW * 8];
+    int part[kBT];
+    int inst;
+    BatchStep step;
+};
+
+// The CTA's dynamic shared memory: BatchShared, then what the instance holds.
+// Functions name it themselves, rather than take pointers into it: loads and
+// stores then are shared-memory ones, and nothing of the hot loops' state has
+// to be in memory for the calls they make now and then.
+constexpr size_t kSharedHead = (sizeof(BatchShared) + 15) & ~(size_t)15;
+__device__ __forceinline__ unsigned char* b_mem() {
+    extern __shared__ __align__(16) unsigned char b_smem[];
+    return b_smem;
+}
+__device__ __forceinline__ BatchShared& b_shared() {
+    return *reinterpret_cast<BatchShared*>(b_mem());
 }
 
+// ---- block-level helpers (every thread of the CTA calls them; `workers` is
+// the number of worker threads; the others take no part) ------------------
 template <int NV>
-__device__ void bmaxf(BatchShared& sh, float (&v)[NV]) {
+__device__ void bmerge(Acc<float> (&v)[NV], int workers) {
+    BatchShared& sh = b_shared();
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < NV; ++q)
-        for (int o = 16; o > 0; o >>= 1) v[q] = fmaxf(v[q], __shfl_xor_sync(0xffffffffu, v[q], o));
+        for (int o = 16; o > 0; o >>= 1) v[q].shfl_xor(kFull, o, 32);
     __syncthreads();
-    if (lane == 0)
+    if (lane == 0 && (int)threadIdx.x < workers)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) sh.fmax_[wp * NV + q] = v[q];
+        for (int q = 0; q < NV; ++q) sh.acc[wp * NV + q] = v[q];
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) {
-            float s = sh.fmax_[q];
-            for (int k = 1; k < kBW; ++k) s = fmaxf(s, sh.fmax_[k * NV + q]);
+            Acc<float> s = sh.acc[q];
+            for (int k = 1; k < workers / 32; ++k) s.merge(sh.acc[k * NV + q]);
             v[q] = s;
         }
+    }
     __syncthreads();
 }
 
 // exclusive block scan of cnt[0..len) into out[0..len], out[len] = total
-__device__ void bscan(BatchShared& sh, const int* cnt, int* out, int len) {
+__device__ void bscan(const int* cnt, int* out, int len, int workers) {
+    BatchShared& sh = b_shared();
     const int t = threadIdx.x;
-    const int per = (len + kBT - 1) / kBT;
+    const int per = (len + workers - 1) / workers;
     const int b = min(len, t * per), e = min(len, b + per);
     int s = 0;
     for (int j = b; j < e; ++j) s += cnt[j];
-    sh.part[t] = s;
+    if (t < workers) sh.part[t] = s;
     __syncthreads();
     if (t == 0) {
         int run = 0;
-        for (int k = 0; k < kBT; ++k) {
+        for (int k = 0; k < workers; ++k) {
             const int v = sh.part[k];
             sh.part[k] = run;
             run += v;
@@ -150,7 +211,7 @@ __device__ void bscan(BatchShared& sh, const int* cnt, int* out, int len) {
         out[len] = run;
     }
     __syncthreads();
-    int run = sh.part[t];
+    int run = t < workers ? sh.part[t] : 0;
     for (int j = b; j < e; ++j) {
         out[j] = run;
         run += cnt[j];
@@ -167,9 +228,8 @@ struct Inst {
     int *cp, *ci, *cnt;
     float *cax, *sax, *scax;
     double* cax64;
-    float *dr, *dc, *sc, *scl, *scu, *srmin, *srmax, *yh32;
-    float *x[2], *xa[2], *xbar, *vt;
-    float *y[2], *ya[2], *axc[2], *mt;
+    float *dr, *dc, *vt, *mt;
+    double *rdr, *rdc;   // 1 / dr, 1 / dc
     double *xh, *yh, *pesx, *pesy, *axh, *atyh;
 };
 
@@ -193,22 +253,10 @@ __device__ Inst make_inst(const BatchArgs& a, const BatchDesc& d) {
     I.cax64 = a.cax64 + d.nz_off;
     I.sax = a.sax + d.nz_off;
     I.scax = a.scax + d.nz_off;
+    I.rdr = a.rdr + d.row_off;
+    I.rdc = a.rdc + d.col_off;
     I.dr = a.dr + d.row_off;
-    I.srmin = a.srmin + d.row_off;
-    I.srmax = a.srmax + d.row_off;
-    I.yh32 = a.yh32 + d.row_off;
     I.dc = a.dc + d.col_off;
-    I.sc = a.sc + d.col_off;
-    I.scl = a.scl + d.col_off;
-    I.scu = a.scu + d.col_off;
-    for (int s = 0; s < 2; ++s) {
-        I.x[s] = a.x[s] + d.col_off;
-        I.xa[s] = a.xa[s] + d.col_off;
-        I.y[s] = a.y[s] + d.row_off;
-        I.ya[s] = a.ya[s] + d.row_off;
-        I.axc[s] = a.axc[s] + d.row_off;
-    }
-    I.xbar = a.xbar + d.col_off;
     I.vt = a.vt + d.col_off;
     I.mt = a.mt + d.row_off;
     I.xh = a.xh + d.col_off;
@@ -218,6 +266,160 @@ __device__ Inst make_inst(const BatchArgs& a, const BatchDesc& d) {
     I.pesy = a.pesy + d.row_off;
     I.axh = a.axh + d.row_off;
     return I;
+}
+
+// The iterates and residual data the iteration works on, and the scaled
+// matrix by slices of 32 columns (rows) of like length: the k-th entries of a
+// slice's rows lie next to each other, padded with (0, entry 0) to its longest
+// row, so a warp reads runs of words and no lane tests a length (a pad adds
+// 0 x, nothing, to a sum; an infinite x ends the LP at its step's dot
+// products). Every row's sum keeps the order of its entries.
+template <int MODE>
+struct Held {
+    using Idx = typename std::conditional<MODE == kHeldOut, int, uint16_t>::type;
+    int m, n;
+    const int *cbase, *rbase;
+    const uint16_t *cid, *rid;     // row numbers by position, or
+    const int *cid32, *rid32;      // (kHeldOut) these
+    const float *cv, *rv;
+    const Idx *ci, *ri;
+    float *xbar, *ab, *ys;  // ys: both slots of y
+    // the vectors below follow each other in shared memory (kHeldAll) and
+    // start at cols and rows; else they are the instance's in global memory
+    float *cols, *rows;
+    const BatchArgs* a;
+    long long c0, r0;
+    __device__ __forceinline__ float* col(int k, float* out) const {
+        if constexpr (MODE == kHeldAll) return cols + k * n;
+        else return out + c0;
+    }
+    __device__ __forceinline__ float* row(int k, float* out) const {
+        if constexpr (MODE == kHeldAll) return rows + k * m;
+        else return out + r0;
+    }
+    __device__ __forceinline__ float* sc() const { return col(0, a->sc); }
+    __device__ __forceinline__ float* scl() const { return col(1, a->scl); }
+    __device__ __forceinline__ float* scu() const { return col(2, a->scu); }
+    __device__ __forceinline__ float* x(int p) const { return col(3 + p, p ? a->x[1] : a->x[0]); }
+    __device__ __forceinline__ float* xa(int p) const { return col(5 + p, p ? a->xa[1] : a->xa[0]); }
+    __device__ __forceinline__ float* g(int p) const { return col(7 + p, p ? a->g[1] : a->g[0]); }
+    __device__ __forceinline__ float* srmin() const { return row(0, a->srmin); }
+    __device__ __forceinline__ float* srmax() const { return row(1, a->srmax); }
+    __device__ __forceinline__ float* yh32() const { return row(2, a->yh32); }
+    __device__ __forceinline__ float* ya(int p) const { return row(3 + p, p ? a->ya[1] : a->ya[0]); }
+    __device__ __forceinline__ float* axc(int p) const { return row(5 + p, p ? a->axc[1] : a->axc[0]); }
+    __device__ __forceinline__ float* y(int p) const {
+        if constexpr (MODE == kHeldOut) return (p ? a->y[1] : a->y[0]) + r0;
+        else return ys + p * m;
+    }
+};
+
+template <int MODE>
+__device__ __forceinline__ Held<MODE> make_work(const BatchArgs& a, const BatchDesc& d) {
+    unsigned char* smem = b_mem() + kSharedHead;
+    Held<MODE> W;
+    const int m = d.m, n = d.n;
+    W.m = m;
+    W.n = n;
+    W.a = &a;
+    W.c0 = d.col_off;
+    W.r0 = d.row_off;
+    W.cols = W.rows = W.ys = nullptr;
+    const int sc = slices_of(n), sr = slices_of(m);
+    if constexpr (MODE == kHeldOut) {
+        W.cbase = a.bases + d.base_off;
+        W.rbase = W.cbase + sc + 1;
+        W.cid = W.rid = nullptr;
+        W.cid32 = a.order_c + d.col_off;
+        W.rid32 = a.order_r + d.row_off;
+        W.cv = a.out_val + d.out_off;
+        W.rv = W.cv + d.pad_c;
+        W.ci = a.out_idx + d.out_off;
+        W.ri = W.ci + d.pad_c;
+        W.xbar = a.xbar + d.col_off;
+        W.ab = a.ab + d.row_off;
+    } else {
+        float* v = reinterpret_cast<float*>(smem);
+        W.cv = v;
+        W.rv = v + d.pad_c;
+        W.xbar = v + d.pad_c + d.pad_r;
+        W.ys = W.xbar + n;
+        W.ab = W.ys + 2 * m;
+        int* p = reinterpret_cast<int*>(W.ab + m);
+        W.cbase = p;
+        W.rbase = p + sc + 1;
+        uint16_t* i = reinterpret_cast<uint16_t*>(p + sc + sr + 2);
+        W.ci = i;
+        W.ri = i + d.pad_c;
+        W.cid = i + d.pad_c + d.pad_r;
+        W.rid = W.cid + n;
+        W.cid32 = W.rid32 = nullptr;
+        W.cols = reinterpret_cast<float*>(smem + matrix_bytes(d));
+        W.rows = W.cols + 9 * (size_t)n;
+    }
+    return W;
+}
+
+// Fills the staged matrix (by the worker warps, a slice at a time).
+template <int MODE>
+__device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, int workers) {
+    const BatchDesc d = *dp;
+    const Inst I = make_inst(a, d);
+    const Held<MODE> W = make_work<MODE>(a, d);
+    using Idx = typename Held<MODE>::Idx;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5, nw = workers >> 5;
+    const int sc = slices_of(I.n), sr = slices_of(I.m);
+    const int* order[2] = {a.order_c + d.col_off, a.order_r + d.row_off};
+    const int* bases = a.bases + d.base_off;
+    if constexpr (MODE != kHeldOut) {
+        for (int s = t; s < sc + sr + 2; s += blockDim.x) const_cast<int*>(W.cbase)[s] = bases[s];
+        for (int j = t; j < I.n; j += blockDim.x)
+            const_cast<uint16_t*>(W.cid)[j] = (uint16_t)order[0][j];
+        for (int i = t; i < I.m; i += blockDim.x)
+            const_cast<uint16_t*>(W.rid)[i] = (uint16_t)order[1][i];
+    }
+    for (int w = wp; w < sc + sr && wp < nw; w += nw) {
+        const bool r = w >= sc;
+        const int s = r ? w - sc : w, q = 32 * s + lane;
+        const int* ptr = r ? I.ap : I.cp;
+        const int* idx = r ? I.ai : I.ci;
+        const float* val = r ? I.sax : I.scax;
+        const int b0 = bases[r ? sc + 1 + s : s], b1 = bases[r ? sc + 2 + s : s + 1];
+        float* v = const_cast<float*>(r ? W.rv : W.cv) + 32LL * b0 + lane;
+        Idx* ix = const_cast<Idx*>(r ? W.ri : W.ci) + 32LL * b0 + lane;
+        int p = 0, e = 0;
+        if (q < (r ? I.m : I.n)) {
+            const int row = order[r ? 1 : 0][q];
+            p = ptr[row];
+            e = ptr[row + 1];
+        }
+        for (int k = b0; k < b1; ++k, ++p, v += 32, ix += 32) {
+            *v = p < e ? val[p] : 0.f;
+            *ix = (Idx)(p < e ? idx[p] : 0);
+        }
+    }
+    __syncthreads();
+}
+
+// The products of the lane's staged row (slice entries 32 b0 .. 32 b1) with
+// v, compensated FP32, in the order of the entries.
+template <class Idx>
+__device__ __forceinline__ Acc<float> padded_dot(const Idx* idx, const float* val,
+                                                 const float* __restrict__ v, int b0, int b1) {
+    using At = typename std::conditional<std::is_same<Idx, int>::value, long long, int>::type;
+    At at = 32 * (At)b0 + (threadIdx.x & 31);
+    int left = b1 - b0;
+    Acc<float> acc;
+#pragma unroll 1
+    for (; left >= 2; left -= 2, at += 64) {
+        const float a0 = val[at], a1 = val[at + 32];
+        const int j0 = idx[at], j1 = idx[at + 32];
+        const float x0 = v[j0], x1 = v[j1];
+        acc.add(a0, x0);
+        acc.add(a1, x1);
+    }
+    if (left) acc.add(val[at], v[idx[at]]);
+    return acc;
 }
 
 // one row of a CSR times v (thread per row, compensated FP32)
@@ -230,18 +432,22 @@ __device__ __forceinline__ Acc<float> row_dot(const int* ptr, const int* idx, co
 
 // Full FP64 column value of delta dx (scaled units), with the at-bound rule:
 // a delta on its FP32 shifted bound is exactly at the bound.
-__device__ __forceinline__ double full_x(const Inst& I, int j, float dx) {
-    if (dx == I.scl[j]) return I.cl[j] / (double)I.dc[j];
-    if (dx == I.scu[j]) return I.cu[j] / (double)I.dc[j];
+template <int MODE>
+__device__ __forceinline__ double full_x(const Inst& I, const Held<MODE>& W, int j, float dx) {
+    if (dx == W.scl()[j]) return I.cl[j] / (double)I.dc[j];
+    if (dx == W.scu()[j]) return I.cu[j] / (double)I.dc[j];
     return I.xh[j] + (double)dx;
 }
 
 // Residual data of the LP seen from the anchor (xh, yh), FP64 -> FP32:
 // sc = c~ + A~^T yh, [scl, scu] = box~ - xh, [srmin, srmax] = rows~ - A~ xh,
 // with A~_ij = a_ij dc_j / dr_i formed in FP64 from the FP64 values.
-__device__ void anchor_data(Inst& I) {
-    const int t = threadIdx.x;
-    for (int i = t; i < I.m; i += kBT) {
+template <int MODE>
+__device__ __noinline__ void anchor_data(const BatchArgs& a, const BatchDesc* d, int t,
+                                         int workers) {
+    const Inst I = make_inst(a, *d);
+    const Held<MODE> W = make_work<MODE>(a, *d);
+    for (int i = t; i < I.m; i += workers) {
         const double dri = I.dr[i];
         double s = 0.0;
         for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) {
@@ -249,11 +455,11 @@ __device__ void anchor_data(Inst& I) {
             s = fma(I.axd[p] * (double)I.dc[j] / dri, I.xh[j], s);
         }
         I.axh[i] = s;
-        I.srmin[i] = (float)(I.rmin[i] / dri - s);
-        I.srmax[i] = (float)(I.rmax[i] / dri - s);
-        I.yh32[i] = (float)I.yh[i];
+        W.srmin()[i] = (float)(I.rmin[i] / dri - s);
+        W.srmax()[i] = (float)(I.rmax[i] / dri - s);
+        W.yh32()[i] = (float)I.yh[i];
     }
-    for (int j = t; j < I.n; j += kBT) {
+    for (int j = t; j < I.n; j += workers) {
         const double dcj = I.dc[j];
         double s = 0.0;
         for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) {
@@ -261,33 +467,36 @@ __device__ void anchor_data(Inst& I) {
             s = fma(I.cax64[p] * dcj / (double)I.dr[i], I.yh[i], s);
         }
         I.atyh[j] = s;
-        I.sc[j] = (float)(I.c[j] * dcj + s);
-        I.scl[j] = (float)(I.cl[j] / dcj - I.xh[j]);
-        I.scu[j] = (float)(I.cu[j] / dcj - I.xh[j]);
+        W.sc()[j] = (float)(I.c[j] * dcj + s);
+        W.scl()[j] = (float)(I.cl[j] / dcj - I.xh[j]);
+        W.scu()[j] = (float)(I.cu[j] / dcj - I.xh[j]);
     }
     __syncthreads();
 }
 
 // ---- setup: CSC, Ruiz, scaled data, power iteration ----------------------
-__device__ void setup(BatchShared& sh, Inst& I, float& eta0, float& omega0) {
-    const int t = threadIdx.x, m = I.m, n = I.n;
+// (t: this thread among the workers, beyond every size for the decision warp)
+__device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t, int workers,
+                                   float& eta0, float& omega0) {
+    const Inst I = make_inst(a, *d);
+    const int m = I.m, n = I.n;
     // CSC by counting sort; each column's entries ordered by row afterwards
-    for (int j = t; j < n; j += kBT) I.cnt[j] = 0;
+    for (int j = t; j < n; j += workers) I.cnt[j] = 0;
     __syncthreads();
-    for (int i = t; i < m; i += kBT)
+    for (int i = t; i < m; i += workers)
         for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) atomicAdd(&I.cnt[I.ai[p]], 1);
     __syncthreads();
-    bscan(sh, I.cnt, I.cp, n);
-    for (int j = t; j < n; j += kBT) I.cnt[j] = I.cp[j];
+    bscan(I.cnt, I.cp, n, workers);
+    for (int j = t; j < n; j += workers) I.cnt[j] = I.cp[j];
     __syncthreads();
-    for (int i = t; i < m; i += kBT)
+    for (int i = t; i < m; i += workers)
         for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) {
             const int q = atomicAdd(&I.cnt[I.ai[p]], 1);
             I.ci[q] = i;
             I.cax64[q] = I.axd[p];
         }
     __syncthreads();
-    for (int j = t; j < n; j += kBT) {  // insertion sort by row index
+    for (int j = t; j < n; j += workers) {  // insertion sort by row index
         const int b = I.cp[j], e = I.cp[j + 1];
         for (int q = b + 1; q < e; ++q) {
             const int r = I.ci[q];
@@ -304,18 +513,18 @@ __device__ void setup(BatchShared& sh, Inst& I, float& eta0, float& omega0) {
         for (int q = b; q < e; ++q) I.cax[q] = (float)I.cax64[q];
     }
     // Ruiz, 10 sweeps (FP32 factors)
-    for (int i = t; i < m; i += kBT) I.dr[i] = 1.f;
-    for (int j = t; j < n; j += kBT) I.dc[j] = 1.f;
+    for (int i = t; i < m; i += workers) I.dr[i] = 1.f;
+    for (int j = t; j < n; j += workers) I.dc[j] = 1.f;
     __syncthreads();
     for (int sweep = 0; sweep < 10; ++sweep) {
-        for (int i = t; i < m; i += kBT) {
+        for (int i = t; i < m; i += workers) {
             float mx = 0.f;
             for (int p = I.ap[i]; p < I.ap[i + 1]; ++p)
                 mx = fmaxf(mx, fabsf(I.ax[p]) * I.dc[I.ai[p]] / I.dr[i]);
             if (mx > 0.f && isfinite(mx)) I.dr[i] *= sqrtf(mx);
         }
         __syncthreads();
-        for (int j = t; j < n; j += kBT) {
+        for (int j = t; j < n; j += workers) {
             float mx = 0.f;
             for (int p = I.cp[j]; p < I.cp[j + 1]; ++p)
                 mx = fmaxf(mx, fabsf(I.cax[p]) / I.dr[I.ci[p]] * I.dc[j]);
@@ -323,50 +532,52 @@ __device__ void setup(BatchShared& sh, Inst& I, float& eta0, float& omega0) {
         }
         __syncthreads();
     }
+    for (int i = t; i < m; i += workers) I.rdr[i] = 1.0 / (double)I.dr[i];
+    for (int j = t; j < n; j += workers) I.rdc[j] = 1.0 / (double)I.dc[j];
     // scaled FP32 matrix; initial weight from the scaled cost and row bounds
     Acc<float> nq[2];
-    for (int i = t; i < m; i += kBT) {
+    for (int i = t; i < m; i += workers) {
         for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) I.sax[p] = I.ax[p] * I.dc[I.ai[p]] / I.dr[i];
         const float lo = (float)I.rmin[i] / I.dr[i], hi = (float)I.rmax[i] / I.dr[i];
         const float q = isfinite(hi) ? hi : (isfinite(lo) ? lo : 0.f);
         nq[1].add(q, q);
     }
-    for (int j = t; j < n; j += kBT) {
+    for (int j = t; j < n; j += workers) {
         for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) I.scax[p] = I.cax[p] * I.dc[j] / I.dr[I.ci[p]];
         const float cs = (float)I.c[j] * I.dc[j];
         nq[0].add(cs, cs);
     }
-    bmerge<2>(sh, nq);
+    bmerge<2>(nq, workers);
     if (t == 0) {
         const double cn = nq[0].result_d(), qn = nq[1].result_d();
         omega0 = (cn > 1e-24 && qn > 1e-24) ? fminf(3.f, fmaxf(0.3f, (float)sqrt(cn / qn))) : 1.f;
     }
     // power iteration for ||A~||_2^2
     const float v0 = rsqrtf((float)n);
-    for (int j = t; j < n; j += kBT) I.vt[j] = v0;
+    for (int j = t; j < n; j += workers) I.vt[j] = v0;
     __syncthreads();
     __shared__ float s_norm;
     for (int it = 0; it < 31; ++it) {
-        for (int i = t; i < m; i += kBT) I.mt[i] = row_dot(I.ap, I.ai, I.sax, I.vt, i).result();
+        for (int i = t; i < m; i += workers) I.mt[i] = row_dot(I.ap, I.ai, I.sax, I.vt, i).result();
         __syncthreads();
         if (it == 30) break;
         Acc<float> nrm[1];
-        for (int j = t; j < n; j += kBT) {
+        for (int j = t; j < n; j += workers) {
             const float wv = row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
-            I.xbar[j] = wv;
+            I.vt[j] = wv;  // normalised below, past the barrier
             nrm[0].add(wv, wv);
         }
-        bmerge<1>(sh, nrm);
+        bmerge<1>(nrm, workers);
         if (t == 0) s_norm = sqrtf((float)nrm[0].result_d());
         __syncthreads();
         const float nw = s_norm;
         if (!(nw > 1e-30f)) break;
-        for (int j = t; j < n; j += kBT) I.vt[j] = I.xbar[j] / nw;
+        for (int j = t; j < n; j += workers) I.vt[j] = I.vt[j] / nw;
         __syncthreads();
     }
     Acc<float> na[1];
-    for (int i = t; i < m; i += kBT) na[0].add(I.mt[i], I.mt[i]);
-    bmerge<1>(sh, na);
+    for (int i = t; i < m; i += workers) na[0].add(I.mt[i], I.mt[i]);
+    bmerge<1>(na, workers);
     if (t == 0) {
         double lam = na[0].result_d();
         if (!(lam > 0) || !isfinite(lam)) lam = 1.0;
@@ -375,344 +586,638 @@ __device__ void setup(BatchShared& sh, Inst& I, float& eta0, float& omega0) {
     __syncthreads();
 }
 
-// ---- FP64 metrics of one candidate (anchor + delta, original units) -----
-struct BMetrics {
-    double pinf, dinf, gap, op, od, prow, err;
-    bool finite;
-};
+// ---- FP64 metrics of both candidates (anchor + delta, original units) ----
+// FP64 comparisons cost a hundred cycles of latency and a slot of the one
+// FP64 unit of an SM; these run on the integer pipe. blt: a < b, false with a
+// NaN; bmax: maximum of values >= 0 (a NaN counts as nothing).
+__device__ __forceinline__ bool blt(double a, double b) {
+    const long long inf = 0x7ff0000000000000LL, sign = (long long)(1ULL << 63);
+    long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    if ((x & ~sign) > inf || (y & ~sign) > inf) return false;
+    x = x < 0 ? sign - x : x;  // -0 -> 0, negatives in their order
+    y = y < 0 ? sign - y : y;
+    return x < y;
+}
+__device__ __forceinline__ double bsel_max(double a, double b) { return blt(a, b) ? b : a; }
+__device__ __forceinline__ double bsel_min(double a, double b) { return blt(b, a) ? b : a; }
+__device__ __forceinline__ double bmax(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return y > x && y <= 0x7ff0000000000000LL ? b : a;
+}
+__device__ __forceinline__ double warp_bmax(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(kFull, hi);
+    const unsigned ml = __reduce_max_sync(kFull, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
 
-__device__ BMetrics metrics(BatchShared& sh, Inst& I, const float* xs, const float* ys,
-                            double cmax) {
-    const int t = threadIdx.x;
-    double r4[4] = {0.0, 0.0, 0.0, 0.0};  // pv, pa, prow, ymax
-    for (int i = t; i < I.m; i += kBT) {
-        const double Ax = (I.axh[i] + row_dot(I.ap, I.ai, I.sax, xs, i).result_d()) * (double)I.dr[i];
-        const double lo = I.rmin[i], hi = I.rmax[i];
-        const double vi = smax(lo - Ax, Ax - hi);
-        r4[0] = smax(r4[0], vi);
-        r4[1] = smax(r4[1], fabs(smin(smax(Ax, lo), hi)));
-        double scv = fabs(Ax);
-        if (isfinite(lo)) scv = smax(scv, fabs(lo));
-        if (isfinite(hi)) scv = smax(scv, fabs(hi));
-        r4[2] = smax(r4[2], smax(0.0, vi) / (1.0 + scv));
-        r4[3] = smax(r4[3], fabs((I.yh[i] + (double)ys[i]) / (double)I.dr[i]));
+// The metrics of the current (0) and averaged (1) iterates; valid in the
+// decision warp's first lane. Two barriers; the candidates share them and the
+// loads of the LP's data.
+template <int MODE>
+__device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int pc, int t,
+                                     int workers, double cmax, BMetrics* out) {
+    BatchShared& sh = b_shared();
+    const Inst I = make_inst(a, *d);
+    const Held<MODE> W = make_work<MODE>(a, *d);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = workers >> 5;
+    const bool works = wp < nw;
+    const float* xs[2] = {W.x(pc), W.xa(pc)};
+    const float* ys[2] = {W.y(pc), W.ya(pc)};
+    double mx[2][4] = {};  // pv, pa, prow, ymax
+    for (int s = wp; works && 32 * s < I.m; s += nw) {
+        const int q = 32 * s + lane;
+        const int i = q < I.m ? (MODE == kHeldOut ? W.rid32[q] : (int)W.rid[q]) : I.m;
+        for (int v = 0; v < 2; ++v) {
+            const Acc<float> ad = padded_dot(W.ri, W.rv, xs[v], W.rbase[s], W.rbase[s + 1]);
+            if (i >= I.m) continue;
+            const double Ax = (I.axh[i] + ad.result_d()) * (double)I.dr[i];
+            const double lo = I.rmin[i], hi = I.rmax[i];
+            const double vi = bsel_max(lo - Ax, Ax - hi);
+            mx[v][0] = bmax(mx[v][0], vi);
+            mx[v][1] = bmax(mx[v][1], dabs(bsel_min(bsel_max(Ax, lo), hi)));
+            if (blt(mx[v][2], vi)) {  // vi / (1 + scale) <= vi
+                double scv = dabs(Ax);
+                if (dfinite(lo)) scv = bsel_max(scv, dabs(lo));
+                if (dfinite(hi)) scv = bsel_max(scv, dabs(hi));
+                mx[v][2] = bmax(mx[v][2], vi / (1.0 + scv));
+            }
+            mx[v][3] = bmax(mx[v][3], dabs((I.yh[i] + (double)ys[v][i]) * I.rdr[i]));
+        }
     }
-    block_max<4, kBW>(r4, sh.dred);
-    __shared__ double s_r[4];
-    if (t == 0)
-        for (int q = 0; q < 4; ++q) s_r[q] = r4[q];
+    if (works)
+        for (int v = 0; v < 2; ++v)
+            for (int q = 0; q < 4; ++q) {
+                const double r = warp_bmax(mx[v][q]);
+                if (lane == 0) sh.dred[wp * 8 + 4 * v + q] = r;
+            }
     __syncthreads();
-    const double yz = 1e-8 * (1.0 + s_r[3]);
+    double yz[2], top[2][3];
+    for (int v = 0; v < 2; ++v) {
+        double ymax = 0.0;
+        for (int k = 0; k < nw; ++k) ymax = bmax(ymax, sh.dred[k * 8 + 4 * v + 3]);
+        yz[v] = 1e-8 * (1.0 + ymax);
+        if (!works)
+            for (int q = 0; q < 3; ++q) {
+                top[v][q] = 0.0;
+                for (int k = 0; k < nw; ++k) top[v][q] = bmax(top[v][q], sh.dred[k * 8 + 4 * v + q]);
+            }
+    }
+    __syncthreads();  // dred is written again below
     const double dz = 1e-8 * (1.0 + cmax);
-    double mx[2] = {0.0, 0.0};  // dv, unbounded
-    double sm[3] = {0.0, 0.0, 0.0};  // op, od (columns), od (rows)
-    for (int j = t; j < I.n; j += kBT) {
-        const double aty = I.atyh[j] + row_dot(I.cp, I.ci, I.scax, ys, j).result_d();
-        const double d = I.c[j] + aty / (double)I.dc[j];
-        const double lo = I.cl[j], hi = I.cu[j];
-        const float xv = xs[j];
-        const double x = xv == I.scl[j] ? lo : (xv == I.scu[j] ? hi : (I.xh[j] + (double)xv) * (double)I.dc[j]);
-        const double bnd = fabs(isfinite(hi) ? hi : lo);
-        const double tol = 1e-9 * (1.0 + bnd);
-        double e;
-        if (x <= lo + tol && d > 0) e = 0.0;
-        else if (x >= hi - tol && d < 0) e = 0.0;
-        else e = fabs(d);
-        mx[0] = smax(mx[0], e);
-        sm[0] += I.c[j] * x;
-        if (d >= 0) {
-            if (isfinite(lo)) sm[1] += d * lo;
-            else if (d > dz) mx[1] = 1.0;
-        } else {
-            if (isfinite(hi)) sm[1] += d * hi;
-            else if (-d > dz) mx[1] = 1.0;
+    double dv[2] = {0.0, 0.0}, op[2] = {0.0, 0.0}, od[2] = {0.0, 0.0};
+    bool unb[2] = {false, false};
+    for (int s = wp; works && 32 * s < I.n; s += nw) {
+        const int q = 32 * s + lane;
+        const int j = q < I.n ? (MODE == kHeldOut ? W.cid32[q] : (int)W.cid[q]) : I.n;
+        for (int v = 0; v < 2; ++v) {
+            const Acc<float> ad = padded_dot(W.ci, W.cv, ys[v], W.cbase[s], W.cbase[s + 1]);
+            if (j >= I.n) continue;
+            const double dcj = I.dc[j], cj = I.c[j];
+            const double aty = I.atyh[j] + ad.result_d();
+            const double d = cj + aty * I.rdc[j];
+            const double lo = I.cl[j], hi = I.cu[j];
+            const float xv = xs[v][j];
+            const double x = xv == W.scl()[j] ? lo : (xv == W.scu()[j] ? hi : (I.xh[j] + (double)xv) * dcj);
+            const double bnd = dabs(dfinite(hi) ? hi : lo);
+            const double tol = 1e-9 * (1.0 + bnd);
+            const double lob = lo + tol, hib = hi - tol;
+            const bool pos = blt(0.0, d), neg = blt(d, 0.0);
+            // (x <= lob is not lob < x, but for a NaN, which is not at a bound)
+            const bool real = blt(x, CUDART_INF) || blt(-CUDART_INF, x);
+            const bool at_lo = pos && real && lob == lob && !blt(lob, x);
+            const bool at_hi = neg && real && hib == hib && !blt(x, hib);
+            if (!at_lo && !at_hi) dv[v] = bmax(dv[v], dabs(d));
+            op[v] += cj * x;
+            if (!neg) {
+                if (dfinite(lo)) od[v] += d * lo;
+                else if (blt(dz, d)) unb[v] = true;
+            } else {
+                if (dfinite(hi)) od[v] += d * hi;
+                else if (blt(dz, -d)) unb[v] = true;
+            }
         }
     }
-    for (int i = t; i < I.m; i += kBT) {
-        const double yv = (I.yh[i] + (double)ys[i]) / (double)I.dr[i];
-        if (yv > yz) {
-            if (isfinite(I.rmax[i])) sm[2] -= yv * I.rmax[i];
-            else mx[1] = 1.0;
-        } else if (yv < -yz) {
-            if (isfinite(I.rmin[i])) sm[2] -= yv * I.rmin[i];
-            else mx[1] = 1.0;
+    for (int i = t; i < I.m; i += workers)
+        for (int v = 0; v < 2; ++v) {
+            const double yv = (I.yh[i] + (double)ys[v][i]) * I.rdr[i];
+            if (blt(yz[v], yv)) {
+                if (dfinite(I.rmax[i])) od[v] -= yv * I.rmax[i];
+                else unb[v] = true;
+            } else if (blt(yv, -yz[v])) {
+                if (dfinite(I.rmin[i])) od[v] -= yv * I.rmin[i];
+                else unb[v] = true;
+            }
         }
-    }
-    block_max<2, kBW>(mx, sh.dred);
-    block_sum<3, kBW>(sm, sh.dred);
-    __shared__ BMetrics s_m;
-    if (t == 0) {
-        BMetrics mt;
-        mt.pinf = smax(s_r[0], 0.0) / (1.0 + s_r[1]);
-        mt.prow = s_r[2];
-        mt.dinf = mx[0] / (1.0 + cmax);
-        mt.op = sm[0];
-        const bool bounded = !(mx[1] > 0.0);
-        mt.od = bounded ? sm[1] + sm[2] : -CUDART_INF;
-        mt.gap = bounded ? smax(0.0, mt.op - mt.od) / (1.0 + fabs(mt.op)) : CUDART_INF;
-        mt.finite = isfinite(mt.pinf) && isfinite(mt.dinf);
-        mt.err = smax(mt.pinf, smax(mt.dinf, isfinite(mt.gap) ? mt.gap : 0.0));
-        s_m = mt;
-    }
+    if (works)
+        for (int v = 0; v < 2; ++v) {
+            const double r = warp_bmax(dv[v]), so = warp_sum(op[v]), sd = warp_sum(od[v]);
+            const bool u = __any_sync(kFull, unb[v]);
+            if (lane == 0) {
+                double* P = sh.dred + wp * 8 + 4 * v;
+                P[0] = r;
+                P[1] = so;
+                P[2] = sd;
+                P[3] = u ? 1.0 : 0.0;
+            }
+        }
     __syncthreads();
-    return s_m;
+    if (!works && lane == 0)
+        for (int v = 0; v < 2; ++v) {
+            double r = 0.0, so = 0.0, sd = 0.0, u = 0.0;
+            for (int k = 0; k < nw; ++k) {
+                const double* P = sh.dred + k * 8 + 4 * v;
+                r = bmax(r, P[0]);
+                so += P[1];
+                sd += P[2];
+                u = bmax(u, P[3]);
+            }
+            BMetrics mt;
+            mt.pinf = top[v][0] / (1.0 + top[v][1]);
+            mt.prow = top[v][2];
+            mt.dinf = r / (1.0 + cmax);
+            mt.op = so;
+            const bool bounded = !(u > 0.0);
+            mt.od = bounded ? sd : -CUDART_INF;
+            mt.gap = bounded ? smax(0.0, mt.op - mt.od) / (1.0 + fabs(mt.op)) : CUDART_INF;
+            mt.finite = isfinite(mt.pinf) && isfinite(mt.dinf);
+            mt.err = smax(mt.pinf, smax(mt.dinf, isfinite(mt.gap) ? mt.gap : 0.0));
+            out[v] = mt;
+        }
+}
+
+// A restart: the chosen candidate becomes the new FP64 anchor and the deltas
+// restart at zero; the warps' squared movements of the anchor go to sh.dred.
+template <int MODE>
+__device__ __noinline__ void re_anchor(const BatchArgs& a, const BatchDesc* d, int pc, int use_avg,
+                                       int t, int workers) {
+    BatchShared& sh = b_shared();
+    const Inst I = make_inst(a, *d);
+    const Held<MODE> W = make_work<MODE>(a, *d);
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    float *x = W.x(pc), *xa = W.xa(pc), *g = W.g(pc);
+    float *y = W.y(pc), *ya = W.ya(pc), *axc = W.axc(pc);
+    double dn[2] = {0.0, 0.0};
+    for (int j = t; j < I.n; j += workers) {
+        const double nx = full_x<MODE>(I, W, j, use_avg ? xa[j] : x[j]);
+        const double dd = nx - I.pesx[j];
+        dn[0] = fma(dd, dd, dn[0]);
+        I.pesx[j] = I.xh[j] = nx;
+        x[j] = xa[j] = g[j] = 0.f;  // g = A~^T 0
+    }
+    for (int i = t; i < I.m; i += workers) {
+        const double ny = I.yh[i] + (double)(use_avg ? ya[i] : y[i]);
+        const double dd = ny - I.pesy[i];
+        dn[1] = fma(dd, dd, dn[1]);
+        I.pesy[i] = I.yh[i] = ny;
+        y[i] = ya[i] = axc[i] = 0.f;
+    }
+    for (int v = 0; v < 2; ++v) {
+        dn[v] = warp_sum(dn[v]);
+        if (lane == 0 && wp < workers / 32) sh.dred[2 * wp + v] = dn[v];
+    }
+}
+
+// a / b for one divisor b, rb = 1 / b: one remainder step (Markstein 1990;
+// the correctly rounded quotient but for rare cases one ulp off)
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q0 = a * rb;
+    return dfinite(q0) ? fma(fma(-b, q0, a), rb, q0) : a / b;
 }
 
 // ---- one LP --------------------------------------------------------------
-__device__ void solve_one(const BatchArgs& a, BatchShared& sh, const BatchDesc& d, int b) {
+// An iteration is bound by latency: the phases' instruction streams and
+// dependent loads, and above all the step decision, a chain of FP64 operations
+// (60 cycles each, a division 575) in one thread. So the decision has a warp
+// of its own, which holds the controller's state in registers, and while it
+// runs the workers form A~^T y of the dual just computed: the next attempt
+// needs it if the step is accepted (after a rejected one the accepted dual's
+// product is still there). Four barriers per attempt:
+//   workers                                  decision warp
+//   primal step (columns t, t + kBT, ..)     --
+//   sums of its dx^2; A~ xbar (by slices)    factors of the next decision
+//   dual step (rows t, t + kBT, ..), sums    merges the warps' dx^2
+//   A~^T y' (by slices)                      merges the rest, decides
+// One iteration of an LP of 113 x 282: 6.2 us with the whole CTA waiting for
+// one thread's decision and a lane walking each row, now 3.4; 650 x 1,625
+// (10,476 nonzeros) 18.7 -> 7.7; 792 x 1,980 (15,561; iterates and residual
+// data do not fit beside the matrix) 22.1 -> 11.9.
+__device__ __forceinline__ void cta_sync() {
+    __syncwarp();
+    asm volatile("barrier.sync 0;" ::: "memory");
+}
+
+// Merge of the warps' partials acc[0], acc[3], ... in their order.
+__device__ __forceinline__ double merge_warps(const Acc<float>* acc, int warps) {
+    Acc<float> s = acc[0];
+#pragma unroll 1
+    for (int k = 1; k < warps; ++k) s.merge(acc[3 * k]);
+    return s.result_d();
+}
+
+// Acc merged over the lanes of a warp, as block_merge does.
+template <int NV>
+__device__ __forceinline__ void lanes_merge(Acc<float> (&v)[NV]) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) v[q].shfl_xor(kFull, o, 32);
+}
+
+// Products of the staged rows: out[id] = row id times v, in the order of its
+// entries (compensated FP32), a warp per slice.
+template <class Idx>
+__device__ __forceinline__ void slice_products(const int* base, const uint16_t* id16,
+                                               const int* id32, const Idx* idx, const float* val,
+                                               const float* __restrict__ v, float* out,
+                                               int rows) {
+    const int lane = threadIdx.x & 31, warps = (blockDim.x >> 5) - 1;
+    for (int s = threadIdx.x >> 5; 32 * s < rows; s += warps) {
+        const int q = 32 * s + lane;
+        const int row = q < rows ? (id16 ? (int)id16[q] : id32[q]) : -1;
+        const Acc<float> acc = padded_dot(idx, val, v, base[s], base[s + 1]);
+        if (row >= 0) out[row] = acc.result();
+    }
+}
+
+template <int MODE>
+__device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc* d,
+                                            const Held<MODE>& W, int workers, double cmax) {
+    BatchShared& sh = b_shared();
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int t = (int)threadIdx.x < workers ? (int)threadIdx.x : 1 << 30;
+    const int m = W.m, n = W.n;
+    for (;;) {
+        const int p = sh.step.parity, q = p ^ 1;
+        const float tau = sh.step.tau, sigma = sh.step.sigma, w = sh.step.w;
+        Acc<float> dx2[1];
+        {   // primal step from g = A~^T y (thread per column), on the deltas
+            const float *__restrict__ sc = W.sc(), *__restrict__ gp = W.g(p);
+            const float *__restrict__ xp = W.x(p), *__restrict__ xap = W.xa(p);
+            const float *__restrict__ lo = W.scl(), *__restrict__ hi = W.scu();
+            float *__restrict__ xq = W.x(q), *__restrict__ xaq = W.xa(q);
+            float* __restrict__ xbar = W.xbar;
+            // (short code: unrolled by 2 or 4, an iteration takes 5-15 % longer)
+#pragma unroll 1
+            for (int j = t; j < n; j += workers) {
+                const float g = sc[j] + gp[j];
+                const float xv = xp[j], av = xap[j];
+                const float xn = fminf(fmaxf(fmaf(-tau, g, xv), lo[j]), hi[j]);
+                xq[j] = xn;
+                xbar[j] = fmaf(2.f, xn, -xv);
+                const float dx = xn - xv;
+                dx2[0].add(dx, dx);
+                xaq[j] = fmaf(w, xn - av, av);
+            }
+        }
+        cta_sync();
+        if (t < workers) {
+            lanes_merge(dx2);
+            if (lane == 0) sh.acc[wp * 3] = dx2[0];
+        }
+        slice_products(W.rbase, W.rid, W.rid32, W.ri, W.rv, W.xbar, W.ab, m);
+        cta_sync();
+        {   // dual step; the projection acts on the full value, so the anchor
+            // enters its argument
+            const float *__restrict__ yp = W.y(p), *__restrict__ axp = W.axc(p);
+            const float *__restrict__ yap = W.ya(p), *__restrict__ ab_ = W.ab;
+            const float *__restrict__ yh = W.yh32(), *__restrict__ lo = W.srmin();
+            const float* __restrict__ hi = W.srmax();
+            float *__restrict__ yq = W.y(q), *__restrict__ axq = W.axc(q);
+            float* __restrict__ yaq = W.ya(q);
+            Acc<float> dots[2];
+#pragma unroll 1
+            for (int i = t; i < m; i += workers) {
+                const float ab = ab_[i], yv = yp[i], ax = axp[i], av = yap[i];
+                const float tt = fmaf(sigma, ab, yv);
+                const float arg = (tt + yh[i]) / sigma;
+                const float yn = fmaf(-sigma, fminf(fmaxf(arg, lo[i]), hi[i]), tt);
+                yq[i] = yn;
+                const float dy = yn - yv;
+                const float adx = 0.5f * (ab - ax);
+                axq[i] = ax + adx;
+                dots[0].add(dy, dy);
+                dots[1].add(dy, adx);
+                yaq[i] = fmaf(w, yn - av, av);
+            }
+            if (t < workers && 32 * wp < m) {  // (warp-uniform)
+                __syncwarp();
+                lanes_merge(dots);
+                if (lane == 0) {
+                    sh.acc[wp * 3 + 1] = dots[0];
+                    sh.acc[wp * 3 + 2] = dots[1];
+                }
+            }
+        }
+        cta_sync();
+        slice_products(W.cbase, W.cid, W.cid32, W.ci, W.cv, W.y(q), W.g(q), n);
+        cta_sync();
+        if (sh.step.done) return;
+        if (!sh.step.check) continue;
+        const int pc = sh.step.parity;
+        metrics<MODE>(a, d, pc, t, workers, cmax, nullptr);
+        cta_sync();
+        if (sh.step.done) return;
+        if (sh.step.restart) {
+            re_anchor<MODE>(a, d, pc, sh.step.use_avg, t, workers);
+            cta_sync();
+            anchor_data<MODE>(a, d, t, workers);  // ends with a barrier
+        }
+    }
+}
+
+// The decision warp's side of the same loop. Its first lane holds the state.
+template <int MODE>
+__device__ __forceinline__ void decision_loop(const BatchArgs& a, const BatchDesc* d, int workers,
+                                              double cmax, double eta, double omega, BatchOut& o) {
+    BatchShared& sh = b_shared();
+    const int lane = threadIdx.x & 31;
+    const int warps_c = min(workers, d->n + 31) / 32, warps_r = min(workers, d->m + 31) / 32;
+    BatchRare& c = sh.rare;
+    double romega = 1.0 / omega;
+    long long k = 1, hn = 0, attempts = 0;
+    int until = a.check, retries = 0;
+    if (lane == 0) {
+        c.epoch_kkt = -1.0;
+        c.prev_cand = CUDART_INF;
+        c.epoch_start = c.restarts = 0;
+        c.status = IGAOS_STATUS_ITERATION_LIMIT;
+        c.asked = c.handed = c.have_pe = 0;
+        c.last.pinf = c.last.dinf = c.last.gap = c.last.prow = CUDART_INF;
+        c.last.op = 0.0;
+    }
+    // the averaging weight 2 / (h + 2), rounded from FP64; for h below 2^24 the
+    // FP32 quotient is the same number (a quotient of such integers is never
+    // within an FP64 rounding of the middle of two floats)
+    auto weight = [](long long h) {
+        return h < (1 << 24) - 2 ? 2.f / (float)(int)(h + 2) : (float)(2.0 / ((double)h + 2.0));
+    };
+    // factors 1 - k^-0.3 and 1 + k^-0.6 (src/pdhg/pdhg.cu:778-782), those of
+    // the next iteration loaded while this one runs
+    auto factors = [&](long long i, float& lo, float& hi) {
+        lo = i < kFacTab ? a.fac[2 * i] : 1.f - powf((float)i, -0.3f);
+        hi = i < kFacTab ? a.fac[2 * i + 1] : 1.f + powf((float)i, -0.6f);
+    };
+    float lo_now, hi_now, lo_next, hi_next;
+    factors(1, lo_now, hi_now);
+    factors(2, lo_next, hi_next);
+    for (;;) {
+        const float w_next = weight(hn + 1);
+        const double flo = lo_now, fhi_eta = (double)hi_now * eta;
+        cta_sync();
+        cta_sync();
+        // fixed-order merges over the warps that hold columns (rows), one
+        // quantity per lane
+        const double dx2 = merge_warps(sh.acc, warps_c);
+        cta_sync();
+        const double dot = merge_warps(sh.acc + 1 + (lane & 1), warps_r);
+        const double dy2 = dot, cross = __shfl_sync(kFull, dot, 1);
+        if (lane == 0) {
+            // step decision (src/pdhg/pdhg.cu:770-794). num, cross, etabar and
+            // the step sizes compare as integers: all are >= 0 there
+            ++attempts;
+            auto less_pos = [](double u, double v) {
+                return __double_as_longlong(u) < __double_as_longlong(v);
+            };
+            const double num = fma(omega, dx2, div_by(dy2, omega, romega));
+            const bool sound = dfinite(dx2) && dfinite(dy2) && dfinite(cross);
+            double etabar = CUDART_INF, eta_new = CUDART_INF;
+            const bool curved = sound && dfinite(num) && dgt0(num) && dgt0(cross);
+            if (curved) {
+                etabar = num / (2.0 * cross);
+                const double up = flo * etabar;
+                if (dfinite(etabar)) eta_new = less_pos(fhi_eta, up) ? fhi_eta : up;
+            }
+            const bool accept = !curved || !less_pos(etabar, eta) || retries >= 20;
+            const bool usable = dfinite(eta_new) && less_pos(1e-12, eta_new);
+            const double capped = less_pos(1e12, eta_new) ? 1e12 : eta_new;
+            eta = usable ? (accept ? capped : eta_new) : (accept ? eta : fmax(eta_new, 1e-12));
+            BatchStep& s = sh.step;
+            if (!sound) {
+                s.done = 1;
+                c.status = IGAOS_STATUS_ERROR;
+            }
+            until -= accept;
+            const int check = accept && sound && (until == 0 || k >= a.maxit);
+            until = until == 0 ? a.check : until;
+            retries = accept ? 0 : retries + 1;
+            hn += accept;
+            k += accept;
+            if (accept) {
+                s.parity ^= 1;
+                s.w = w_next;
+                lo_now = lo_next;
+                hi_now = hi_next;
+            }
+            s.check = check;
+            s.tau = (float)div_by(eta, omega, romega);
+            s.sigma = (float)(eta * omega);
+            if (accept) factors(k + 1, lo_next, hi_next);
+        }
+        cta_sync();
+        if (sh.step.done) break;
+        if (!sh.step.check) continue;
+        const int pc = sh.step.parity;
+        metrics<MODE>(a, d, pc, 1 << 30, workers, cmax, c.now);
+        if (lane == 0) {
+            const BMetrics &mc = c.now[0], &ma = c.now[1];
+            const long long kd = k - 1;  // index of the iteration just accepted
+            auto passes = [&](const BMetrics& u) {
+                return u.pinf <= a.tol && u.dinf <= a.tol && u.prow <= a.tol && isfinite(u.gap) &&
+                       u.gap <= a.tol;
+            };
+            const double ec = mc.finite ? mc.err : CUDART_INF;
+            const double ea = ma.finite ? ma.err : CUDART_INF;
+            BatchStep& s = sh.step;
+            c.last = (ec <= ea) ? mc : ma;
+            s.use_avg = ea < ec;
+            s.restart = 0;
+            if (passes(mc)) {
+                c.last = mc;
+                s.use_avg = 0;
+                s.done = 1;
+                c.status = IGAOS_STATUS_NEAR_OPTIMAL;
+            } else if (passes(ma)) {
+                c.last = ma;
+                s.use_avg = 1;
+                s.done = 1;
+                c.status = IGAOS_STATUS_NEAR_OPTIMAL;
+            } else if (kd >= a.maxit) {
+                s.done = 1;
+            } else if (kd >= a.handoff_at && !c.asked &&
+                       (c.asked = 1, atomicAdd(a.handoff_count, 1u) < (unsigned)a.handoff_max)) {
+                s.done = 1;  // left for the FP64 finish
+                c.handed = 1;
+            } else {
+                const double cand = fmin(ec, ea);
+                if (c.epoch_kkt < 0.0) {
+                    c.epoch_kkt = cand;
+                    c.prev_cand = cand;
+                }
+                const long long te = kd - c.epoch_start;
+                s.restart = (isfinite(cand) && isfinite(c.epoch_kkt) && c.epoch_kkt > 0.0 &&
+                             (cand <= 0.2 * c.epoch_kkt ||
+                              (cand <= 0.8 * c.epoch_kkt && isfinite(c.prev_cand) && cand > c.prev_cand))) ||
+                            (double)te >= 0.36 * (double)kd;
+                c.prev_cand = cand;
+                if (s.restart) {
+                    hn = 0;
+                    c.epoch_start = kd;
+                    c.epoch_kkt = cand;
+                    c.prev_cand = CUDART_INF;
+                    ++c.restarts;
+                }
+            }
+        }
+        cta_sync();
+        if (sh.step.done) break;
+        if (sh.step.restart) {
+            cta_sync();  // the anchor's movement is in sh.dred
+            if (lane == 0) {
+                double dxn = 0.0, dyn = 0.0;
+                for (int v = 0; v < workers / 32; ++v) {
+                    dxn += sh.dred[2 * v];
+                    dyn += sh.dred[2 * v + 1];
+                }
+                if (c.have_pe && dxn > 1e-24 && dyn > 1e-24) {  // primal weight
+                    const double om = sqrt(omega * sqrt(dyn / dxn));
+                    if (isfinite(om) && om > 0.0) omega = fmin(fmax(om, 1e-6), 1e6);
+                }
+                c.have_pe = 1;
+                romega = 1.0 / omega;
+                sh.step.tau = (float)(eta / omega);
+                sh.step.sigma = (float)(eta * omega);
+                sh.step.w = weight(hn);
+            }
+            cta_sync();
+        }
+    }
+    o.status = c.status;
+    o.handed = c.handed;
+    o.objective = c.last.op;
+    o.pinf = c.last.pinf;
+    o.dinf = c.last.dinf;
+    o.gap = c.last.gap;
+    o.prow = c.last.prow;
+    o.iterations = k - 1;
+    o.attempts = attempts;
+    o.restarts = c.restarts;
+}
+
+template <int MODE>
+__device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
     const long long t_begin = global_ns();
-    Inst I = make_inst(a, d);
-    const int t = threadIdx.x, m = I.m, n = I.n;
+    BatchShared& sh = b_shared();
+    const BatchDesc* dp = a.desc + b;
+    const BatchDesc d = *dp;
+    const int workers = min((int)blockDim.x - 32, kBT);
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool decider = threadIdx.x >= blockDim.x - 32;
+    const int t = (int)threadIdx.x < workers ? (int)threadIdx.x : 1 << 30;
+    const int m = d.m, n = d.n;
+    const Held<MODE> W = make_work<MODE>(a, d);
     __shared__ float s_eta0, s_omega0;
     __shared__ double s_cmax;
-    for (int j = t; j < n; j += kBT) I.xh[j] = I.pesx[j] = 0.0;
-    for (int i = t; i < m; i += kBT) I.yh[i] = I.pesy[i] = 0.0;
-    setup(sh, I, s_eta0, s_omega0);
-    anchor_data(I);
     {
-        double cm[1] = {0.0};
-        for (int j = t; j < n; j += kBT) cm[0] = smax(cm[0], fabs(I.c[j]));
-        block_max<1, kBW>(cm, sh.dred);
-        if (t == 0) s_cmax = cm[0];
+        const Inst I = make_inst(a, d);
+        for (int j = t; j < n; j += workers) I.xh[j] = I.pesx[j] = 0.0;
+        for (int i = t; i < m; i += workers) I.yh[i] = I.pesy[i] = 0.0;
     }
-    for (int j = t; j < n; j += kBT) I.x[0][j] = I.xa[0][j] = 0.f;
-    for (int i = t; i < m; i += kBT) I.y[0][i] = I.ya[0][i] = I.axc[0][i] = 0.f;
-    // controller state (thread 0)
-    __shared__ double s_epoch_kkt, s_prev_cand, s_omega, s_eta;
-    __shared__ long long s_k, s_hn, s_epoch_start, s_attempts, s_restarts;
-    __shared__ int s_retries, s_have_pe, s_done, s_status, s_use_avg, s_restart, s_avg_better;
-    __shared__ int s_asked, s_handed;
-    __shared__ BMetrics s_last;
-    if (t == 0) {
-        s_eta = s_eta0;
-        s_omega = s_omega0;
-        s_k = 1;
-        s_hn = 0;
-        s_epoch_kkt = -1.0;
-        s_prev_cand = CUDART_INF;
-        s_epoch_start = 0;
-        s_attempts = 0;
-        s_restarts = 0;
-        s_retries = 0;
-        s_have_pe = 0;
-        s_done = 0;
-        s_status = IGAOS_STATUS_ITERATION_LIMIT;
-        s_use_avg = 0;
-        s_asked = 0;
-        s_handed = 0;
-        sh.parity = 0;
-        s_last.pinf = s_last.dinf = CUDART_INF;
-        s_last.gap = CUDART_INF;
-        s_last.op = 0.0;
-        s_last.prow = CUDART_INF;
+    setup(a, dp, t, workers, s_eta0, s_omega0);
+    fill_work<MODE>(a, dp, workers);
+    anchor_data<MODE>(a, dp, t, workers);
+    {
+        double cm = 0.0;
+        for (int j = t; j < n; j += workers) cm = bmax(cm, fabs(a.c[d.col_off + j]));
+        cm = warp_bmax(cm);
+        if (lane == 0 && t < workers) sh.dred[wp] = cm;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < workers / 32; ++k) cm = bmax(cm, sh.dred[k]);
+            s_cmax = cm;
+        }
+    }
+    for (int j = t; j < n; j += workers) {
+        W.x(0)[j] = W.xa(0)[j] = 0.f;
+        W.g(0)[j] = 0.f;  // A~^T 0
+    }
+    for (int i = t; i < m; i += workers) W.y(0)[i] = W.ya(0)[i] = W.axc(0)[i] = 0.f;
+    const double eta = s_eta0, omega = s_omega0;
+    if (threadIdx.x == 0) {
+        sh.step.tau = (float)(eta / omega);
+        sh.step.sigma = (float)(eta * omega);
+        sh.step.w = 1.f;
+        sh.step.parity = sh.step.done = sh.step.check = sh.step.restart = sh.step.use_avg = 0;
     }
     __syncthreads();
-    const long long maxit = a.maxit;
-    while (!s_done) {
-        if (t == 0) {
-            sh.tau = (float)(s_eta / s_omega);
-            sh.sigma = (float)(s_eta * s_omega);
-            sh.w = (float)(2.0 / ((double)s_hn + 2.0));
-        }
-        __syncthreads();
-        const int p = sh.parity, q = p ^ 1;
-        const float tau = sh.tau, sigma = sh.sigma, w = sh.w;
-        Acc<float> dots[3];
-        // primal step fused with A^T y (thread per column), on the deltas
-        for (int j = t; j < n; j += kBT) {
-            const float g = I.sc[j] + row_dot(I.cp, I.ci, I.scax, I.y[p], j).result();
-            const float xv = I.x[p][j];
-            const float xn = fminf(fmaxf(fmaf(-tau, g, xv), I.scl[j]), I.scu[j]);
-            I.x[q][j] = xn;
-            I.xbar[j] = fmaf(2.f, xn, -xv);
-            const float dx = xn - xv;
-            dots[0].add(dx, dx);
-            const float av = I.xa[p][j];
-            I.xa[q][j] = fmaf(w, xn - av, av);
-        }
-        __syncthreads();
-        // dual step fused with A xbar (thread per row); the projection acts
-        // on the full value, so the anchor enters its argument
-        for (int i = t; i < m; i += kBT) {
-            const float ab = row_dot(I.ap, I.ai, I.sax, I.xbar, i).result();
-            const float yv = I.y[p][i];
-            const float tt = fmaf(sigma, ab, yv);
-            const float arg = (tt + I.yh32[i]) / sigma;
-            const float yn = fmaf(-sigma, fminf(fmaxf(arg, I.srmin[i]), I.srmax[i]), tt);
-            I.y[q][i] = yn;
-            const float dy = yn - yv;
-            const float ax = I.axc[p][i];
-            const float adx = 0.5f * (ab - ax);
-            I.axc[q][i] = ax + adx;
-            dots[1].add(dy, dy);
-            dots[2].add(dy, adx);
-            const float av = I.ya[p][i];
-            I.ya[q][i] = fmaf(w, yn - av, av);
-        }
-        bmerge<3>(sh, dots);
-        // step decision (src/pdhg/pdhg.cu:770-794)
-        if (t == 0) {
-            ++s_attempts;
-            const double dx2 = dots[0].result_d(), dy2 = dots[1].result_d(),
-                         cross = dots[2].result_d();
-            const double eta = s_eta, om = s_omega;
-            const double num = om * dx2 + dy2 / om;
-            const double etabar = (num > 0.0 && cross > 0.0) ? num / (2.0 * cross) : CUDART_INF;
-            const long long k = s_k;
-            const float flo = k < kFacTab ? a.fac[2 * k] : 1.f - powf((float)k, -0.3f);
-            const float fhi = k < kFacTab ? a.fac[2 * k + 1] : 1.f + powf((float)k, -0.6f);
-            const double eta_new =
-                isfinite(etabar) ? fmin((double)flo * etabar, (double)fhi * eta) : CUDART_INF;
-            bool acc_ = !(eta > etabar) || num <= 0.0 || cross <= 0.0;
-            if (!acc_) acc_ = ++s_retries > 20;
-            if (!isfinite(dx2) || !isfinite(dy2) || !isfinite(cross)) {
-                s_done = 1;
-                s_status = IGAOS_STATUS_ERROR;
-            }
-            if (acc_) {
-                if (isfinite(eta_new) && eta_new > 1e-12) s_eta = fmin(eta_new, 1e12);
-                sh.parity ^= 1;
-                ++s_hn;
-                s_retries = 0;
-                sh.kdone = s_k;  // index of the iteration just accepted
-                ++s_k;
-            } else {
-                s_eta = fmax(eta_new, 1e-12);
-            }
-            sh.accept = acc_;
-        }
-        __syncthreads();
-        if (!sh.accept || s_done) continue;
-        const long long k = sh.kdone;
-        const int pc = sh.parity;
-        if (k % a.check == 0 || k >= maxit) {
-            const BMetrics mc = metrics(sh, I, I.x[pc], I.y[pc], s_cmax);
-            const BMetrics ma = metrics(sh, I, I.xa[pc], I.ya[pc], s_cmax);
-            if (t == 0) {
-                auto passes = [&](const BMetrics& u) {
-                    return u.pinf <= a.tol && u.dinf <= a.tol && u.prow <= a.tol &&
-                           isfinite(u.gap) && u.gap <= a.tol;
-                };
-                const double ec = mc.finite ? mc.err : CUDART_INF;
-                const double ea = ma.finite ? ma.err : CUDART_INF;
-                s_last = (ec <= ea) ? mc : ma;
-                s_use_avg = ea < ec;
-                s_restart = 0;
-                if (passes(mc)) {
-                    s_last = mc;
-                    s_use_avg = 0;
-                    s_done = 1;
-                    s_status = IGAOS_STATUS_NEAR_OPTIMAL;
-                } else if (passes(ma)) {
-                    s_last = ma;
-                    s_use_avg = 1;
-                    s_done = 1;
-                    s_status = IGAOS_STATUS_NEAR_OPTIMAL;
-                } else if (k >= maxit) {
-                    s_done = 1;
-                } else if (k >= a.handoff_at && !s_asked &&
-                           (s_asked = 1, atomicAdd(a.handoff_count, 1u) < (unsigned)a.handoff_max)) {
-                    s_done = 1;  // left for the FP64 finish
-                    s_handed = 1;
-                } else {
-                    const double cand = fmin(ec, ea);
-                    if (s_epoch_kkt < 0.0) {
-                        s_epoch_kkt = cand;
-                        s_prev_cand = cand;
-                    }
-                    const long long te = k - s_epoch_start;
-                    s_restart = (isfinite(cand) && isfinite(s_epoch_kkt) && s_epoch_kkt > 0.0 &&
-                                 (cand <= 0.2 * s_epoch_kkt ||
-                                  (cand <= 0.8 * s_epoch_kkt && isfinite(s_prev_cand) &&
-                                   cand > s_prev_cand))) ||
-                                (double)te >= 0.36 * (double)k;
-                    s_prev_cand = cand;
-                    if (s_restart) {
-                        s_avg_better = ea < ec;
-                        s_hn = 0;
-                        s_epoch_start = k;
-                        s_epoch_kkt = cand;
-                        s_prev_cand = CUDART_INF;
-                        ++s_restarts;
-                    }
-                }
-            }
-            __syncthreads();
-            if (s_restart) {
-                // the restart point becomes the new FP64 anchor; deltas restart
-                // at zero; primal weight from the anchors' movement
-                const float* dxs = s_avg_better ? I.xa[pc] : I.x[pc];
-                const float* dys = s_avg_better ? I.ya[pc] : I.y[pc];
-                double dn[2] = {0.0, 0.0};
-                for (int j = t; j < n; j += kBT) {
-                    const double nx = full_x(I, j, dxs[j]);
-                    const double dd = nx - I.pesx[j];
-                    dn[0] = fma(dd, dd, dn[0]);
-                    I.pesx[j] = nx;
-                }
-                for (int i = t; i < m; i += kBT) {
-                    const double ny = I.yh[i] + (double)dys[i];
-                    const double dd = ny - I.pesy[i];
-                    dn[1] = fma(dd, dd, dn[1]);
-                    I.pesy[i] = ny;
-                }
-                block_sum<2, kBW>(dn, sh.dred);
-                if (t == 0 && s_have_pe) {
-                    const double dxn = dn[0], dyn = dn[1];
-                    if (dxn > 1e-24 && dyn > 1e-24) {
-                        const double om = sqrt(s_omega * sqrt(dyn / dxn));
-                        if (isfinite(om) && om > 0.0) s_omega = fmin(fmax(om, 1e-6), 1e6);
-                    }
-                }
-                if (t == 0) s_have_pe = 1;
-                // the new anchor is the restart point (held in pes)
-                for (int j = t; j < n; j += kBT) {
-                    I.xh[j] = I.pesx[j];
-                    I.x[pc][j] = I.xa[pc][j] = 0.f;
-                }
-                for (int i = t; i < m; i += kBT) {
-                    I.yh[i] = I.pesy[i];
-                    I.y[pc][i] = I.ya[pc][i] = I.axc[pc][i] = 0.f;
-                }
-                __syncthreads();
-                anchor_data(I);
-            }
-        }
-    }
-    // answer: anchor + delta of the chosen candidate, original units
-    const int pf = sh.parity;
-    const float* xs = s_use_avg ? I.xa[pf] : I.x[pf];
-    const float* ys = s_use_avg ? I.ya[pf] : I.y[pf];
-    double* xo = a.x_out ? a.x_out + d.col_off : nullptr;
-    double* yo = a.y_out ? a.y_out + d.row_off : nullptr;
-    if (xo)
-        for (int j = t; j < n; j += kBT) {
-            const float xv = xs[j];
-            xo[j] = xv == I.scl[j] ? I.cl[j]
-                                   : (xv == I.scu[j] ? I.cu[j] : (I.xh[j] + (double)xv) * (double)I.dc[j]);
-        }
-    if (yo)
-        for (int i = t; i < m; i += kBT) yo[i] = (I.yh[i] + (double)ys[i]) / (double)I.dr[i];
-    if (t == 0) {
+    if (decider) {
         BatchOut o;
-        o.status = s_status;
-        o.handed = s_handed;
-        o.objective = s_last.op;
-        o.pinf = s_last.pinf;
-        o.dinf = s_last.dinf;
-        o.gap = s_last.gap;
-        o.prow = s_last.prow;
-        o.iterations = s_k - 1;
-        o.attempts = s_attempts;
-        o.restarts = s_restarts;
-        o.ns = global_ns() - t_begin;
-        a.out[b] = o;
+        decision_loop<MODE>(a, dp, workers, s_cmax, eta, omega, o);
+        if (lane == 0) {
+            o.ns = global_ns() - t_begin;
+            a.out[b] = o;
+        }
+    } else {
+        worker_loop<MODE>(a, dp, W, workers, s_cmax);
+        const Inst I = make_inst(a, d);
+        // answer: anchor + delta of the chosen candidate, original units
+        const int pf = sh.step.parity;
+        const float* xs = sh.step.use_avg ? W.xa(pf) : W.x(pf);
+        const float* ys = sh.step.use_avg ? W.ya(pf) : W.y(pf);
+        double* xo = a.x_out + d.col_off;
+        double* yo = a.y_out + d.row_off;
+        for (int j = t; j < n; j += workers) {
+            const float xv = xs[j];
+            xo[j] = xv == W.scl()[j]
+                        ? I.cl[j]
+                        : (xv == W.scu()[j] ? I.cu[j] : (I.xh[j] + (double)xv) * (double)I.dc[j]);
+        }
+        for (int i = t; i < m; i += workers) yo[i] = (I.yh[i] + (double)ys[i]) / (double)I.dr[i];
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBT) k_batch(BatchArgs a) {
-    __shared__ BatchShared sh;
+// Classes of instances: threads, CTAs per SM the kernel is compiled
+// for, and the shared memory that leaves that many resident. An instance goes
+// to the first class whose threads reach its columns and rows (or are kBT) and
+// whose shared memory holds it; the last class takes the rest.
+struct BatchClass {
+    int threads, ctas;  // threads: without the decision warp
+    size_t smem;
+};
+constexpr int kClasses = 4;
+constexpr BatchClass kClass[kClasses] = {
+    {128, 6, 36 * 1024}, {256, 4, 55 * 1024}, {512, 2, 112 * 1024}, {512, 1, 226 * 1024}};
+
+size_t held_bytes(const BatchDesc& d, int mode) {
+    return kSharedHead +
+           (mode == kHeldOut ? 0 : matrix_bytes(d) + (mode == kHeldAll ? state_bytes(d) : 0));
+}
+
+// Rows by decreasing length into `order` (counting sort, stable), and the
+// first staged entry of each slice of 32 (then the total), in units of 32,
+// onto `bases`; returns the entries.
+long long sort_slices(const std::vector<int>& len, int* order, std::vector<int>& bases) {
+    const int rows = (int)len.size();
+    int longest = 0;
+    for (int l : len) longest = std::max(longest, l);
+    std::vector<int> start(longest + 2, 0);
+    for (int l : len) ++start[longest - l + 1];
+    for (int k = 0; k <= longest; ++k) start[k + 1] += start[k];
+    for (int r = 0; r < rows; ++r) order[start[longest - len[r]]++] = r;
+    int run = 0;
+    for (int q = 0; q < rows; q += 32) {
+        bases.push_back(run);
+        run += len[order[q]];
+    }
+    bases.push_back(run);
+    return 32LL * run;
+}
+
+template <int K>
+__global__ void __launch_bounds__(kClass[K].threads + 32, kClass[K].ctas)
+    k_batch(const __grid_constant__ BatchArgs a) {
+    BatchShared& sh = b_shared();
     for (;;) {
         if (threadIdx.x == 0) sh.inst = (int)atomicAdd(a.queue, 1u);
         __syncthreads();
@@ -720,8 +1225,13 @@ __global__ void __launch_bounds__(kBT) k_batch(BatchArgs a) {
         __syncthreads();
         if (qi >= a.count) break;
         const int b = a.order[qi];
-        const BatchDesc d = a.desc[b];
-        if (d.m > 0 && d.n > 0) solve_one(a, sh, d, b);
+        if (a.desc[b].m <= 0 || a.desc[b].n <= 0) continue;
+        const int mode = a.desc[b].mode;
+        if (K < kClasses - 1 || mode == kHeldAll) solve_one<kHeldAll>(a, b);
+        else if constexpr (K == kClasses - 1) {
+            if (mode == kHeldMatrix) solve_one<kHeldMatrix>(a, b);
+            else solve_one<kHeldOut>(a, b);
+        }
     }
 }
 
@@ -800,6 +1310,45 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             return (long long)desc[p1].nnz + desc[p1].m + desc[p1].n >
                    (long long)desc[p2].nnz + desc[p2].m + desc[p2].n;
         });
+        // sorted slices of every instance's columns and rows
+        std::vector<int> order_c(cols), order_r(rows), bases, len;
+        long long out_off = 0;
+        for (int b = 0; b < count; ++b) {
+            BatchDesc& d = desc[b];
+            d.base_off = (long long)bases.size();
+            len.assign(d.n, 0);
+            for (int p = 0; p < d.nnz; ++p) ++len[ai[d.nz_off + p]];
+            d.pad_c = sort_slices(len, order_c.data() + d.col_off, bases);
+            len.resize(d.m);
+            for (int i = 0; i < d.m; ++i) len[i] = ap[d.ap_off + i + 1] - ap[d.ap_off + i];
+            d.pad_r = sort_slices(len, order_r.data() + d.row_off, bases);
+        }
+        // classes, each in that order
+        std::vector<int> cls_of(count), cls_order;
+        int cls_count[kClasses] = {}, cls_first[kClasses] = {};
+        size_t cls_smem[kClasses] = {};
+        for (int b = 0; b < count; ++b) {
+            BatchDesc& d = desc[b];
+            const int reach = std::max(d.m, d.n);
+            int k = 0;
+            d.mode = kHeldAll;
+            while (k < kClasses - 1 && ((reach > kClass[k].threads && kClass[k].threads < kBT) ||
+                                        held_bytes(d, kHeldAll) > kClass[k].smem))
+                ++k;
+            while (held_bytes(d, d.mode) > kClass[k].smem) --d.mode;
+            if (d.mode == kHeldOut) {
+                d.out_off = out_off;
+                out_off += d.pad_c + d.pad_r;
+            }
+            cls_of[b] = k;
+            cls_smem[k] = std::max(cls_smem[k], held_bytes(d, d.mode));
+        }
+        for (int k = kClasses - 1; k >= 0; --k) {
+            cls_first[k] = (int)cls_order.size();
+            for (int b : order)
+                if (cls_of[b] == k) cls_order.push_back(b);
+            cls_count[k] = (int)cls_order.size() - cls_first[k];
+        }
         std::vector<float> fac(2 * kFacTab);
         for (int k = 0; k < kFacTab; ++k) {
             const double kk = k < 1 ? 1.0 : (double)k;
@@ -820,11 +1369,10 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             return dp;
         };
         BatchArgs A{};
-        A.count = count;
-        A.order = up(order.data(), order.size());
+        const int* d_order = up(cls_order.data(), cls_order.size());
         A.desc = up(desc.data(), desc.size());
-        A.queue = ar.alloc<unsigned int>(1);
-        CU(cudaMemsetAsync(A.queue, 0, sizeof(unsigned int), st));
+        unsigned int* queue = ar.alloc<unsigned int>(kClasses);
+        CU(cudaMemsetAsync(queue, 0, kClasses * sizeof(unsigned int), st));
         A.ap = up(ap, (size_t)ap_off);
         A.ai = up(ai, (size_t)nz);
         double* axd = up(ax, (size_t)nz);
@@ -845,14 +1393,19 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         A.sax = ar.alloc<float>(nz);
         A.scax = ar.alloc<float>(nz);
         float** colv[] = {&A.dc, &A.sc, &A.scl, &A.scu, &A.x[0], &A.x[1], &A.xa[0], &A.xa[1],
-                          &A.xbar, &A.vt};
+                          &A.xbar, &A.vt, &A.g[0], &A.g[1]};
+        A.order_c = up(order_c.data(), order_c.size());
+        A.order_r = up(order_r.data(), order_r.size());
+        A.bases = up(bases.data(), bases.size());
+        A.out_val = ar.alloc<float>(out_off);
+        A.out_idx = ar.alloc<int>(out_off);
         for (float** v : colv) *v = ar.alloc<float>(cols);
         float** rowv[] = {&A.dr, &A.srmin, &A.srmax, &A.yh32, &A.y[0], &A.y[1], &A.ya[0],
-                          &A.ya[1], &A.axc[0], &A.axc[1], &A.mt};
+                          &A.ya[1], &A.axc[0], &A.axc[1], &A.mt, &A.ab};
         for (float** v : rowv) *v = ar.alloc<float>(rows);
-        double** col64[] = {&A.xh, &A.pesx, &A.atyh};
+        double** col64[] = {&A.xh, &A.pesx, &A.atyh, &A.rdc};
         for (double** v : col64) *v = ar.alloc<double>(cols);
-        double** row64[] = {&A.yh, &A.pesy, &A.axh};
+        double** row64[] = {&A.yh, &A.pesy, &A.axh, &A.rdr};
         for (double** v : row64) *v = ar.alloc<double>(rows);
         A.fac = up(fac.data(), fac.size());
         A.tol = o.tolerance;
@@ -875,18 +1428,55 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         A.x_out = ar.alloc<double>(cols);
         A.y_out = ar.alloc<double>(rows);
         A.out = ar.alloc<BatchOut>(count);
-        int sms = 0, dev = 0, per_sm = 0;
+        int sms = 0, dev = 0;
         CU(cudaGetDevice(&dev));
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, kBT, 0));
-        const int grid = std::max(1, std::min(count, sms * std::max(1, per_sm)));
-        cudaEvent_t e0, e1;
-        CU(cudaEventCreate(&e0));
-        CU(cudaEventCreate(&e1));
-        CU(cudaEventRecord(e0, st));
-        k_batch<<<grid, kBT, 0, st>>>(A);
-        CU(cudaGetLastError());
-        CU(cudaEventRecord(e1, st));
+        // one persistent launch per class, the largest instances' first; the
+        // others beside it on their own streams, taking the SMs it leaves
+        struct Fork {
+            cudaStream_t s[kClasses] = {};
+            cudaEvent_t e[kClasses + 2] = {};
+            ~Fork() {
+                for (auto& v : s)
+                    if (v) cudaStreamDestroy(v);
+                for (auto& v : e)
+                    if (v) cudaEventDestroy(v);
+            }
+        } fk;
+        CU(cudaEventCreate(&fk.e[kClasses]));
+        CU(cudaEventCreate(&fk.e[kClasses + 1]));
+        CU(cudaEventRecord(fk.e[kClasses], st));
+        void (*const kernels[kClasses])(BatchArgs) = {k_batch<0>, k_batch<1>, k_batch<2>, k_batch<3>};
+        bool first = true;
+        for (int k = kClasses - 1; k >= 0; --k) {
+            if (cls_count[k] == 0) continue;
+            cudaStream_t sk = st;
+            if (!first) {
+                CU(cudaStreamCreateWithFlags(&fk.s[k], cudaStreamNonBlocking));
+                sk = fk.s[k];
+                CU(cudaStreamWaitEvent(sk, fk.e[kClasses], 0));
+            }
+            const int threads = kClass[k].threads + 32;
+            int per_sm = 0;
+            CU(cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kClass[k].smem));
+            CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k], threads,
+                                                             cls_smem[k]));
+            BatchArgs Ak = A;
+            Ak.count = cls_count[k];
+            Ak.order = d_order + cls_first[k];
+            Ak.queue = queue + k;
+            const int grid = std::min(cls_count[k], sms * std::max(1, per_sm));
+            kernels[k]<<<grid, threads, cls_smem[k], sk>>>(Ak);
+            CU(cudaGetLastError());
+            if (!first) {
+                CU(cudaEventCreateWithFlags(&fk.e[k], cudaEventDisableTiming));
+                CU(cudaEventRecord(fk.e[k], sk));
+                CU(cudaStreamWaitEvent(st, fk.e[k], 0));
+            }
+            first = false;
+        }
+        CU(cudaEventRecord(fk.e[kClasses + 1], st));
         std::vector<BatchOut> out(count);
         CU(cudaMemcpyAsync(out.data(), A.out, sizeof(BatchOut) * count, cudaMemcpyDeviceToHost, st));
         std::vector<double> xk, yk;  // the launch's answers when the caller wants none
@@ -902,9 +1492,7 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         CU(cudaMemcpyAsync(y, A.y_out, sizeof(double) * rows, cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
         float kms = 0.f;
-        CU(cudaEventElapsedTime(&kms, e0, e1));
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        CU(cudaEventElapsedTime(&kms, fk.e[kClasses], fk.e[kClasses + 1]));
         // Instances the launch handed off or left at the cap are solved again,
         // alone, by the single-LP engine in FP64 through the public entry
         // points, from the launch's answer (igaos_pdhg_set_start), with the
