@@ -294,16 +294,16 @@ __global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallTh
             }
         }
         cluster_barrier();
-        if (rank == 0 && threadIdx.x == 0) {
+        if (rank == 0 && threadIdx.x < 32) {
+            const StepState st = load_step(&sctl, sfac, da.n_fac < kFacEntries ? da.n_fac : kFacEntries);
             Acc<T> s0, s1, s2;
             for (int i = 0; i < nr; ++i) {
                 s0.merge(spart[0][i]);
                 s1.merge(spart[1][i]);
                 s2.merge(spart[2][i]);
             }
-            decide_step(&sctl, s0.result_d(), s1.result_d(), s2.result_d(), sfac,
-                        da.n_fac < kFacEntries ? da.n_fac : kFacEntries);
-            publish();
+            decide_step(&sctl, st, s0.result_d(), s1.result_d(), s2.result_d());
+            if (threadIdx.x == 0) publish();
         }
         cluster_barrier();
     }

@@ -138,6 +138,7 @@ struct DevCtl {
     // correctly rounded 1/sigma in each precision (the dual step's quotient,
     // see DualEpi in kernels.cuh)
     double isigma;
+    double iomega;  // correctly rounded 1/omega (the step decision's quotients)
 };
 
 __host__ __device__ inline void ctl_derive(DevCtl* c) {
@@ -149,6 +150,7 @@ __host__ __device__ inline void ctl_derive(DevCtl* c) {
     c->w_f = (float)c->w;
     c->isigma = 1.0 / c->sigma;
     c->isigma_f = 1.0f / c->sigma_f;
+    c->iomega = 1.0 / c->omega;
 }
 
 // FP64 KKT metrics of one candidate (see k_kkt_* in kernels.cuh).
@@ -572,26 +574,41 @@ __device__ __forceinline__ void warp_item(const WarpSched& ws, const Csr<T>& A,
 #ifndef IGX_ITEM_PREFETCH
 #define IGX_ITEM_PREFETCH 1
 #endif
+
+// A warp's first item: rows [r0, r1), 2^lg lanes per row, the lane's row's
+// entries [b, e); r1 = 0 where the schedule has none for it.
+struct FirstItem {
+    int r0 = 0, r1 = 0, lg = 0, b = 0, e = 0;
+};
+template <typename T>
+__device__ __forceinline__ FirstItem first_item(const WarpSched& ws, const Csr<T>& A) {
+    FirstItem f;
+    const int w = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (w >= ws.nwarps) return f;
+    f.r0 = __ldg(ws.row + w);
+    f.r1 = __ldg(ws.row + w + 1);
+    f.lg = __ldg(ws.lg + w);
+    const int r = f.r0 + ((threadIdx.x & 31) >> f.lg);
+    if (r < f.r1) {
+        f.b = __ldg(A.ptr + r);
+        f.e = __ldg(A.ptr + r + 1);
+    }
+    return f;
+}
+
+// The items of this warp, from its first.
 template <typename T, class E>
-__device__ __forceinline__ void warp_rows_all(const WarpSched& ws, const Csr<T>& A,
-                                              const T* __restrict__ x, E& epi) {
-    const int stride = gridDim.x * kWarps;
-#if IGX_ITEM_PREFETCH
+__device__ __forceinline__ void warp_rows_from(const WarpSched& ws, const Csr<T>& A,
+                                               const T* __restrict__ x, E& epi,
+                                               const FirstItem& f) {
     // software-pipelined: the next item's schedule entries are loaded when
     // this item starts, and its row pointers between this item's products
     // and its reduction, so each item starts with [b, e) in registers
+    const int stride = gridDim.x * kWarps;
     const int lane = threadIdx.x & 31;
     int w = blockIdx.x * kWarps + (threadIdx.x >> 5);
     if (w >= ws.nwarps) return;
-    int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1), lg = __ldg(ws.lg + w);
-    int b = 0, e = 0;
-    {
-        const int r = r0 + (lane >> lg);
-        if (r < r1) {
-            b = __ldg(A.ptr + r);
-            e = __ldg(A.ptr + r + 1);
-        }
-    }
+    int r0 = f.r0, r1 = f.r1, lg = f.lg, b = f.b, e = f.e;
     for (;;) {
         const int wn = w + stride;
         const bool more = wn < ws.nwarps;
@@ -624,7 +641,15 @@ __device__ __forceinline__ void warp_rows_all(const WarpSched& ws, const Csr<T>&
         b = nb;
         e = ne;
     }
+}
+
+template <typename T, class E>
+__device__ __forceinline__ void warp_rows_all(const WarpSched& ws, const Csr<T>& A,
+                                              const T* __restrict__ x, E& epi) {
+#if IGX_ITEM_PREFETCH
+    warp_rows_from<T>(ws, A, x, epi, first_item<T>(ws, A));
 #else
+    const int stride = gridDim.x * kWarps;
     for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5); w < ws.nwarps; w += stride)
         warp_item<T>(ws, A, x, w, epi);
 #endif

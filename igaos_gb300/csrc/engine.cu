@@ -617,25 +617,34 @@ int Engine::grid_dual() const {
     if constexpr (std::is_same<T, double>::value) return occ_[0] == 4 ? sA_.ctas64w : sA_.ctas64;
     return sA_.ctas;
 }
+// An attempt kernel on the engine's stream, as a programmatic launch (it waits
+// for its predecessor itself, see follow_previous).
+template <typename A>
+static void launch_following(void (*kernel)(A), int grid, const A& args, cudaStream_t st) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU(cudaLaunchKernelEx(&cfg, kernel, args));
+}
 template <typename T>
 void Engine::launch_primal(const PrimalArgs<T>& pa) {
     const int gp = grid_primal<T>();
-    if constexpr (std::is_same<T, double>::value) {
-        if (occ_[1] == 4) k_primal<double, 4><<<gp, kThreads, 0, st_>>>(pa);
-        else k_primal<double, 3><<<gp, kThreads, 0, st_>>>(pa);
-    } else {
-        k_primal<T><<<gp, kThreads, 0, st_>>>(pa);
-    }
+    if constexpr (std::is_same<T, double>::value)
+        launch_following(occ_[1] == 4 ? k_primal<double, 4> : k_primal<double, 3>, gp, pa, st_);
+    else launch_following(k_primal<T>, gp, pa, st_);
 }
 template <typename T>
 void Engine::launch_dual(const DualArgs<T>& da) {
     const int gd = grid_dual<T>();
-    if constexpr (std::is_same<T, double>::value) {
-        if (occ_[0] == 4) k_dual<double, 4><<<gd, kThreads, 0, st_>>>(da);
-        else k_dual<double, 3><<<gd, kThreads, 0, st_>>>(da);
-    } else {
-        k_dual<T><<<gd, kThreads, 0, st_>>>(da);
-    }
+    if constexpr (std::is_same<T, double>::value)
+        launch_following(occ_[0] == 4 ? k_dual<double, 4> : k_dual<double, 3>, gd, da, st_);
+    else launch_following(k_dual<T>, gd, da, st_);
 }
 
 // Enqueues `count` line-search attempts (2 launches each). With graphs the

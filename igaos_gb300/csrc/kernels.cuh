@@ -51,6 +51,23 @@ __device__ __forceinline__ CtlView<float> read_ctl<float>(const DevCtl* c) {
                           c->isigma_f};
 }
 
+// The attempt kernels follow one another by programmatic launches: a kernel's
+// CTAs take their places as the last one's leave and wait here for its
+// results; in FP64 they first load what does not change (schedule, row
+// pointers; in FP32 that cost the large LPs more in registers than it gave).
+// A kernel lets the next one start when its products are done: from its
+// start on, waiting CTAs slowed FP32 attempts of large LPs by 8 %. 1,024 FP64
+// iterations of a 2,000 x 5,000 LP: 17.7 -> 15.7 ms; of an 8,000 x 20,000 LP in
+// FP32 16.1 -> 14.9; 256 of the 200,000 x 500,000 LP in FP64 28.6 -> 28.4.
+// (One resident launch per chunk with grid-wide barriers was slower than
+// either: 30.8 ms against 28.4 for 1,024 iterations of a 20,000 x 50,000 LP.)
+__device__ __forceinline__ void follow_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename T>
 struct PrimalArgs {
     WarpSched ws;
@@ -109,12 +126,17 @@ struct PrimalEpi {
 template <typename T, int OCC = HotCtas<T>::value>
 __global__ void __launch_bounds__(kThreads, OCC) k_primal(PrimalArgs<T> a) {
     __shared__ __align__(16) double smred[kWarps * 4];
+    FirstItem first;
+    if constexpr (sizeof(T) == 8) first = first_item<T>(a.ws, a.AT);
+    follow_previous();
     const CtlView<T> cv = read_ctl<T>(a.ctl);
     if (cv.stop) return;
+    if constexpr (sizeof(T) == 4) first = first_item<T>(a.ws, a.AT);
     const int p = cv.parity, q = p ^ 1;
     PrimalEpi<T> epi{a.c, a.lo, a.hi, a.x[p], a.xavg[p], a.x[q], a.xavg[q], a.xbar,
                      cv.tau, cv.w, (T)0};
-    warp_rows_all<T>(a.ws, a.AT, a.y[p], epi);
+    warp_rows_from<T>(a.ws, a.AT, a.y[p], epi, first);
+    let_next();
     const T dx2 = epi.dx2;
     T v[1] = {dx2};
     block_sum_t<T, 1>(v, reinterpret_cast<T*>(smred));
@@ -192,48 +214,147 @@ struct DualEpi {
     }
 };
 
-// Adaptive step decision (src/pdhg/pdhg.cu:770-794), one thread. Host-side
-// arithmetic of the reference has no FMA contraction; the explicit _rn
-// intrinsics keep it that way here.
-__device__ inline void decide_step(DevCtl* c, double dx2, double dy2, double cross,
-                                   const double* fac, int n_fac) {
+// a / b, correctly rounded, from ib = 1 / b correctly rounded: the product and
+// two remainder steps (Markstein 1990: the first leaves an error below an ulp,
+// the second rounds correctly). 300 cycles of latency, a division 575.
+// Operands far from 1 by hundreds of binades divide.
+__device__ __forceinline__ double div_exact(double a, double b, double ib) {
+    auto tame = [](double v) {
+        const int ex = (__double2hiint(v) >> 20) & 0x7ff;
+        return ex > 512 && ex < 1536;
+    };
+    if (!tame(a) || !tame(b)) return __ddiv_rn(a, b);
+    double q = __dmul_rn(a, ib);
+    q = fma(fma(-b, q, a), ib, q);
+    return fma(fma(-b, q, a), ib, q);
+}
+
+// What a step decision reads of the control block, loaded ahead of the dot
+// products it waits for (by every lane of the deciding warp).
+struct StepState {
+    double eta, omega, iomega, f_lo, f_hi;
+    long long k, hn;
+    int retries;
+};
+__device__ __forceinline__ StepState load_step(const DevCtl* c, const double* fac, int n_fac) {
+    StepState s;
+    s.eta = c->eta;
+    s.omega = c->omega;
+    s.iomega = c->iomega;
+    s.k = c->k;
+    s.hn = c->hn;
+    s.retries = c->retries;
+    // growth/shrink factors 1 - k^-0.3 and 1 + k^-0.6, tabulated by the host
+    // (std::pow, as the reference) for the iterations of this chunk
+    const long long fi = s.k - c->fac_base;
+    if (fac && fi >= 0 && fi < n_fac) {
+        s.f_lo = fac[2 * fi];
+        s.f_hi = fac[2 * fi + 1];
+    } else {
+        const double kk = (double)s.k;
+        s.f_lo = __dsub_rn(1.0, pow(kk, -0.3));
+        s.f_hi = __dadd_rn(1.0, pow(kk, -0.6));
+    }
+    return s;
+}
+
+// Adaptive step decision (src/pdhg/pdhg.cu:770-794) by one warp, every lane
+// with the same operands. Host-side arithmetic of the reference has no FMA
+// contraction; the explicit _rn intrinsics keep it that way here. The chain of
+// FP64 operations (60 cycles each, a comparison 100, a division 575) is the
+// serial part of every attempt: comparisons run on the integer pipe, quotients
+// by omega on its reciprocal, and the divisions that are left go side by side
+// in two lanes: etabar with the next averaging weight, then tau's with
+// 1/sigma. With six divisions in one thread, its loads behind the dot products
+// and FP64 comparisons, 1,024 FP64 iterations of a 60 x 150 LP took 17.5 ms,
+// now 16.0, and of a 2,000 x 5,000 LP 19.6, now 17.9.
+__device__ __forceinline__ void decide_step(DevCtl* c, const StepState& s, double dx2, double dy2,
+                                            double cross) {
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    auto nonneg_less = [](double a, double b) {  // a, b >= 0
+        return __double_as_longlong(a) < __double_as_longlong(b);
+    };
+    const double num = __dadd_rn(__dmul_rn(s.omega, dx2), div_exact(dy2, s.omega, s.iomega));
+    const bool sound = dfinite(dx2) && dfinite(dy2) && dfinite(cross);
+    const bool curved = sound && dfinite(num) && dgt0(num) && dgt0(cross);
+    // lane 0: etabar; lane 1: the weight 2 / (hn + 2) after an acceptance
+    const double den = lane == 1 ? (double)(s.hn + 1) + 2.0 : (curved ? __dmul_rn(2.0, cross) : 1.0);
+    const double quo = __ddiv_rn(lane == 1 ? 2.0 : num, den);
+    const double etabar = curved ? __shfl_sync(full, quo, 0) : CUDART_INF;
+    const double w_next = __shfl_sync(full, quo, 1);
+    double eta_new = CUDART_INF;
+    if (dfinite(etabar)) {
+        const double lo = __dmul_rn(s.f_lo, etabar), hi = __dmul_rn(s.f_hi, s.eta);
+        eta_new = nonneg_less(hi, lo) ? hi : lo;
+    }
+    const bool accept = !nonneg_less(etabar, s.eta) || s.retries >= 20;
+    const bool usable = dfinite(eta_new) && nonneg_less(1e-12, eta_new);
+    double eta = s.eta;
+    if (accept) {
+        if (usable) eta = nonneg_less(1e12, eta_new) ? 1e12 : eta_new;
+    } else {
+        eta = usable ? eta_new : 1e-12;
+    }
+    const double sigma = __dmul_rn(eta, s.omega);
+    // lane 0: tau; lane 1: 1 / sigma
+    const double out = __ddiv_rn(lane == 1 ? 1.0 : eta, lane == 1 ? sigma : s.omega);
+    const double isigma = __shfl_sync(full, out, 1);
+    if (lane != 0) return;
     c->dots[0] = dx2;
     c->dots[1] = dy2;
     c->dots[2] = cross;
-    if (!isfinite(dx2) || !isfinite(dy2) || !isfinite(cross)) c->nan_flag = 1;
-    const double eta = c->eta, omega = c->omega;
-    const double num = __dadd_rn(__dmul_rn(omega, dx2), __ddiv_rn(dy2, omega));
-    const double etabar =
-        (num > 0.0 && cross > 0.0) ? __ddiv_rn(num, __dmul_rn(2.0, cross)) : CUDART_INF;
-    // growth/shrink factors 1 - k^-0.3 and 1 + k^-0.6, tabulated by the host
-    // (std::pow, as the reference) for the iterations of this chunk
-    const long long fi = c->k - c->fac_base;
-    double f_lo, f_hi;
-    if (fac && fi >= 0 && fi < n_fac) {
-        f_lo = fac[2 * fi];
-        f_hi = fac[2 * fi + 1];
-    } else {
-        const double kk = (double)c->k;
-        f_lo = __dsub_rn(1.0, pow(kk, -0.3));
-        f_hi = __dadd_rn(1.0, pow(kk, -0.6));
-    }
-    double eta_new = CUDART_INF;
-    if (isfinite(etabar)) eta_new = smin(__dmul_rn(f_lo, etabar), __dmul_rn(f_hi, eta));
-    bool accept = !(eta > etabar) || num <= 0.0 || cross <= 0.0;
-    if (!accept) accept = ++c->retries > 20;
+    if (!sound) c->nan_flag = 1;
     c->attempts += 1;
+    c->eta = eta;
     if (accept) {
-        if (isfinite(eta_new) && eta_new > 1e-12) c->eta = smin(eta_new, 1e12);
         c->parity ^= 1;
-        c->hn += 1;
+        c->hn = s.hn + 1;
         c->accepted += 1;
         c->retries = 0;
-        if (c->k >= c->k_stop || c->nan_flag) c->stop = 1;
-        c->k += 1;
+        if (s.k >= c->k_stop || c->nan_flag) c->stop = 1;
+        c->k = s.k + 1;
+        c->w = w_next;
+        c->w_f = (float)w_next;
     } else {
-        c->eta = smax(eta_new, 1e-12);
+        c->retries = s.retries + 1;
     }
-    ctl_derive(c);
+    c->tau = out;
+    c->sigma = sigma;
+    c->tau_f = (float)out;
+    c->sigma_f = (float)sigma;
+    c->isigma = isigma;
+    c->isigma_f = 1.0f / (float)sigma;
+}
+
+// The attempt's end, by one CTA that sees every partial: their fixed-order
+// compensated merge (of n_primal and `gd` CTAs) and the step decision. A launch
+// of at most 32 CTAs has its partials in the first warp's lanes; the other
+// warps' zeros would change nothing.
+template <typename T>
+__device__ __forceinline__ void finish_attempt(const DualArgs<T>& a, int gd, double* smred) {
+    StepState st;
+    if (threadIdx.x < 32) st = load_step(a.ctl, a.fac, a.n_fac);
+    Acc<T> s[3];
+    for (int i = threadIdx.x; i < a.n_primal; i += kThreads) s[0].merge(a.part_primal[i]);
+    for (int i = threadIdx.x; i < gd; i += kThreads) {
+        s[1].merge(a.part[2 * i]);
+        s[2].merge(a.part[2 * i + 1]);
+    }
+    if (a.n_primal <= 32 && gd <= 32) {
+        if (threadIdx.x < 32)
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) s[q].shfl_xor(0xffffffffu, o, 32);
+    } else {
+        block_merge<T, 3>(s, reinterpret_cast<Acc<T>*>(smred));
+    }
+    if (threadIdx.x < 32) {
+        double d[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) d[q] = __shfl_sync(0xffffffffu, s[q].result_d(), 0);
+        decide_step(a.ctl, st, d[0], d[1], d[2]);
+    }
 }
 
 // Dual half of one attempt, fused into the A xbar SpMV:
@@ -246,12 +367,17 @@ __device__ inline void decide_step(DevCtl* c, double dx2, double dy2, double cro
 template <typename T, int OCC = HotCtas<T>::value>
 __global__ void __launch_bounds__(kThreads, OCC) k_dual(DualArgs<T> a) {
     __shared__ __align__(16) double smred[kWarps * 4];
+    FirstItem first;
+    if constexpr (sizeof(T) == 8) first = first_item<T>(a.ws, a.A);
+    follow_previous();
     const CtlView<T> cv = read_ctl<T>(a.ctl);
     if (cv.stop) return;
+    if constexpr (sizeof(T) == 4) first = first_item<T>(a.ws, a.A);
     const int p = cv.parity, q = p ^ 1;
     DualEpi<T> epi{a.rmin, a.rmax, a.y[p], a.axc[p], a.yavg[p], a.yhat, a.y[q], a.axc[q], a.yavg[q],
                    cv.sigma, cv.isigma, cv.w, (T)0, (T)0};
-    warp_rows_all<T>(a.ws, a.A, a.xbar, epi);
+    warp_rows_from<T>(a.ws, a.A, a.xbar, epi, first);
+    let_next();
     T v[2] = {epi.dy2, epi.cross};
     block_sum_t<T, 2>(v, reinterpret_cast<T*>(smred));
     if (threadIdx.x == 0) {
@@ -262,16 +388,7 @@ __global__ void __launch_bounds__(kThreads, OCC) k_dual(DualArgs<T> a) {
         a.part[2 * blockIdx.x + 1] = e1;
     }
     if (!last_cta(&a.ctl->ticket)) return;
-    // fixed-order compensated merge of all CTA partials
-    Acc<T> s[3];
-    for (int i = threadIdx.x; i < a.n_primal; i += kThreads) s[0].merge(a.part_primal[i]);
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += kThreads) {
-        s[1].merge(a.part[2 * i]);
-        s[2].merge(a.part[2 * i + 1]);
-    }
-    block_merge<T, 3>(s, reinterpret_cast<Acc<T>*>(smred));
-    if (threadIdx.x == 0)
-        decide_step(a.ctl, s[0].result_d(), s[1].result_d(), s[2].result_d(), a.fac, a.n_fac);
+    finish_attempt(a, gridDim.x, smred);
 }
 
 // ------------------------------------------------------------- plain SpMV
