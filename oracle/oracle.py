@@ -28,10 +28,10 @@ STAGED = os.path.join(HERE, "_ref", "src")
 
 def reference_dir():
     """The reference tree: $IGAOS_REFERENCE_DIR, else a `reference` directory
-    beside the repository; None when neither exists."""
+    beside the repository; None when neither holds the sources."""
     d = os.environ.get("IGAOS_REFERENCE_DIR") or os.path.join(
         os.path.dirname(os.path.dirname(HERE)), "reference")
-    return d if os.path.isdir(d) else None
+    return d if os.path.isfile(os.path.join(d, "src", "pdhg", "pdhg.cu")) else None
 
 
 def build(ref: bool = False) -> None:
