@@ -1,52 +1,48 @@
 // Small LPs: the line-search attempts of a chunk in one thread-block cluster.
 //
-// For an LP whose warp schedules give each warp of one cluster a few items,
-// an attempt is a few microseconds of work and the grid-wide kernels spend
-// it on launch latency and chains of dependent L2 loads (schedule -> row
-// pointer -> entries -> gathers). One cluster of kSmallCluster CTAs instead
-// runs the whole chunk in one launch, with the LP held on chip:
-//   * each CTA stages its warps' rows of A~ and A~^T (row pointers, indices,
-//     values) in shared memory once per launch;
-//   * every CTA keeps a replica of the two gathered vectors (xbar and both
-//     parity slots of y) in its shared memory; the PDHG step of a row writes
-//     its new entry to every CTA's replica through distributed shared memory
-//     (and to global memory for the host-side KKT checks);
+// For an LP of a few thousand rows and columns an attempt is a microsecond of
+// work, and the grid-wide kernels spend ten and more on launches, on chains of
+// dependent L2 loads (schedule -> row pointer -> entries -> gathers ->
+// partials) and on the step decision. One cluster of C CTAs (1 to 16) instead
+// runs the whole chunk in one launch, with the LP and its iterates on chip:
+//   * each CTA stages its rows of A~ and A~^T (row pointers, 16-bit indices,
+//     values) and their vectors (both parity slots of the iterates, bounds,
+//     costs) in shared memory once per launch, and writes the accepted
+//     iterates back at its end;
+//   * every CTA keeps a replica of the gathered vectors (xbar and both parity
+//     slots of y); the step of a row writes its new entry to every CTA's
+//     through distributed shared memory, and so go the partial sums;
 //   * per attempt: primal half, cluster barrier, dual half, cluster barrier,
-//     step decision by rank 0 (fixed-order merge of the per-CTA partials, the
-//     same decide_step), cluster barrier.
-// The control block, its step-factor table and the per-CTA partials stay in
-// rank 0's shared memory for the launch (rank 0 writes the block back at the
-// end). A warp keeps the same items for the whole launch, so its epilogue
-// reads of its own rows see its own earlier global writes.
+//     then every CTA takes the same step decision (decide_step) in a warp of
+//     its own from the same partials, while its other warps form A~^T y' of
+//     the dual just computed: the next attempt starts from it if the step is
+//     accepted (else from the accepted dual's, which is kept).
+// The sums are those of the kernel each precision would otherwise run, bit for
+// bit, whatever C: work is dealt in virtual warps (below) and their partials
+// are merged in the same order.
 #pragma once
 
 #include <cooperative_groups.h>
 
 #include <type_traits>
 
+#include "engine.hpp"
 #include "kernels.cuh"
 
 namespace igx {
 
-constexpr int kSmallCluster = 8;
-constexpr int kSmallThreads = 512;
-constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr int kSmallItems = 8;  // warp items per warp at most
-constexpr size_t kSmallSmemMax = 200 * 1024;  // dynamic shared memory per CTA
-constexpr int kFacEntries = 512;                // step-factor table entries staged
-
-// Dynamic shared memory of one CTA (bytes) for a rank's staged rows.
-struct SmallLayout {
-    long long ent_at, rows_at, ent_a, rows_a;  // staged entries / row pointers
-};
-__host__ __device__ inline size_t small_smem_bytes(int m, int n, const SmallLayout& L, int s) {
-    size_t b = (size_t)(n + 2 * (size_t)m) * s;                  // replicas
-    b = (b + 15) & ~(size_t)15;
-    b += (size_t)(L.ent_at + L.ent_a) * s;                       // values
-    b = (b + 15) & ~(size_t)15;
-    b += (size_t)(L.ent_at + L.ent_a) * 4 + (size_t)(L.rows_at + L.rows_a) * 4;
-    return b + 64;
-}
+constexpr int kSmallCluster = 16;       // most CTAs
+constexpr int kSmallWarps = 16;         // warps of a CTA that own rows
+constexpr int kSmallThreads = 32 * (kSmallWarps + 3);  // and the decision's three
+constexpr size_t kSmallSmemMax = 222 * 1024;  // dynamic shared memory per CTA
+// FP32: a virtual warp v < kSmallVirtual takes the schedule's items v, v +
+// kSmallVirtual, ..., at most kSmallItems of them; its lanes' sums run over
+// them. Sixteen virtual warps make a partial, eight partials the total.
+constexpr int kSmallVirtual = 128;
+constexpr int kSmallItems = 8;
+// FP64: a virtual warp is an item; eight make a partial, as in a CTA of the
+// grid-wide kernels, and the partials merge as finish_attempt merges them.
+constexpr int kSmallMaxItems = kSmallVirtual * kSmallItems;
 
 __device__ __forceinline__ int cluster_rank() {
     unsigned r;
@@ -60,82 +56,52 @@ __device__ __forceinline__ int cluster_count() {
 }
 // all threads of every CTA of the cluster; release/acquire at cluster scope
 // (global and distributed shared memory)
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-
-// One schedule's rows as staged by a CTA: entries and row pointers in
-// shared memory (row pointers are local entry offsets), the warp's item
-// descriptors {first row, end row, log2 G, first local row pointer}.
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// v into the entry `at` (an address in this CTA's replica) of every CTA's
 template <typename T>
-struct Staged {
-    const int* ptr;
-    const int* idx;
-    const T* val;
-};
+__device__ __forceinline__ void cluster_put(T* at, T v, int ctas) {
+    if (ctas == 1) {
+        *at = v;
+        return;
+    }
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    for (int r = 0; r < ctas; ++r) *cl.map_shared_rank(at, r) = v;
+}
 
 // Writes a row's new entry into the same slot of every CTA's replica.
 template <typename T>
 struct ClusterBcast {
     T* base;  // this CTA's replica
-    int nr;
-    __device__ __forceinline__ void operator()(int i, T v) const {
-        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-        for (int r = 0; r < nr; ++r) *cl.map_shared_rank(base + i, r) = v;
-    }
+    int ctas;
+    __device__ __forceinline__ void operator()(int i, T v) const { cluster_put(base + i, v, ctas); }
 };
 
-// Entries and row-pointer slots of the items w0, w0 + stride, ... of a
-// schedule (one warp's share), counted the same way by the host to size the
-// shared memory.
+// One orientation as staged by a CTA: entries and row pointers (local entry
+// offsets) in shared memory, an item being {first row, rows, log2 G, first
+// row pointer}.
 template <typename T>
-__device__ __forceinline__ int2 stage_count(const WarpSched& ws, const Csr<T>& A, int w0,
-                                            int stride) {
-    int2 c{0, 0};
-    for (int w = w0; w < ws.nwarps; w += stride) {
-        const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
-        c.x += __ldg(A.ptr + r1) - __ldg(A.ptr + r0);
-        c.y += r1 - r0 + 1;
-    }
-    return c;
-}
+struct Staged {
+    const int* ptr;
+    const uint16_t* idx;
+    const T* val;
+    const int4* item;
+};
 
-// The warp copies its items' row pointers (rebased to its local entry
-// offsets), indices and values into shared memory and records one
-// descriptor {r0, r1, log2 G, first row-pointer slot} per item.
+// lane sums of one staged item, reduced and handed to the lanes of its rows
+// (the sums and their order are those of lane_products and reduce_rows)
 template <typename T>
-__device__ __forceinline__ int stage_rows(const WarpSched& ws, const Csr<T>& A, int w0, int stride,
-                                          int ent0, int row0, int* sptr, int* sidx, T* sval,
-                                          int4* desc) {
+__device__ __forceinline__ Acc<T> staged_sums(const int4 d, const Staged<T>& S,
+                                              const T* __restrict__ sx) {
     const int lane = threadIdx.x & 31;
-    int k = 0, ce = ent0, cp = row0;
-    for (int w = w0; w < ws.nwarps; w += stride, ++k) {
-        const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
-        const int e0 = __ldg(A.ptr + r0), e1 = __ldg(A.ptr + r1);
-        for (int t = lane; t <= r1 - r0; t += 32) sptr[cp + t] = __ldg(A.ptr + r0 + t) - e0 + ce;
-        for (int q = lane; q < e1 - e0; q += 32) {
-            sidx[ce + q] = __ldg(A.idx + e0 + q);
-            sval[ce + q] = __ldg(A.val + e0 + q);
-        }
-        if (lane == 0) desc[k] = make_int4(r0, r1, __ldg(ws.lg + w), cp);
-        cp += r1 - r0 + 1;
-        ce += e1 - e0;
-    }
-    return k;
-}
-
-// warp_item on staged rows, x gathered from a shared-memory replica.
-template <typename T, class E>
-__device__ __forceinline__ void warp_item_staged(const int4 d, const Staged<T>& S,
-                                                 const T* __restrict__ sx, E& epi) {
-    const int lane = threadIdx.x & 31;
-    const int r0 = d.x, nr = d.y - d.x, lg = d.z, pb = d.w;
+    const int nr = d.y, lg = d.z, pb = d.w;
     const int G = 1 << lg;
     const int g = lane >> lg, gl = lane & (G - 1);
-    const bool has_epi = lane < (32 >> lg) && lane < nr;
-    typename E::Pre pre{};
-    if (has_epi) pre = epi.load(r0 + lane);
     Acc<T> acc;
     if (g < nr) {
         const int b = S.ptr[pb + g], e = S.ptr[pb + g + 1];
@@ -153,161 +119,438 @@ __device__ __forceinline__ void warp_item_staged(const int4 d, const Staged<T>& 
             for (int u = 0; u < kLaneBatch; ++u) acc.add(a[u], sx[j[u]]);
         }
     }
-    for (int o = G >> 1; o > 0; o >>= 1) acc.shfl_xor(0xffffffffu, o, G);
-    const Acc<T> mine = acc.shfl_from(0xffffffffu, (lane << lg) & 31);
-    if (has_epi) epi.apply(r0 + lane, mine, pre);
+    return reduce_rows<T>(acc, lg);
+}
+
+// Sum over a warp in the order of block_sum_t.
+template <typename T>
+__device__ __forceinline__ T lanes_sum(T v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The sums of a half's virtual warps lie padded with zeros to small_pad.
+template <typename T>
+__host__ __device__ inline int small_pad(int virt) {
+    return std::is_same<T, float>::value ? kSmallVirtual : (virt + 7) & ~7;
+}
+template <typename T>
+__host__ __device__ inline size_t small_bytes(int m, int n, const SmallPlan& p) {
+    size_t b = (size_t)(n + 2 * m) * sizeof(T);                                // replicas
+    b = (b + 15) & ~(size_t)15;
+    if (p.held) {
+        b += (size_t)p.cap.items_at * 32 * (7 * sizeof(T) + 2 * sizeof(Acc<T>));  // columns' vectors
+        b += (size_t)p.cap.items_a * 32 * 9 * sizeof(T);                          // rows' vectors
+    }
+    b += (size_t)2 * (small_pad<T>(p.virt_at) + small_pad<T>(p.virt_a)) * sizeof(T);  // partials
+    b += (size_t)p.cap.entries * sizeof(T);                                    // values
+    b = (b + 15) & ~(size_t)15;
+    b += (size_t)(p.cap.items_at + p.cap.items_a) * sizeof(int4);              // items
+    b += (size_t)p.cap.pointers * 4 + (size_t)p.cap.entries * 2;               // pointers, indices
+    return b + 32;
+}
+
+// FP32: the three totals, by one warp: partials of 16 virtual warps, plain
+// sums, each in a lane; eight of them merged, compensated.
+__device__ __forceinline__ void small_totals(const float* dx, const float* dy, const float* cr,
+                                             double* total) {
+    const int lane = threadIdx.x & 31, q = lane >> 3;
+    const float4* v = reinterpret_cast<const float4*>((q == 0 ? dx : q == 1 ? dy : cr) + 16 * (lane & 7));
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 f = v[k];
+        s = s + f.x;
+        s = s + f.y;
+        s = s + f.z;
+        s = s + f.w;
+    }
+    Acc<float> t;
+#pragma unroll
+    for (int r = 0; r < kSmallVirtual / 16; ++r) {
+        Acc<float> part;
+        part.s = __shfl_sync(0xffffffffu, s, (lane & 24) + r);
+        t.merge(part);
+    }
+    const double d = t.result_d();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) total[k] = __shfl_sync(0xffffffffu, d, 8 * k);
+}
+// FP64: one total by one warp (three warps side by side): partials of 8, 32
+// of them over the lanes (the levels of the tree that only add zeros left
+// out), groups of 32 in turn.
+__device__ __forceinline__ double small_total(const double* v, int pad) {
+    const int lane = threadIdx.x & 31;
+    double total = 0.0;
+    for (int g = 0; 256 * g < pad; ++g) {
+        const int k0 = 8 * (32 * g + lane);
+        double s = 0.0;
+        if (k0 < pad) {
+            const double2* a = reinterpret_cast<const double2*>(v + k0);
+            const double2 b0 = a[0], b1 = a[1], b2 = a[2], b3 = a[3];
+            s = b0.x + b0.y;
+            s = s + b1.x;
+            s = s + b1.y;
+            s = s + b2.x;
+            s = s + b2.y;
+            s = s + b3.x;
+            s = s + b3.y;
+        }
+        int o = 16;
+        if (pad < 256)
+            while (o && 8 * o >= pad) o >>= 1;
+        for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s = __shfl_sync(0xffffffffu, s, 0);
+        total = g == 0 ? s : total + s;
+    }
+    return total;
 }
 
 // The attempts of one chunk (up to max_attempts, until the control block's
-// stop flag), one cluster of kSmallCluster CTAs. Dynamic shared memory:
-// replicas xbar (n), y slot 0 (m), y slot 1 (m); then the staged values,
-// indices and row pointers of A~^T (primal half) and A~ (dual half).
-template <typename T>
-__global__ void __cluster_dims__(kSmallCluster, 1, 1) __launch_bounds__(kSmallThreads, 1)
-    k_attempts_cluster(PrimalArgs<T> pa, DualArgs<T> da, int m, int n, int max_attempts) {
+// stop flag). What an attempt costs is latency: the two barriers, and FP64
+// operations of one warp at 60 cycles and more each (its SMSP's unit takes a
+// warp through in 64), so only what the next half waits for stands before a
+// barrier's arrival: the averages and ||dx||^2 are formed behind it. 2,048 FP32
+// iterations of a 2,000 x 5,000 LP: 19.5 -> 14.8 ms (with one deciding CTA, its
+// answer published behind a third barrier, and the vectors in global memory).
+template <typename T, bool HELD>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+    k_attempts_cluster(PrimalArgs<T> pa, DualArgs<T> da, int m, int n, int max_attempts,
+                       SmallPlan plan) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ __align__(16) double smred[kSmallWarps * 4];
-    __shared__ int4 sdesc[2][kSmallWarps][kSmallItems];
-    __shared__ int scnt[2][kSmallWarps + 1][2];
-    __shared__ int snit[2][kSmallWarps];
-    // control block, step-factor table and partials live in rank 0's shared
-    // memory for the whole launch; every CTA holds the view of the step
-    // being attempted, written by rank 0 through distributed shared memory
-    __shared__ DevCtl sctl;
-    __shared__ double sfac[2 * kFacEntries];
-    __shared__ Acc<T> spart[3][kSmallCluster];
     __shared__ CtlView<T> sview;
-    const int rank = cluster_rank(), nr = cluster_count();
-    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    // rank 0 thread 0: the view of the next attempt into every CTA
-    auto publish = [&]() {
-        CtlView<T> v;
-        v.parity = sctl.parity;
-        v.stop = sctl.stop;
-        if constexpr (std::is_same<T, double>::value) {
-            v.tau = sctl.tau;
-            v.sigma = sctl.sigma;
-            v.w = sctl.w;
-            v.isigma = sctl.isigma;
-        } else {
-            v.tau = sctl.tau_f;
-            v.sigma = sctl.sigma_f;
-            v.w = sctl.w_f;
-            v.isigma = sctl.isigma_f;
-        }
-        for (int r = 0; r < nr; ++r) *cl.map_shared_rank(&sview, r) = v;
-    };
+    __shared__ double stotal[2];
+    __shared__ int scnt[2][kSmallWarps + 1][3];
+    const int rank = cluster_rank(), ctas = plan.ctas;
     const int wi = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-    const int w0 = rank * kSmallWarps + wi, stride = nr * kSmallWarps;
+    const bool owns = wi < kSmallWarps;
+    // warps of the SMSPs 1 to 3 first: the decision's runs on SMSP 0; the rows
+    // of A from the other end, off the warps that hold columns, if few
+    const int at_pos = (wi & 3) ? (wi >> 2) * 3 + (wi & 3) - 1 : 12 + (wi >> 2);
+    const int deal_step = kSmallWarps * ctas;
+    const int first_at = at_pos * ctas + rank;
+    const int first_a = (at_pos < 12 ? 11 - at_pos : at_pos) * ctas + rank;
 
-    // ---- layout: each warp's share of both schedules, prefix over warps
-    {
-        const int2 ca = stage_count<T>(pa.ws, pa.AT, w0, stride);
-        const int2 cd = stage_count<T>(da.ws, da.A, w0, stride);
-        if (lane == 0) {
-            scnt[0][wi + 1][0] = ca.x;
-            scnt[0][wi + 1][1] = ca.y;
-            scnt[1][wi + 1][0] = cd.x;
-            scnt[1][wi + 1][1] = cd.y;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < 2; ++s) {
-            scnt[s][0][0] = 0;
-            scnt[s][0][1] = 0;
-            for (int k = 1; k <= kSmallWarps; ++k) {
-                scnt[s][k][0] += scnt[s][k - 1][0];
-                scnt[s][k][1] += scnt[s][k - 1][1];
-            }
-        }
-    }
-    __syncthreads();
-    const int ent_at = scnt[0][kSmallWarps][0], ent_a = scnt[1][kSmallWarps][0];
-    const int rows_at = scnt[0][kSmallWarps][1];
+    // ---- carve
+    const int sat = HELD ? plan.cap.items_at * 32 : 0, sa = HELD ? plan.cap.items_a * 32 : 0;
+    const int pad_at = small_pad<T>(plan.virt_at), pad_a = small_pad<T>(plan.virt_a);
     T* sxbar = reinterpret_cast<T*>(smem);
     T* sy[2] = {sxbar + n, sxbar + n + m};
-    size_t off = ((size_t)(n + 2 * (size_t)m) * sizeof(T) + 15) & ~(size_t)15;
-    T* val_at = reinterpret_cast<T*>(smem + off);
-    T* val_a = val_at + ent_at;
-    off = (off + (size_t)(ent_at + ent_a) * sizeof(T) + 15) & ~(size_t)15;
-    int* idx_at = reinterpret_cast<int*>(smem + off);
-    int* idx_a = idx_at + ent_at;
-    int* ptr_at = idx_a + ent_a;
-    int* ptr_a = ptr_at + rows_at;
-    const int nit_at = stage_rows<T>(pa.ws, pa.AT, w0, stride, scnt[0][wi][0], scnt[0][wi][1],
-                                     ptr_at, idx_at, val_at, sdesc[0][wi]);
-    const int nit_a = stage_rows<T>(da.ws, da.A, w0, stride, scnt[1][wi][0], scnt[1][wi][1], ptr_a,
-                                    idx_a, val_a, sdesc[1][wi]);
-    if (lane == 0) {
-        snit[0][wi] = nit_at;
-        snit[1][wi] = nit_a;
-    }
-    if (rank == 0) {
-        for (int i = threadIdx.x; i < 2 * da.n_fac && i < 2 * kFacEntries; i += kSmallThreads)
-            sfac[i] = da.fac[i];
-        if (threadIdx.x == 0) sctl = *pa.ctl;
-    }
-    {  // replica of the current dual slot
-        const int p0 = __ldcg(&pa.ctl->parity);
-        const T* yg = pa.y[p0];
-        for (int i = threadIdx.x; i < m; i += kSmallThreads) sy[p0][i] = yg[i];
+    size_t off = ((size_t)(n + 2 * m) * sizeof(T) + 15) & ~(size_t)15;
+    Acc<T>* sg = reinterpret_cast<Acc<T>*>(smem + off);   // A~^T y of both slots
+    T* vat = reinterpret_cast<T*>(sg + 2 * sat);  // c, lo, hi, x[2], xavg[2]
+    T* va = vat + 7 * sat;                        // rmin, rmax, yhat, y[2], axc[2], yavg[2]
+    T* part_dx = va + 9 * sa;                     // of every other attempt
+    T *part_dy = part_dx + 2 * pad_at, *part_cr = part_dy + pad_a;
+    T* val = part_cr + pad_a;
+    off = (size_t)(reinterpret_cast<unsigned char*>(val + plan.cap.entries) - smem);
+    off = (off + 15) & ~(size_t)15;
+    int4* item = reinterpret_cast<int4*>(smem + off);
+    int* ptr = reinterpret_cast<int*>(item + plan.cap.items_at + plan.cap.items_a);
+    uint16_t* idx = reinterpret_cast<uint16_t*>(ptr + plan.cap.pointers);
+
+    // ---- each warp's share of both schedules: items, entries, row pointers
+    auto items_of = [&](int o, auto&& f) {  // every item of this warp, in order
+        const WarpSched& ws = o ? da.ws : pa.ws;
+        const int virt = o ? plan.virt_a : plan.virt_at;
+        for (int v = o ? first_a : first_at; v < virt; v += deal_step)
+            for (int w = v; w < ws.nwarps; w += virt) f(ws, w);
+    };
+    if (owns)
+        for (int o = 0; o < 2; ++o) {
+            const Csr<T>& A = o ? da.A : pa.AT;
+            int c = 0, e = 0, r = 0;
+            items_of(o, [&](const WarpSched& ws, int w) {
+                const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
+                ++c;
+                e += __ldg(A.ptr + r1) - __ldg(A.ptr + r0);
+                r += r1 - r0 + 1;
+            });
+            if (lane == 0) {
+                scnt[o][wi + 1][0] = c;
+                scnt[o][wi + 1][1] = e;
+                scnt[o][wi + 1][2] = r;
+            }
+        }
+    for (int i = threadIdx.x; i < 2 * (pad_at + pad_a); i += kSmallThreads) part_dx[i] = T(0);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        int run = 0;  // rows of A after those of A~^T, in one sequence
+        for (int o = 0; o < 2; ++o) {
+            scnt[o][0][threadIdx.x] = run;
+            for (int k = 1; k <= kSmallWarps; ++k) run = scnt[o][k][threadIdx.x] += run;
+        }
     }
     __syncthreads();
-    cluster_barrier();  // every CTA running and staged before any remote write
-    if (rank == 0 && threadIdx.x == 0) publish();
-    cluster_barrier();
-    const Staged<T> st_at{ptr_at, idx_at, val_at}, st_a{ptr_a, idx_a, val_a};
-
-    for (int att = 0; att < max_attempts; ++att) {
-        const CtlView<T> cv = sview;
-        if (cv.stop) break;  // the same value in every CTA: published before the same barrier
-        const int p = cv.parity, q = p ^ 1;
-        {
-            PrimalEpi<T, ClusterBcast<T>> epi{pa.c,    pa.lo,   pa.hi,  pa.x[p], pa.xavg[p],
-                                              pa.x[q], pa.xavg[q], pa.xbar, cv.tau, cv.w,
-                                              (T)0,    ClusterBcast<T>{sxbar, nr}};
-            for (int k = 0; k < snit[0][wi]; ++k) warp_item_staged<T>(sdesc[0][wi][k], st_at, sy[p], epi);
-            T v[1] = {epi.dx2};
-            block_sum_t<T, 1, kSmallWarps>(v, reinterpret_cast<T*>(smred));
-            if (threadIdx.x == 0) {
-                Acc<T> e;
-                e.s = v[0];
-                *cl.map_shared_rank(&spart[0][rank], 0) = e;
-            }
+    const int p0 = __ldcg(&pa.ctl->parity);
+    const int items_at = scnt[1][0][0];  // of this CTA
+    const int it0 = owns ? scnt[0][wi][0] : 0, it1 = owns ? scnt[1][wi][0] : 0;
+    if (owns)
+        for (int o = 0; o < 2; ++o) {
+            const Csr<T>& A = o ? da.A : pa.AT;
+            int k = scnt[o][wi][0], ce = scnt[o][wi][1], cp = scnt[o][wi][2];
+            items_of(o, [&](const WarpSched& ws, int w) {
+                const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
+                const int e0 = __ldg(A.ptr + r0), e1 = __ldg(A.ptr + r1);
+                for (int t = lane; t <= r1 - r0; t += 32) ptr[cp + t] = __ldg(A.ptr + r0 + t) - e0 + ce;
+                for (int q = lane; q < e1 - e0; q += 32) {
+                    idx[ce + q] = (uint16_t)__ldg(A.idx + e0 + q);
+                    val[ce + q] = __ldg(A.val + e0 + q);
+                }
+                if (lane == 0) item[k] = make_int4(r0, r1 - r0, __ldg(ws.lg + w), cp);
+                const int i = r0 + lane;
+                if (HELD && lane < r1 - r0) {
+                    if (o == 0) {
+                        T* v = vat + 32 * k + lane;
+                        v[0] = __ldg(pa.c + i);
+                        v[sat] = __ldg(pa.lo + i);
+                        v[2 * sat] = __ldg(pa.hi + i);
+                        v[(3 + p0) * sat] = pa.x[p0][i];
+                        v[(5 + p0) * sat] = pa.xavg[p0][i];
+                    } else {
+                        T* v = va + 32 * (k - items_at) + lane;
+                        v[0] = __ldg(da.rmin + i);
+                        v[sa] = __ldg(da.rmax + i);
+                        v[2 * sa] = da.yhat ? __ldg(da.yhat + i) : T(0);
+                        v[(3 + p0) * sa] = da.y[p0][i];
+                        v[(5 + p0) * sa] = da.axc[p0][i];
+                        v[(7 + p0) * sa] = da.yavg[p0][i];
+                    }
+                }
+                cp += r1 - r0 + 1;
+                ce += e1 - e0;
+                ++k;
+            });
         }
-        cluster_barrier();
-        {
-            DualEpi<T, ClusterBcast<T>> epi{da.rmin,    da.rmax, da.y[p],  da.axc[p], da.yavg[p],
-                                            da.yhat,    da.y[q], da.axc[q], da.yavg[q], cv.sigma,
-                                            cv.isigma,  cv.w,    (T)0,     (T)0,
-                                            ClusterBcast<T>{sy[q], nr}};
-            for (int k = 0; k < snit[1][wi]; ++k) warp_item_staged<T>(sdesc[1][wi][k], st_a, sxbar, epi);
-            T v[2] = {epi.dy2, epi.cross};
-            block_sum_t<T, 2, kSmallWarps>(v, reinterpret_cast<T*>(smred));
-            if (threadIdx.x == 0) {
-                Acc<T> e0, e1;
-                e0.s = v[0];
-                e1.s = v[1];
-                *cl.map_shared_rank(&spart[1][rank], 0) = e0;
-                *cl.map_shared_rank(&spart[2][rank], 0) = e1;
-            }
-        }
-        cluster_barrier();
-        if (rank == 0 && threadIdx.x < 32) {
-            const StepState st = load_step(&sctl, sfac, da.n_fac < kFacEntries ? da.n_fac : kFacEntries);
-            Acc<T> s0, s1, s2;
-            for (int i = 0; i < nr; ++i) {
-                s0.merge(spart[0][i]);
-                s1.merge(spart[1][i]);
-                s2.merge(spart[2][i]);
-            }
-            decide_step(&sctl, st, s0.result_d(), s1.result_d(), s2.result_d());
-            if (threadIdx.x == 0) publish();
-        }
-        cluster_barrier();
+    for (int i = threadIdx.x; i < m; i += kSmallThreads) sy[p0][i] = pa.y[p0][i];
+    // the deciding warp's state (every lane's)
+    StepState st{};
+    long long attempts = 0, accepted = 0, k_stop = 0;
+    int nan_flag = 0;
+    double dots[3] = {0.0, 0.0, 0.0};
+    if (wi == kSmallWarps) {
+        st = load_step(pa.ctl, da.fac, da.n_fac);
+        k_stop = pa.ctl->k_stop;
+        nan_flag = pa.ctl->nan_flag;
+        if (lane == 0) sview = read_ctl<T>(pa.ctl);
     }
-    if (rank == 0 && threadIdx.x == 0) *pa.ctl = sctl;  // the host reads it after the launch
+    const long long fac_base = pa.ctl->fac_base;
+    __syncthreads();
+    const Staged<T> S{ptr, idx, val, item};
+    // A~^T y of slot q into sg, this warp's items
+    auto product_at = [&](int q) {
+        int k = it0;
+        items_of(0, [&](const WarpSched&, int) {
+            sg[q * sat + 32 * k + lane] = staged_sums<T>(item[k], S, sy[q]);
+            ++k;
+        });
+    };
+    if (HELD && owns) product_at(p0);
+    cluster_arrive();  // every CTA running and staged before any remote write
+    cluster_wait();
+
+    int att = 0;
+    for (; att < max_attempts; ++att) {
+        const CtlView<T> cv = sview;
+        if (cv.stop) break;  // the same in every CTA
+        const int p = cv.parity, q = p ^ 1;
+        T* dx_to = part_dx + (att & 1) * pad_at;  // other CTAs may still read the last ones
+        if (owns) {  // primal half
+            if constexpr (HELD) {
+                int k = it0;
+                for (int v = first_at; v < plan.virt_at; v += deal_step)
+                    for (int w = v; w < pa.ws.nwarps; w += plan.virt_at, ++k) {
+                        const int4 d = item[k];
+                        if (lane >= d.y) continue;
+                        T* z = vat + 32 * k + lane;
+                        const T x = z[(3 + p) * sat];
+                        const T g = z[0] + sg[p * sat + 32 * k + lane].result();
+                        const T xn = primal_step(cv.tau, g, x, z[sat], z[2 * sat]);
+                        z[(3 + q) * sat] = xn;
+                        cluster_put(sxbar + d.x + lane, fma((T)2, xn, -x), ctas);
+                    }
+            } else {
+                int k = it0;
+                PrimalEpi<T, ClusterBcast<T>> epi{pa.c,       pa.lo,      pa.hi,   pa.x[p], pa.xavg[p],
+                                                  pa.x[q],    pa.xavg[q], pa.xbar, cv.tau,  cv.w,
+                                                  T(0),       ClusterBcast<T>{sxbar, ctas}};
+                for (int v = first_at; v < plan.virt_at; v += deal_step) {
+                    epi.dx2 = T(0);
+                    for (int w = v; w < pa.ws.nwarps; w += plan.virt_at, ++k) {
+                        const int4 d = item[k];
+                        typename PrimalEpi<T, ClusterBcast<T>>::Pre pre{};
+                        if (lane < d.y) pre = epi.load(d.x + lane);
+                        const Acc<T> g = staged_sums<T>(d, S, sy[p]);
+                        if (lane < d.y) epi.apply(d.x + lane, g, pre);
+                    }
+                    const T dx2 = lanes_sum(epi.dx2);
+                    if (lane == 0) cluster_put(dx_to + v, dx2, ctas);
+                }
+            }
+        }
+        cluster_arrive();
+        if (HELD && owns) {  // ||dx||^2 and the average, for barriers to come
+            int k = it0;
+            for (int v = first_at; v < plan.virt_at; v += deal_step) {
+                T dx2 = T(0);
+                for (int w = v; w < pa.ws.nwarps; w += plan.virt_at, ++k) {
+                    if (lane >= item[k].y) continue;
+                    T* z = vat + 32 * k + lane;
+                    const T xn = z[(3 + q) * sat], xa = z[(5 + p) * sat];
+                    const T dx = xn - z[(3 + p) * sat];
+                    dx2 = fma(dx, dx, dx2);
+                    z[(5 + q) * sat] = fma(cv.w, xn - xa, xa);
+                }
+                __syncwarp();
+                dx2 = lanes_sum(dx2);
+                if (lane == 0) cluster_put(dx_to + v, dx2, ctas);
+            }
+        }
+        __syncwarp();
+        cluster_wait();
+        if (owns) {  // dual half
+            int k = it1;
+            DualEpi<T, ClusterBcast<T>> epi{da.rmin,    da.rmax,   da.y[p],    da.axc[p], da.yavg[p], da.yhat,
+                                            da.y[q],    da.axc[q], da.yavg[q], cv.sigma,  cv.isigma,
+                                            cv.w,       T(0),      T(0),       ClusterBcast<T>{sy[q], ctas}};
+            for (int v = first_a; v < plan.virt_a; v += deal_step) {
+                epi.dy2 = epi.cross = T(0);
+                for (int w = v; w < da.ws.nwarps; w += plan.virt_a, ++k) {
+                    const int4 d = item[k];
+                    if constexpr (HELD) {
+                        const T ab = staged_sums<T>(d, S, sxbar).result();
+                        if (lane >= d.y) continue;
+                        T* z = va + 32 * (k - items_at) + lane;
+                        const T y = z[(3 + p) * sa];
+                        const T yn = dual_step(cv.sigma, cv.isigma, ab, y, da.yhat != nullptr, z[2 * sa],
+                                               z[0], z[sa]);
+                        z[(3 + q) * sa] = yn;
+                        cluster_put(sy[q] + d.x + lane, yn, ctas);
+                        const T dy = yn - y;
+                        const T adx = (T)0.5 * (ab - z[(5 + p) * sa]);
+                        z[(5 + q) * sa] = adx;
+                        epi.dy2 = fma(dy, dy, epi.dy2);
+                        epi.cross = fma(dy, adx, epi.cross);
+                    } else {
+                        typename DualEpi<T, ClusterBcast<T>>::Pre pre{};
+                        if (lane < d.y) pre = epi.load(d.x + lane);
+                        const Acc<T> ab = staged_sums<T>(d, S, sxbar);
+                        if (lane < d.y) epi.apply(d.x + lane, ab, pre);
+                    }
+                }
+                __syncwarp();
+                const T dy2 = lanes_sum(epi.dy2), cross = lanes_sum(epi.cross);
+                if (lane == 0) {
+                    cluster_put(part_dy + v, dy2, ctas);
+                    cluster_put(part_cr + v, cross, ctas);
+                }
+            }
+        }
+        cluster_arrive();
+        if (HELD && owns) {
+            int k = it1;
+            items_of(1, [&](const WarpSched&, int) {
+                if (lane < item[k].y) {
+                    T* z = va + 32 * (k - items_at) + lane;
+                    z[(5 + q) * sa] = z[(5 + p) * sa] + z[(5 + q) * sa];
+                    const T ya = z[(7 + p) * sa];
+                    z[(7 + q) * sa] = fma(cv.w, z[(3 + q) * sa] - ya, ya);
+                }
+                ++k;
+            });
+        }
+        __syncwarp();
+        cluster_wait();
+        if (owns) {
+            if (HELD) product_at(q);
+        } else if (wi == kSmallWarps || sizeof(T) == 8) {
+            if constexpr (std::is_same<T, double>::value) {
+                const double t = wi == kSmallWarps       ? small_total(dx_to, pad_at)
+                                 : wi == kSmallWarps + 1 ? small_total(part_dy, pad_a)
+                                                         : small_total(part_cr, pad_a);
+                if (wi > kSmallWarps && lane == 0) stotal[wi - kSmallWarps - 1] = t;
+                asm volatile("bar.sync 1, 96;" ::: "memory");
+                dots[0] = t;
+                dots[1] = stotal[0];
+                dots[2] = stotal[1];
+            } else {
+                small_totals(dx_to, part_dy, part_cr, dots);
+            }
+            if (wi == kSmallWarps) {  // as decide_step
+                const StepOut o = step_rule(st, dots[0], dots[1], dots[2]);
+                const double sigma = __dmul_rn(o.eta, st.omega);
+                CtlView<T> nv = cv;
+                if constexpr (std::is_same<T, double>::value) {
+                    const double out = __ddiv_rn(lane == 1 ? 1.0 : o.eta, lane == 1 ? sigma : st.omega);
+                    nv.isigma = __shfl_sync(0xffffffffu, out, 1);
+                    nv.tau = out;
+                } else {
+                    nv.tau = (float)div_exact(o.eta, st.omega, st.iomega);
+                    nv.isigma = 1.0f / (float)sigma;
+                }
+                nv.sigma = (T)sigma;
+                if (!o.sound) nan_flag = 1;
+                if (o.accept) {
+                    nv.parity = q;
+                    nv.w = (T)o.w;
+                    nv.stop = st.k >= k_stop || nan_flag;
+                }
+                if (lane == 0) sview = nv;
+                st.eta = o.eta;
+                st.retries = o.accept ? 0 : st.retries + 1;
+                if (o.accept) {
+                    ++accepted;
+                    ++st.hn;
+                    ++st.k;
+                }
+                ++attempts;
+            }
+        }
+        __syncthreads();
+        if (wi == kSmallWarps)
+            step_factors(st, fac_base, da.fac, da.n_fac);  // of the next decision
+    }
+    // the accepted iterates, for the host's checks
+    const int p = sview.parity;
+    if (HELD && owns) {
+        int k = it0;
+        items_of(0, [&](const WarpSched&, int) {
+            const int4 d = item[k];
+            const T* z = vat + 32 * k + lane;
+            if (lane < d.y) {
+                pa.x[p][d.x + lane] = z[(3 + p) * sat];
+                pa.xavg[p][d.x + lane] = z[(5 + p) * sat];
+            }
+            ++k;
+        });
+        k = it1;
+        items_of(1, [&](const WarpSched&, int) {
+            const int4 d = item[k];
+            const T* z = va + 32 * (k - items_at) + lane;
+            if (lane < d.y) {
+                da.y[p][d.x + lane] = z[(3 + p) * sa];
+                da.axc[p][d.x + lane] = z[(5 + p) * sa];
+                da.yavg[p][d.x + lane] = z[(7 + p) * sa];
+            }
+            ++k;
+        });
+    }
+    cluster_arrive();  // no CTA leaves while another may still write to it
+    cluster_wait();    // (and every CTA has read the control block)
+    if (rank == 0 && wi == kSmallWarps && lane == 0 && attempts) {
+        DevCtl* c = pa.ctl;
+        for (int k = 0; k < 3; ++k) c->dots[k] = dots[k];
+        c->eta = st.eta;
+        c->k = st.k;
+        c->hn = st.hn;
+        c->attempts += attempts;
+        c->accepted += accepted;
+        c->retries = st.retries;
+        c->parity = p;
+        c->stop = sview.stop;
+        c->nan_flag = nan_flag;
+        ctl_derive(c);
+    }
 }
 
 }  // namespace igx

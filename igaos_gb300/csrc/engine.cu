@@ -70,48 +70,113 @@ void build_warps(const int* ptr, int rows, std::vector<int>& wrow, std::vector<u
     }
 }
 
-// Whether one cluster of the attempt kernel with `bytes` of dynamic shared
-// memory can be resident on this device (else the grid-wide kernels serve).
-static bool cluster_fits(bool f64, int bytes) {
-    const void* fn = f64 ? (const void*)k_attempts_cluster<double> : (const void*)k_attempts_cluster<float>;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+// One cluster of the attempt kernel: its launch configuration, and whether one
+// can be resident on this device (else the grid-wide kernels serve).
+static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* at, const SmallPlan& plan,
+                                         cudaStream_t st) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = plan.ctas;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kSmallCluster);
+    cfg.gridDim = dim3(plan.ctas);
     cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = bytes;
+    cfg.dynamicSmemBytes = plan.bytes;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+template <typename T>
+static bool cluster_fits(const SmallPlan& plan) {
+    const void* fn = plan.held ? (const void*)k_attempts_cluster<T, true>
+                               : (const void*)k_attempts_cluster<T, false>;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = cluster_config(at, plan, nullptr);
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmallSmemMax) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     return clusters > 0;
 }
 
-// Per-rank staged entries and row-pointer slots of a schedule for the cluster
-// attempt kernel (rank r's warps take items r * kSmallWarps + wi + k *
-// kSmallCluster * kSmallWarps); false when a warp would hold more than
-// kSmallItems items.
-static bool small_share(const int* ptr, int rows, std::vector<long long>& ent,
-                        std::vector<long long>& slots) {
-    // a warp item holds at most 32 rows: more rows than that many items hold
-    // cannot fit (no need to build the schedule to know)
-    if ((long long)rows > 32LL * kSmallCluster * kSmallWarps * kSmallItems) return false;
-    std::vector<int> wr;
-    std::vector<unsigned char> wl;
-    build_warps(ptr, rows, wr, wl);
-    const int nw = (int)wl.size(), stride = kSmallCluster * kSmallWarps;
-    if (nw > stride * kSmallItems) return false;
-    ent.assign(kSmallCluster, 0);
-    slots.assign(kSmallCluster, 0);
+// Adds a schedule's items to the shares of the CTAs that the cluster kernel
+// deals them to.
+static void small_share(const int* ptr, const std::vector<int>& wr, int virt, int ctas, bool at,
+                        std::vector<SmallShare>& share) {
+    const int nw = (int)wr.size() - 1;
     for (int w = 0; w < nw; ++w) {
-        const int r = (w % stride) / kSmallWarps;
-        ent[r] += ptr[wr[w + 1]] - ptr[wr[w]];
-        slots[r] += wr[w + 1] - wr[w] + 1;
+        SmallShare& s = share[(w % virt) % ctas];
+        ++(at ? s.items_at : s.items_a);
+        s.entries += ptr[wr[w + 1]] - ptr[wr[w]];
+        s.pointers += wr[w + 1] - wr[w] + 1;
+    }
+}
+
+// LPs whose FP32 attempts take the cluster: at most kSmallItems items per
+// virtual warp, and replicas and share of eight CTAs within 200 KB (the sums of
+// an FP32 attempt are not those of the grid-wide kernels, so the line stays
+// where results have it). FP64 attempts take it where the same holds: their
+// sums are the grid-wide kernels'.
+static bool small_lp(int m, int n, const int* pa, const std::vector<int>& wa, const int* pat,
+                     const std::vector<int>& wat) {
+    const int na = (int)wa.size() - 1, nat = (int)wat.size() - 1;
+    if (std::max(na, nat) > kSmallMaxItems || std::max(m, n) > 0xffff) return false;
+    std::vector<SmallShare> share(8);
+    for (int o = 0; o < 2; ++o) {
+        const std::vector<int>& wr = o ? wat : wa;
+        const int* ptr = o ? pat : pa;
+        for (int w = 0; w + 1 < (int)wr.size(); ++w) {
+            SmallShare& s = share[(w % kSmallVirtual) / 16];
+            s.entries += ptr[wr[w + 1]] - ptr[wr[w]];
+            s.pointers += wr[w + 1] - wr[w] + 1;
+        }
+    }
+    for (const SmallShare& s : share) {
+        size_t b = (((size_t)n + 2 * (size_t)m) * 4 + 15) & ~(size_t)15;
+        b = (b + (size_t)s.entries * 4 + 15) & ~(size_t)15;
+        if (b + (size_t)s.entries * 4 + (size_t)s.pointers * 4 + 64 > 200 * 1024) return false;
     }
     return true;
+}
+
+// The smallest cluster that holds the LP with at most 8 virtual warps a CTA (two
+// per SMSP); else the largest that holds it, in FP32 one of 8; else, in FP32, one
+// that holds the matrix only. 1,024 iterations of a 300 x 700 LP (22 virtual
+// warps) on 2, 4 and 8 CTAs: FP64 9.4, 7.6, 7.4 ms, FP32 6.4, 5.9, 5.9; of a
+// 60 x 150 LP (5) on 1 and 2: 8.1, 8.6; 2,048 FP32 ones of a 2,000 x 5,000 LP (128)
+// on 8 and 16: 14.8, 15.2.
+template <typename T>
+static SmallPlan small_plan(int m, int n, const int* pa, const std::vector<int>& wa,
+                            const int* pat, const std::vector<int>& wat) {
+    constexpr bool f32 = std::is_same<T, float>::value;
+    const int na = (int)wa.size() - 1, nat = (int)wat.size() - 1;
+    SmallPlan best;
+    for (int held = 1; held >= (f32 ? 0 : 1) && best.ctas == 0; --held)
+        for (int ctas = 1; ctas <= kSmallCluster; ctas *= 2) {
+            SmallPlan p;
+            p.ctas = ctas;
+            p.held = held;
+            p.virt_a = f32 ? std::min(kSmallVirtual, na) : na;
+            p.virt_at = f32 ? std::min(kSmallVirtual, nat) : nat;
+            std::vector<SmallShare> share(ctas);
+            small_share(pa, wa, p.virt_a, ctas, false, share);
+            small_share(pat, wat, p.virt_at, ctas, true, share);
+            for (const SmallShare& s : share) {
+                p.cap.items_at = std::max(p.cap.items_at, s.items_at);
+                p.cap.items_a = std::max(p.cap.items_a, s.items_a);
+                p.cap.entries = std::max(p.cap.entries, s.entries);
+                p.cap.pointers = std::max(p.cap.pointers, s.pointers);
+            }
+            p.bytes = small_bytes<T>(m, n, p);
+            if (p.bytes > kSmallSmemMax || !cluster_fits<T>(p)) continue;
+            best = p;
+            if (8 * ctas >= std::max(p.virt_at, p.virt_a) || (f32 && ctas >= 8)) break;
+        }
+    return best;
 }
 
 // Launch width: enough CTAs for every warp item, capped at what stays
@@ -272,8 +337,10 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
             if (kTuneEntries[c] == kLaneEntries) sA_ = candA_[c];
             cap_ctas_A_ = std::max(cap_ctas_A_, candA_[c].ctas);
         }
-        std::vector<long long> ent_a, slot_a, ent_at, slot_at;
-        bool fit = small_share(P.data(), m, ent_a, slot_a);
+        std::vector<int> wa, wat;  // default schedules' items, for the cluster path
+        std::vector<unsigned char> lg;
+        if ((long long)std::max(m, n) <= 32LL * kSmallMaxItems) build_warps(P.data(), m, wa, lg);
+        const std::vector<int> pa_rows = P;
         // FP32 copy of A with every row padded to a multiple of 4 entries
         // (16-byte aligned rows, pads: value 0 and the row's first index) for
         // 16-byte vector loads (lane_products); built below when the LP runs
@@ -291,32 +358,22 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
             if (kTuneEntries[c] == kLaneEntries) sAT_ = candAT_[c];
             cap_ctas_AT_ = std::max(cap_ctas_AT_, candAT_[c].ctas);
         }
-        fit = small_share(P.data(), n, ent_at, slot_at) && fit;
         // small LPs: the attempts of a chunk in one thread-block cluster with
-        // the LP staged in its shared memory (cluster.cuh) when the largest
-        // rank's share fits. FP32 only by default: on the 2,000 x 5,000 LP an
-        // FP32 attempt takes 7.9 us there against 12.1 us on the grid-wide
-        // kernels, an FP64 attempt 17.9 us against 17.3 us (FP64 arithmetic
-        // on 8 SMs). IGAOS_PDHG_CLUSTER=0: never; =all: FP64 too.
+        // the LP in its shared memory (cluster.cuh): 1,024 FP64 iterations
+        // of a 60 x 150 LP take 8.1 ms, 14.7 with the grid-wide kernels;
+        // of a 2,000 x 5,000 LP 11.0 and 15.5.
+        // IGAOS_PDHG_CLUSTER=0: never.
         const char* e = std::getenv("IGAOS_PDHG_CLUSTER");
-        const bool allow = !(e && std::strcmp(e, "0") == 0);
-        const bool with64 = e && std::strcmp(e, "all") == 0;
-        if (allow && fit) {
-            for (int k = 0; k < (with64 ? 2 : 1); ++k) {
-                const int sz = k ? 8 : 4;
-                size_t worst = 0;
-                for (int r = 0; r < kSmallCluster; ++r)
-                    worst = std::max(worst, small_smem_bytes(m, n,
-                                                             SmallLayout{ent_at[r], slot_at[r], ent_a[r],
-                                                                         slot_a[r]},
-                                                             sz));
-                if (worst <= kSmallSmemMax && cluster_fits(k == 1, (int)worst))
-                    small_bytes_[k] = (int)worst;
+        if (!(e && std::strcmp(e, "0") == 0) && !wa.empty()) {
+            build_warps(P.data(), n, wat, lg);
+            if (small_lp(m, n, pa_rows.data(), wa, P.data(), wat)) {
+                small_[0] = small_plan<float>(m, n, pa_rows.data(), wa, P.data(), wat);
+                small_[1] = small_plan<double>(m, n, pa_rows.data(), wa, P.data(), wat);
             }
         }
         // the cluster path stages A by its unpadded row pointers: no padded
         // copy for LPs it runs
-        if (!P4.empty() && small_bytes_[0] == 0) {
+        if (!P4.empty() && small_[0].ctas == 0) {
             ap4_ = ar_.alloc<int>(m + 1);
             ai4_ = ar_.alloc<int>((size_t)P4[m]);
             ax4_ = ar_.alloc<float>((size_t)P4[m]);
@@ -547,8 +604,8 @@ void Engine::ensure_work() {
     w.pesx = ar_.alloc<T>(n);
     w.yb = ar_.alloc<T>(m);
     w.pesy = ar_.alloc<T>(m);
-    w.part_p = ar_.alloc<double>(std::max(cap_ctas_AT_, kSmallCluster));
-    w.part_d = ar_.alloc<double>(2 * (size_t)std::max(cap_ctas_A_, kSmallCluster));
+    w.part_p = ar_.alloc<double>(cap_ctas_AT_);
+    w.part_d = ar_.alloc<double>(2 * (size_t)cap_ctas_A_);
     have = true;
 }
 
@@ -655,15 +712,17 @@ void Engine::launch_attempts(int count, const Vecs& v, bool graphs) {
     PrimalArgs<T> pa;
     DualArgs<T> da;
     attempt_args<T>(v, pa, da);
-    if (const int sb = small_bytes_[std::is_same<T, double>::value ? 1 : 0]) {
+    if (const SmallPlan& plan = small_[std::is_same<T, double>::value ? 1 : 0]; plan.ctas) {
         // one cluster runs the whole chunk with the LP in shared memory (it
         // stages the default schedule)
         pa.ws = sRAT_.view();
         da.ws = sRA_.view();
         ++launches_;
-        CU(cudaFuncSetAttribute(k_attempts_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sb));
-        k_attempts_cluster<T><<<kSmallCluster, kSmallThreads, sb, st_>>>(pa, da, m, n, count);
-        CU(cudaGetLastError());
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = cluster_config(at, plan, st_);
+        CU(cudaLaunchKernelEx(&cfg,
+                              plan.held ? k_attempts_cluster<T, true> : k_attempts_cluster<T, false>,
+                              pa, da, m, n, count, plan));
         return;
     }
     launches_ += 2LL * count;
@@ -716,7 +775,7 @@ void Engine::tune() {
     int def = 0;
     for (int c = 0; c < kTuneCount; ++c)
         if (kTuneEntries[c] == kLaneEntries) def = c;
-    if (small_bytes_[pi]) {
+    if (small_[pi].ctas) {
         choice_[pi][0] = choice_[pi][1] = def;
         return;
     }

@@ -97,6 +97,19 @@ struct Work {
 template <typename T> struct PrimalArgs;  // kernels.cuh
 template <typename T> struct DualArgs;
 
+// How the attempts of a small LP run in one thread-block cluster (cluster.cuh).
+struct SmallShare {  // what one CTA holds
+    int items_at = 0, items_a = 0;
+    long long entries = 0, pointers = 0;
+};
+struct SmallPlan {
+    int ctas = 0;                 // 0: the grid-wide kernels
+    int virt_at = 0, virt_a = 0;  // virtual warps per orientation
+    int held = 0;                 // 1: the iterates and their bounds in shared memory
+    SmallShare cap;               // the most of any CTA
+    size_t bytes = 0;             // dynamic shared memory per CTA
+};
+
 struct GraphKey {
     int prec, count;
     uintptr_t vecs;
@@ -280,9 +293,9 @@ class Engine {
     };
     RepBufs rep_{};
     bool have_rep_ = false;
-    // dynamic shared memory of the cluster attempt kernel for FP32 / FP64
-    // (0: that precision uses the grid-wide kernels)
-    int small_bytes_[2] = {0, 0};
+    // the cluster attempt kernel for FP32 / FP64 (no CTAs: that precision uses
+    // the grid-wide kernels)
+    SmallPlan small_[2];
     void ensure_rep();
     void rep_sum(const double* v, const double* w, const unsigned char* mask, int len, double* out);
     void rep_cgls(int iters, double rtol);

@@ -89,6 +89,10 @@ struct PrimalArgs {
 // xavg' = xavg + w (x' - xavg), w = 2/(hn+2) (kern_mix2, :129-141, :795-799),
 // written to the other parity slot so that a rejected attempt leaves the
 // accepted state untouched.
+template <typename T>
+__device__ __forceinline__ T primal_step(T tau, T g, T x, T lo, T hi) {
+    return clamp_val(fma(-tau, g, x), lo, hi);
+}
 // Hook called with each row's new gathered-vector entry (xbar_j, y'_i):
 // nothing for the grid-wide kernels.
 struct NoBcast {
@@ -110,7 +114,7 @@ struct PrimalEpi {
     }
     __device__ __forceinline__ void apply(int j, const Acc<T>& acc, const Pre& v) {
         const T g = v.c + acc.result();
-        const T xn = clamp_val(fma(-tau, g, v.x), v.lo, v.hi);
+        const T xn = primal_step(tau, g, v.x, v.lo, v.hi);
         xn_out[j] = xn;
         const T xb = fma((T)2, xn, -v.x);
         xbar[j] = xb;
@@ -183,6 +187,14 @@ struct DualArgs {
 // iterations to the same objective, bit for bit, on the 14 golden LPs, six
 // Netlib LPs and a 1 x 1 LP; giving in-range rows an exact 0 instead froze
 // the 1 x 1 LP's step size: with dy = 0 the line search sees no curvature.)
+template <typename T>
+__device__ __forceinline__ T dual_step(T sigma, T isigma, T ab, T y, bool anchored, T yh, T lo, T hi) {
+    const T t = fma(sigma, ab, y);
+    const T u = anchored ? t + yh : t;
+    const T q0 = u * isigma;
+    const T q = fma(fma(-sigma, q0, u), isigma, q0);
+    return fma(-sigma, clamp_val(q, lo, hi), t);
+}
 template <typename T, class B = NoBcast>
 struct DualEpi {
     const T *rmin, *rmax, *yc, *axc, *ya, *yhat;
@@ -198,11 +210,7 @@ struct DualEpi {
     }
     __device__ __forceinline__ void apply(int i, const Acc<T>& acc, const Pre& v) {
         const T ab = acc.result();
-        const T t = fma(sigma, ab, v.y);
-        const T u = yhat ? t + v.yh : t;
-        const T q0 = u * isigma;
-        const T q = fma(fma(-sigma, q0, u), isigma, q0);
-        const T yn = fma(-sigma, clamp_val(q, v.lo, v.hi), t);
+        const T yn = dual_step(sigma, isigma, ab, v.y, yhat != nullptr, v.yh, v.lo, v.hi);
         yn_out[i] = yn;
         bc(i, yn);
         const T dy = yn - v.y;
@@ -236,17 +244,11 @@ struct StepState {
     long long k, hn;
     int retries;
 };
-__device__ __forceinline__ StepState load_step(const DevCtl* c, const double* fac, int n_fac) {
-    StepState s;
-    s.eta = c->eta;
-    s.omega = c->omega;
-    s.iomega = c->iomega;
-    s.k = c->k;
-    s.hn = c->hn;
-    s.retries = c->retries;
-    // growth/shrink factors 1 - k^-0.3 and 1 + k^-0.6, tabulated by the host
-    // (std::pow, as the reference) for the iterations of this chunk
-    const long long fi = s.k - c->fac_base;
+// growth/shrink factors 1 - k^-0.3 and 1 + k^-0.6, tabulated by the host
+// (std::pow, as the reference) for the iterations of this chunk
+__device__ __forceinline__ void step_factors(StepState& s, long long fac_base, const double* fac,
+                                             int n_fac) {
+    const long long fi = s.k - fac_base;
     if (fac && fi >= 0 && fi < n_fac) {
         s.f_lo = fac[2 * fi];
         s.f_hi = fac[2 * fi + 1];
@@ -255,6 +257,16 @@ __device__ __forceinline__ StepState load_step(const DevCtl* c, const double* fa
         s.f_lo = __dsub_rn(1.0, pow(kk, -0.3));
         s.f_hi = __dadd_rn(1.0, pow(kk, -0.6));
     }
+}
+__device__ __forceinline__ StepState load_step(const DevCtl* c, const double* fac, int n_fac) {
+    StepState s;
+    s.eta = c->eta;
+    s.omega = c->omega;
+    s.iomega = c->iomega;
+    s.k = c->k;
+    s.hn = c->hn;
+    s.retries = c->retries;
+    step_factors(s, c->fac_base, fac, n_fac);
     return s;
 }
 
@@ -268,8 +280,11 @@ __device__ __forceinline__ StepState load_step(const DevCtl* c, const double* fa
 // 1/sigma. With six divisions in one thread, its loads behind the dot products
 // and FP64 comparisons, 1,024 FP64 iterations of a 60 x 150 LP took 17.5 ms,
 // now 16.0, and of a 2,000 x 5,000 LP 19.6, now 17.9.
-__device__ __forceinline__ void decide_step(DevCtl* c, const StepState& s, double dx2, double dy2,
-                                            double cross) {
+struct StepOut {
+    double eta, w;  // the next attempt's step size; the averaging weight after an acceptance
+    bool accept, sound;
+};
+__device__ __forceinline__ StepOut step_rule(const StepState& s, double dx2, double dy2, double cross) {
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
     auto nonneg_less = [](double a, double b) {  // a, b >= 0
@@ -296,26 +311,33 @@ __device__ __forceinline__ void decide_step(DevCtl* c, const StepState& s, doubl
     } else {
         eta = usable ? eta_new : 1e-12;
     }
+    return StepOut{eta, w_next, accept, sound};
+}
+__device__ __forceinline__ void decide_step(DevCtl* c, const StepState& s, double dx2, double dy2,
+                                            double cross) {
+    const int lane = threadIdx.x & 31;
+    const StepOut o = step_rule(s, dx2, dy2, cross);
+    const double eta = o.eta;
     const double sigma = __dmul_rn(eta, s.omega);
     // lane 0: tau; lane 1: 1 / sigma
     const double out = __ddiv_rn(lane == 1 ? 1.0 : eta, lane == 1 ? sigma : s.omega);
-    const double isigma = __shfl_sync(full, out, 1);
+    const double isigma = __shfl_sync(0xffffffffu, out, 1);
     if (lane != 0) return;
     c->dots[0] = dx2;
     c->dots[1] = dy2;
     c->dots[2] = cross;
-    if (!sound) c->nan_flag = 1;
+    if (!o.sound) c->nan_flag = 1;
     c->attempts += 1;
     c->eta = eta;
-    if (accept) {
+    if (o.accept) {
         c->parity ^= 1;
         c->hn = s.hn + 1;
         c->accepted += 1;
         c->retries = 0;
         if (s.k >= c->k_stop || c->nan_flag) c->stop = 1;
         c->k = s.k + 1;
-        c->w = w_next;
-        c->w_f = (float)w_next;
+        c->w = o.w;
+        c->w_f = (float)o.w;
     } else {
         c->retries = s.retries + 1;
     }
