@@ -70,6 +70,22 @@ void build_warps(const int* ptr, int rows, std::vector<int>& wrow, std::vector<u
     }
 }
 
+// A kernel as a programmatic launch: it waits for its predecessor in the stream
+// itself (see follow_previous).
+template <typename... P, typename... A>
+static void launch_following(void (*kernel)(P...), dim3 grid, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CU(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
 // One cluster of the attempt kernel: its launch configuration, and whether one
 // can be resident on this device (else the grid-wide kernels serve).
 static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* at, const SmallPlan& plan,
@@ -279,6 +295,10 @@ static int grid_for(long long n, int per_block = kThreads, int cap = 152 * 16) {
     return (int)g;
 }
 
+// The control block and the metrics behind it, on the device and in the host
+// mirror: one copy brings both.
+constexpr size_t kMetAt = (sizeof(DevCtl) + 63) & ~(size_t)63;
+
 // ------------------------------------------------------------------ setup
 Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, const double* ax,
                const int* cp, const int* ci, const double* acx, const double* c,
@@ -415,18 +435,17 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
     idr_ = ar_.alloc<double>(m);
     idc_ = ar_.alloc<double>(n);
     // control + scratch
-    ctl_ = ar_.alloc<DevCtl>(1);
-    met_ = ar_.alloc<DevMetrics>(2);
+    ctl_ = reinterpret_cast<DevCtl*>(ar_.alloc<char>(kMetAt + 2 * sizeof(DevMetrics)));
+    met_ = reinterpret_cast<DevMetrics*>(reinterpret_cast<char*>(ctl_) + kMetAt);
     CU(cudaMemsetAsync(ctl_, 0, sizeof(DevCtl), st_));
     {  // one pinned block for every host mirror (a pinned allocation costs ~1 ms)
-        const size_t o_met = (sizeof(DevCtl) + 63) & ~(size_t)63;
-        const size_t o_scal = o_met + ((2 * sizeof(DevMetrics) + 63) & ~(size_t)63);
+        const size_t o_scal = kMetAt + ((2 * sizeof(DevMetrics) + 63) & ~(size_t)63);
         const size_t o_fac = o_scal + 16 * sizeof(double);
         const size_t o_rep = o_fac + 2 * kFac * sizeof(double);
         CU(cudaMallocHost(&h_pin_, o_rep + 16 * sizeof(double)));
         char* b = static_cast<char*>(h_pin_);
         h_ctl_ = reinterpret_cast<DevCtl*>(b);
-        h_met_ = reinterpret_cast<DevMetrics*>(b + o_met);
+        h_met_ = reinterpret_cast<DevMetrics*>(b + kMetAt);
         h_scal_ = reinterpret_cast<double*>(b + o_scal);
         h_fac_ = reinterpret_cast<double*>(b + o_fac);
         h_rep_ = reinterpret_cast<double*>(b + o_rep);
@@ -674,34 +693,19 @@ int Engine::grid_dual() const {
     if constexpr (std::is_same<T, double>::value) return occ_[0] == 4 ? sA_.ctas64w : sA_.ctas64;
     return sA_.ctas;
 }
-// An attempt kernel on the engine's stream, as a programmatic launch (it waits
-// for its predecessor itself, see follow_previous).
-template <typename A>
-static void launch_following(void (*kernel)(A), int grid, const A& args, cudaStream_t st) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CU(cudaLaunchKernelEx(&cfg, kernel, args));
-}
 template <typename T>
 void Engine::launch_primal(const PrimalArgs<T>& pa) {
     const int gp = grid_primal<T>();
     if constexpr (std::is_same<T, double>::value)
-        launch_following(occ_[1] == 4 ? k_primal<double, 4> : k_primal<double, 3>, gp, pa, st_);
-    else launch_following(k_primal<T>, gp, pa, st_);
+        launch_following(occ_[1] == 4 ? k_primal<double, 4> : k_primal<double, 3>, gp, st_, pa);
+    else launch_following(k_primal<T>, gp, st_, pa);
 }
 template <typename T>
 void Engine::launch_dual(const DualArgs<T>& da) {
     const int gd = grid_dual<T>();
     if constexpr (std::is_same<T, double>::value)
-        launch_following(occ_[0] == 4 ? k_dual<double, 4> : k_dual<double, 3>, gd, da, st_);
-    else launch_following(k_dual<T>, gd, da, st_);
+        launch_following(occ_[0] == 4 ? k_dual<double, 4> : k_dual<double, 3>, gd, st_, da);
+    else launch_following(k_dual<T>, gd, st_, da);
 }
 
 // Enqueues `count` line-search attempts (2 launches each). With graphs the
@@ -869,9 +873,12 @@ double Engine::elapsed() const {
 // Launch attempts until the device raises `stop` (iteration k_stop accepted
 // or NaN). The first batch covers the accepted iterations still needed plus
 // the rejections the history predicts; the rest are topped up in small
-// batches (a stopped launch is a no-op).
+// batches (a stopped launch is a no-op); one cluster's launch covers any number
+// of rejections (it ends at the stop). With `check`, the KKT pass of the two
+// candidates is enqueued behind each batch and its metrics come with the
+// control block, in h_met_.
 template <typename T>
-void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out) {
+void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out, bool check) {
     for (;;) {
         const long long need = h_ctl_->k_stop - (h_ctl_->k - 1);
         const double rej = h_ctl_->accepted > 0
@@ -880,10 +887,15 @@ void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out) {
         long long want = (long long)std::ceil((double)need * (1.0 + 1.2 * rej)) + (rej > 0 ? 1 : 0);
         int cnt = want <= 1 ? 1 : want <= 4 ? 4 : want <= 8 ? 8 : want <= 16 ? 16
                   : want <= 32 ? 32 : want <= 64 ? 64 : want <= 72 ? 72 : want <= 80 ? 80 : 96;
+        if (small_[std::is_same<T, double>::value ? 1 : 0].ctas)
+            cnt = (int)std::min<long long>(1 << 30, 32 * std::max(1LL, need));
         CU(cudaEventRecord(ev_[2], st_));
         launch_attempts<T>(cnt, v, graphs);
         CU(cudaEventRecord(ev_[3], st_));
-        download_ctl();
+        if (check) enqueue_check<T>(v);
+        CU(cudaMemcpyAsync(h_ctl_, ctl_, check ? kMetAt + 2 * sizeof(DevMetrics) : sizeof(DevCtl),
+                           cudaMemcpyDeviceToHost, st_));
+        CU(cudaStreamSynchronize(st_));
         float ms = 0.f;
         CU(cudaEventElapsedTime(&ms, ev_[2], ev_[3]));
         attempt_ms_ += ms;
@@ -893,12 +905,11 @@ void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out) {
 }
 
 template <typename T>
-void Engine::kkt(const Vecs& v, const T* x0, const T* y0, const T* x1, const T* y1, int ncand) {
+void Engine::launch_kkt(const Vecs& v, const Candidates<T>& x, const Candidates<T>& y, int ncand,
+                        const DevCtl* ctl) {
     KktArgs<T> ka;
-    ka.x[0] = x0;
-    ka.y[0] = y0;
-    ka.x[1] = x1;
-    ka.y[1] = y1;
+    ka.x = x;
+    ka.y = y;
     ka.ax[0] = kkt_ax_;
     ka.ax[1] = kkt_ax_ + m;
     ka.aty[0] = kkt_aty_;
@@ -920,17 +931,49 @@ void Engine::kkt(const Vecs& v, const T* x0, const T* y0, const T* x1, const T* 
     ka.part = kkt_part_;
     ka.out = met_;
     ka.ticket = ticket_ + 2;
-    launches_ += 4;
-    k_kkt_prod<T><<<dim3(sA_.ctas, ncand), kThreads, 0, st_>>>(sA_.view(), csrA<T>(), x0, x1,
-                                                              kkt_ax_, kkt_ax_ + m);
-    k_kkt_prod<T><<<dim3(sAT_.ctas, ncand), kThreads, 0, st_>>>(sAT_.view(), csrAT<T>(), y0, y1,
-                                                               kkt_aty_, kkt_aty_ + n);
+    ka.ctl = ctl;
+    KktProdArgs<T> kp;
+    kp.ws[0] = sA_.view();
+    kp.ws[1] = sAT_.view();
+    kp.M[0] = csrA<T>();
+    kp.M[1] = csrAT<T>();
+    kp.in[0] = x;
+    kp.in[1] = y;
+    for (int k = 0; k < 2; ++k) {
+        kp.out[0][k] = kkt_ax_ + (size_t)k * m;
+        kp.out[1][k] = kkt_aty_ + (size_t)k * n;
+    }
+    kp.ncand = ncand;
+    kp.ctl = ctl;
+    launches_ += 3;
+    launch_following(k_kkt_prod<T>, dim3(std::max(sA_.ctas, sAT_.ctas), 2 * ncand), st_, kp);
     // about four rows (columns) per thread, at most 2 CTAs per SM per candidate
-    k_kkt_rows<T><<<dim3(grid_for(m, 4 * kThreads, 152 * 2), ncand), kThreads, 0, st_>>>(ka, m);
-    k_kkt_cols<T><<<dim3(grid_for(n, 4 * kThreads, 152 * 2), ncand), kThreads, 0, st_>>>(ka, n, m);
-    CU(cudaGetLastError());
+    launch_following(k_kkt_rows<T>, dim3(grid_for(m, 4 * kThreads, 152 * 2), ncand), st_, ka, m);
+    launch_following(k_kkt_cols<T>, dim3(grid_for(n, 4 * kThreads, 152 * 2), ncand), st_, ka, n, m);
+}
+
+template <typename T>
+void Engine::kkt(const Vecs& v, const T* x0, const T* y0, const T* x1, const T* y1, int ncand) {
+    launch_kkt<T>(v, Candidates<T>{{{x0, x1}, {x0, x1}}}, Candidates<T>{{{y0, y1}, {y0, y1}}}, ncand,
+                  nullptr);
     CU(cudaMemcpyAsync(h_met_, met_, ncand * sizeof(DevMetrics), cudaMemcpyDeviceToHost, st_));
     CU(cudaStreamSynchronize(st_));
+}
+
+// The KKT pass of the current and the averaged iterate of the chunk enqueued
+// before it (see candidate_parity).
+template <typename T>
+void Engine::enqueue_check(const Vecs& v) {
+    if (v.fyhat) {  // FP64 metrics of the full iterates anchor + delta
+        launch_anchor_full(ctl_, 0);
+        const double *x0 = anc_.xf[0], *x1 = anc_.xf[1], *y0 = anc_.yf[0], *y1 = anc_.yf[1];
+        launch_kkt<double>(base_, Candidates<double>{{{x0, x1}, {x0, x1}}},
+                           Candidates<double>{{{y0, y1}, {y0, y1}}}, 2, ctl_);
+        return;
+    }
+    Work<T>& w = work<T>();
+    launch_kkt<T>(v, Candidates<T>{{{w.x[0], w.xavg[0]}, {w.x[1], w.xavg[1]}}},
+                  Candidates<T>{{{w.y[0], w.yavg[0]}, {w.y[1], w.yavg[1]}}}, 2, ctl_);
 }
 
 // The reference iteration loop with its 64-iteration checks: termination,
@@ -1261,7 +1304,9 @@ LoopOut Engine::loop(const Vecs& v, const LoopOpts& o) {
                t.gap <= o.tol;
     };
     while (k_done < MAXIT) {
-        run_until_stop<T>(v, o.graphs, out);
+        // the check's metrics, unless the iterate is changed before it
+        const bool ahead = o.perturb_at <= 0 && h_ctl_->k_stop % CHECK == 0;
+        run_until_stop<T>(v, o.graphs, out, ahead);
         k_done = h_ctl_->k - 1;
         out.spmvs = 2 * h_ctl_->attempts;
         if (h_ctl_->nan_flag) {
@@ -1277,11 +1322,10 @@ LoopOut Engine::loop(const Vecs& v, const LoopOpts& o) {
                 CU(cudaGetLastError());
                 perturbed = true;
             }
-            if (anch) {  // FP64 metrics of the full iterates anchor + delta
-                anchor_full(p);
-                kkt<double>(base_, anc_.xf[0], anc_.yf[0], anc_.xf[1], anc_.yf[1], 2);
-            } else {
-                kkt<T>(v, w.x[p], w.y[p], w.xavg[p], w.yavg[p], 2);
+            if (!ahead) {
+                enqueue_check<T>(v);
+                CU(cudaMemcpyAsync(h_met_, met_, 2 * sizeof(DevMetrics), cudaMemcpyDeviceToHost, st_));
+                CU(cudaStreamSynchronize(st_));
             }
             const DevMetrics mc = h_met_[0], ma = h_met_[1];
             const double ec = mc.finite ? mc.err : kInf;
@@ -1718,7 +1762,7 @@ void Engine::iterate(int precision, long long iters, double* x, double* y, doubl
         h_ctl_->k_stop = h_ctl_->k + iters - 1;
         upload_ctl();
         LoopOut out;
-        if (iters > 0) run_until_stop<T>(base_, false, out);
+        if (iters > 0) run_until_stop<T>(base_, false, out, false);
         else download_ctl();
         const int p = h_ctl_->parity;
         down(w.x[p], x, false);
@@ -1877,18 +1921,32 @@ void Engine::anchor_zero(int p) {
     CU(cudaMemsetAsync(w.axc[p], 0, sizeof(float) * m, st_));
 }
 
-void Engine::anchor_full(int p) {
+// parity: of the control block, or (ctl == nullptr) as given
+void Engine::launch_anchor_full(const DevCtl* ctl, int p) {
     Work<float>& w = w32_;
-    const int gn = grid_for(n), gm = grid_for(m);
-    k_anchor_full_cols<<<gn, kThreads, 0, st_>>>(n, anc_.xh, w.x[p], av_.fcl, av_.fcu, base_.scl,
-                                                 base_.scu, anc_.xf[0]);
-    k_anchor_full_cols<<<gn, kThreads, 0, st_>>>(n, anc_.xh, w.xavg[p], av_.fcl, av_.fcu,
-                                                 base_.scl, base_.scu, anc_.xf[1]);
-    k_anchor_full_rows<<<gm, kThreads, 0, st_>>>(m, anc_.yh, w.y[p], anc_.yf[0]);
-    k_anchor_full_rows<<<gm, kThreads, 0, st_>>>(m, anc_.yh, w.yavg[p], anc_.yf[1]);
-    launches_ += 4;
-    CU(cudaGetLastError());
+    AnchorFullArgs a;
+    a.n = n;
+    a.m = m;
+    a.xh = anc_.xh;
+    a.yh = anc_.yh;
+    for (int s = 0; s < 2; ++s) {
+        const int q = ctl ? s : p;
+        a.dx.at[s][0] = w.x[q];
+        a.dx.at[s][1] = w.xavg[q];
+        a.dy.at[s][0] = w.y[q];
+        a.dy.at[s][1] = w.yavg[q];
+        a.x[s] = anc_.xf[s];
+        a.y[s] = anc_.yf[s];
+    }
+    a.flo = av_.fcl;
+    a.fhi = av_.fcu;
+    a.scl = base_.scl;
+    a.scu = base_.scu;
+    a.ctl = ctl;
+    ++launches_;
+    launch_following(k_anchor_full, dim3(grid_for(std::max(n, m)), 2), st_, a);
 }
+void Engine::anchor_full(int p) { launch_anchor_full(nullptr, p); }
 
 void Engine::anchor_to(const double* x, const double* y) {
     if (x != anc_.xh)

@@ -96,6 +96,7 @@ struct Work {
 
 template <typename T> struct PrimalArgs;  // kernels.cuh
 template <typename T> struct DualArgs;
+template <typename T> struct Candidates;
 
 // How the attempts of a small LP run in one thread-block cluster (cluster.cuh).
 struct SmallShare {  // what one CTA holds
@@ -266,7 +267,11 @@ class Engine {
         launch_primal<T>(pa);
         launch_dual<T>(da);
     }
-    template <typename T> void run_until_stop(const Vecs& v, bool graphs, LoopOut& out);
+    template <typename T> void run_until_stop(const Vecs& v, bool graphs, LoopOut& out, bool check);
+    template <typename T> void launch_kkt(const Vecs& v, const Candidates<T>& x,
+                                          const Candidates<T>& y, int ncand, const DevCtl* ctl);
+    template <typename T> void enqueue_check(const Vecs& v);
+    void launch_anchor_full(const DevCtl* ctl, int p);
     template <typename T> void kkt(const Vecs& v, const T* x0, const T* y0, const T* x1,
                                    const T* y1, int ncand);
     template <typename T> void spmv_dev(bool transpose, const T* x, T* y);

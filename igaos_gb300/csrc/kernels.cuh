@@ -682,9 +682,9 @@ __global__ void k_convert(int n, const TI* __restrict__ in, TO* __restrict__ out
 // --------------------------------------------------------------- KKT pass
 // FP64 metrics of candidate pairs (x~, y~) in ORIGINAL units, one fused
 // device pass replacing metrics_of + evaluate (src/pdhg/pdhg.cu:698-733,
-// 173-254). Candidate v = blockIdx.y. Four launches:
-//   prod (A)  : A~ x~ over the warp schedule, stored in FP64 (scaled units)
-//   prod (A^T): A~^T y~, likewise
+// 173-254). Candidate v = blockIdx.y. Three launches:
+//   prod      : A~ x~ and A~^T y~ over the warp schedules, stored in FP64
+//               (scaled units)
 //   rows      : one thread per row: pinf numerator/normaliser, prow, max |y|
 //   cols      : one thread per column: reduced costs d, dinf, c^T x, the
 //               column part of the Lagrangian bound; then one thread per row
@@ -696,11 +696,30 @@ __global__ void k_convert(int n, const TI* __restrict__ in, TO* __restrict__ out
 // rows or columns per thread, and their maxima reduce on the integer pipe:
 // with a row per thread, the FP64 compares of the block reductions cost
 // more of that pipe than the metrics themselves.
+// In the solve loop the pass is enqueued behind a chunk of attempts before the
+// host knows its outcome: the candidates are those of the control block's
+// parity, and a chunk that has not stopped (more attempts are to come) makes
+// the pass a no-op. What a check of a small LP costs is launches and the
+// host's two waits: with the pass launched after the chunk's answer, two
+// product kernels and four for the anchored iterates, a check took 143 us of a
+// 2,000 x 5,000 LP's solve, now 114.
+
+// One vector of each candidate, by the parity of the accepted iterate.
+template <typename T>
+struct Candidates {
+    const T* at[2][2];  // [parity][candidate]
+};
+// The parity of the candidates to evaluate: the control block's; 0 without
+// one; -1 while its chunk runs on. First in a kernel: waits for its predecessor.
+__device__ __forceinline__ int candidate_parity(const DevCtl* ctl) {
+    follow_previous();
+    if (!ctl) return 0;
+    return __ldcg(&ctl->stop) ? __ldcg(&ctl->parity) : -1;
+}
 
 template <typename T>
 struct KktArgs {
-    const T* x[2];
-    const T* y[2];
+    Candidates<T> x, y;
     const double* ax[2];                      // A~ x~ per candidate (scaled units)
     const double* aty[2];                     // A~^T y~ per candidate (scaled units)
     const double *dr, *dc;
@@ -715,25 +734,40 @@ struct KktArgs {
     double* part;   // >= 2 * blocks * 8 doubles
     DevMetrics* out;
     unsigned int* ticket;
+    const DevCtl* ctl;  // of the chunk just enqueued, or nullptr
 };
 
 // Products of both candidates: out[v] = M v_in[v] in FP64 (the same warp
 // traversal and accumulator as every other product of the engine).
 template <typename T>
-__global__ void __launch_bounds__(kThreads, HotCtas<T>::value)
-    k_kkt_prod(WarpSched ws, Csr<T> M, const T* in0, const T* in1, double* out0, double* out1) {
-    const T* __restrict__ in = blockIdx.y ? in1 : in0;
-    double* __restrict__ out = blockIdx.y ? out1 : out0;
+struct KktProdArgs {
+    WarpSched ws[2];  // A, A^T
+    Csr<T> M[2];
+    Candidates<T> in[2];
+    double* out[2][2];  // [orientation][candidate]
+    int ncand;
+    const DevCtl* ctl;
+};
+// Both candidates' products with A~ and A~^T: blockIdx.y = candidate + ncand * orientation.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, HotCtas<T>::value) k_kkt_prod(KktProdArgs<T> a) {
+    const int o = blockIdx.y >= a.ncand, v = blockIdx.y - o * a.ncand;
+    const int p = candidate_parity(a.ctl);
+    if (p < 0) return;
+    double* __restrict__ out = a.out[o][v];
     auto f = [&](int r, const Acc<T>& acc) { out[r] = acc.result_d(); };
     PlainEpi<decltype(f)> epi{f};
-    warp_rows_all<T>(ws, M, in, epi);
+    warp_rows_all<T>(a.ws[o], a.M[o], a.in[o].at[p][v], epi);
+    let_next();
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_kkt_rows(KktArgs<T> a, int m) {
     __shared__ __align__(16) double smred[kWarps * 4];
-    const int v = blockIdx.y;
-    const T* __restrict__ yv = a.y[v];
+    const int v = blockIdx.y, p = candidate_parity(a.ctl);
+    if (p < 0) return;
+    let_next();
+    const T* __restrict__ yv = a.y.at[p][v];
     const double* __restrict__ axv = a.ax[v];
     double pv = 0.0, pa = 0.0, prow = 0.0, ymax = 0.0;
     // comparisons on the integer pipe (dmax, dmin, ...; see device.cuh)
@@ -778,8 +812,9 @@ __global__ void __launch_bounds__(kThreads) k_kkt_rows(KktArgs<T> a, int m) {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_kkt_cols(KktArgs<T> a, int n, int m) {
     __shared__ __align__(16) double smred[kWarps * 4];
-    const int v = blockIdx.y;
-    const T* __restrict__ xv = a.x[v];
+    const int v = blockIdx.y, p = candidate_parity(a.ctl);
+    if (p < 0) return;
+    const T* __restrict__ xv = a.x.at[p][v];
     const double* __restrict__ atyv = a.aty[v];
     const double dz = 1e-8 * (1.0 + a.cmax);
     double dv = 0.0, op = 0.0, od = 0.0, unb = 0.0;
@@ -802,7 +837,7 @@ __global__ void __launch_bounds__(kThreads) k_kkt_cols(KktArgs<T> a, int n, int 
         }
     }
     // row part of the Lagrangian bound (src/pdhg/pdhg.cu:232-242)
-    const T* __restrict__ yv = a.y[v];
+    const T* __restrict__ yv = a.y.at[p][v];
     const double yz = 1e-8 * (1.0 + a.out[v].ymax);
     double odr = 0.0, unbr = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
@@ -890,22 +925,30 @@ __global__ void k_anchor_rows(int m, const double* __restrict__ srmin,
     }
 }
 
-// Full FP64 iterate anchor + delta. A primal delta sitting on its FP32
-// shifted bound is exactly at the bound (the same rule as unscale_x).
-__global__ void k_anchor_full_cols(int n, const double* __restrict__ xh, const float* __restrict__ dx,
-                                   const float* __restrict__ flo, const float* __restrict__ fhi,
-                                   const double* __restrict__ scl, const double* __restrict__ scu,
-                                   double* __restrict__ out) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+// Full FP64 iterates anchor + delta of the current and the averaged one (v =
+// blockIdx.y). A primal delta sitting on its FP32 shifted bound is exactly at
+// the bound (the same rule as unscale_x).
+struct AnchorFullArgs {
+    int n, m;
+    const double *xh, *yh;
+    Candidates<float> dx, dy;
+    const float *flo, *fhi;
+    const double *scl, *scu;
+    double *x[2], *y[2];
+    const DevCtl* ctl;
+};
+__global__ void __launch_bounds__(kThreads) k_anchor_full(AnchorFullArgs a) {
+    const int v = blockIdx.y, p = candidate_parity(a.ctl);
+    if (p < 0) return;
+    let_next();
+    const float* __restrict__ dx = a.dx.at[p][v];
+    const float* __restrict__ dy = a.dy.at[p][v];
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.n; j += gridDim.x * blockDim.x) {
         const float d = dx[j];
-        out[j] = d == flo[j] ? scl[j] : (d == fhi[j] ? scu[j] : xh[j] + (double)d);
+        a.x[v][j] = d == a.flo[j] ? a.scl[j] : (d == a.fhi[j] ? a.scu[j] : a.xh[j] + (double)d);
     }
-}
-
-__global__ void k_anchor_full_rows(int m, const double* __restrict__ yh, const float* __restrict__ dy,
-                                   double* __restrict__ out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-        out[i] = yh[i] + (double)dy[i];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.m; i += gridDim.x * blockDim.x)
+        a.y[v][i] = a.yh[i] + (double)dy[i];
 }
 
 }  // namespace igx
