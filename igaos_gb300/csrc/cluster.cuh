@@ -54,14 +54,20 @@ __device__ __forceinline__ int cluster_count() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return (int)r;
 }
-// all threads of every CTA of the cluster; release/acquire at cluster scope
-// (global and distributed shared memory)
-__device__ __forceinline__ void cluster_arrive() {
+// All threads of every CTA of the cluster, in two halves; release/acquire at
+// cluster scope (global and distributed shared memory). The release alone
+// takes about 1,000 cycles after remote stores, 500 without: work that
+// nobody waits for goes between the halves. One CTA has no first half.
+__device__ __forceinline__ void cluster_arrive(int ctas) {
     __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_wait() {
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_wait(int ctas) {
+    __syncwarp();
+    if (ctas > 1)
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+        __syncthreads();
 }
 // v into the entry `at` (an address in this CTA's replica) of every CTA's
 template <typename T>
@@ -82,44 +88,36 @@ struct ClusterBcast {
     __device__ __forceinline__ void operator()(int i, T v) const { cluster_put(base + i, v, ctas); }
 };
 
-// One orientation as staged by a CTA: entries and row pointers (local entry
-// offsets) in shared memory, an item being {first row, rows, log2 G, first
-// row pointer}.
+// A CTA's items as staged: item = {first row, rows, log2 G, first slot}; entry u
+// of a lane (its row's entries gl, gl + G, ...) lies at slot first + 32 u +
+// lane, padded with zeros to the longest row's entries per lane (the item's
+// count, in the bits of log2 G from 8 up).
 template <typename T>
 struct Staged {
-    const int* ptr;
     const uint16_t* idx;
     const T* val;
-    const int4* item;
 };
+__host__ __device__ inline int staged_count(int longest, int lg) {
+    return (longest + (1 << lg) - 1) >> lg;
+}
 
-// lane sums of one staged item, reduced and handed to the lanes of its rows
-// (the sums and their order are those of lane_products and reduce_rows)
+// row sums of one staged item, handed to the lanes of its rows (the sums and
+// their order are those of lane_products and reduce_rows)
 template <typename T>
 __device__ __forceinline__ Acc<T> staged_sums(const int4 d, const Staged<T>& S,
                                               const T* __restrict__ sx) {
-    const int lane = threadIdx.x & 31;
-    const int nr = d.y, lg = d.z, pb = d.w;
-    const int G = 1 << lg;
-    const int g = lane >> lg, gl = lane & (G - 1);
+    int at = d.w + (threadIdx.x & 31), left = d.z >> 8;
     Acc<T> acc;
-    if (g < nr) {
-        const int b = S.ptr[pb + g], e = S.ptr[pb + g + 1];
-        for (int p = b + gl; p < e; p += kLaneBatch * G) {
-            T a[kLaneBatch];
-            int j[kLaneBatch];
-#pragma unroll
-            for (int u = 0; u < kLaneBatch; ++u) {
-                const int q = p + u * G;
-                const bool ok = q < e;
-                a[u] = ok ? S.val[q] : T(0);
-                j[u] = ok ? S.idx[q] : 0;
-            }
-#pragma unroll
-            for (int u = 0; u < kLaneBatch; ++u) acc.add(a[u], sx[j[u]]);
-        }
+#pragma unroll 1
+    for (; left >= 2; left -= 2, at += 64) {
+        const T a0 = S.val[at], a1 = S.val[at + 32];
+        const int j0 = S.idx[at], j1 = S.idx[at + 32];
+        const T x0 = sx[j0], x1 = sx[j1];
+        acc.add(a0, x0);
+        acc.add(a1, x1);
     }
-    return reduce_rows<T>(acc, lg);
+    if (left) acc.add(S.val[at], sx[S.idx[at]]);
+    return reduce_rows<T>(acc, d.z & 0xff);
 }
 
 // Sum over a warp in the order of block_sum_t.
@@ -143,10 +141,10 @@ __host__ __device__ inline size_t small_bytes(int m, int n, const SmallPlan& p) 
         b += (size_t)p.cap.items_a * 32 * 9 * sizeof(T);                          // rows' vectors
     }
     b += (size_t)2 * (small_pad<T>(p.virt_at) + small_pad<T>(p.virt_a)) * sizeof(T);  // partials
-    b += (size_t)p.cap.entries * sizeof(T);                                    // values
+    b += (size_t)p.cap.slots * sizeof(T);                                    // values
     b = (b + 15) & ~(size_t)15;
     b += (size_t)(p.cap.items_at + p.cap.items_a) * sizeof(int4);              // items
-    b += (size_t)p.cap.pointers * 4 + (size_t)p.cap.entries * 2;               // pointers, indices
+    b += (size_t)p.cap.slots * 2;                                              // indices
     return b + 32;
 }
 
@@ -220,16 +218,18 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ CtlView<T> sview;
     __shared__ double stotal[2];
-    __shared__ int scnt[2][kSmallWarps + 1][3];
+    __shared__ int scnt[2][kSmallWarps + 1][2];
     const int rank = cluster_rank(), ctas = plan.ctas;
     const int wi = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
     const bool owns = wi < kSmallWarps;
-    // warps of the SMSPs 1 to 3 first: the decision's runs on SMSP 0; the rows
-    // of A from the other end, off the warps that hold columns, if few
-    const int at_pos = (wi & 3) ? (wi >> 2) * 3 + (wi & 3) - 1 : 12 + (wi >> 2);
+    // columns go to the lower warps first, of these to the SMSPs 1 to 3 (their
+    // products run beside the decision's warp, on SMSP 0); rows to the upper
+    // ones, over the SMSPs in turn
+    const int low = wi & 7;
+    const int at_pos = (wi & 8) + ((low & 3) ? (low >> 2) * 3 + (low & 3) - 1 : 6 + (low >> 2));
     const int deal_step = kSmallWarps * ctas;
     const int first_at = at_pos * ctas + rank;
-    const int first_a = (at_pos < 12 ? 11 - at_pos : at_pos) * ctas + rank;
+    const int first_a = (kSmallWarps - 1 - wi) * ctas + rank;
 
     // ---- carve
     const int sat = HELD ? plan.cap.items_at * 32 : 0, sa = HELD ? plan.cap.items_a * 32 : 0;
@@ -243,11 +243,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     T* part_dx = va + 9 * sa;                     // of every other attempt
     T *part_dy = part_dx + 2 * pad_at, *part_cr = part_dy + pad_a;
     T* val = part_cr + pad_a;
-    off = (size_t)(reinterpret_cast<unsigned char*>(val + plan.cap.entries) - smem);
+    off = (size_t)(reinterpret_cast<unsigned char*>(val + plan.cap.slots) - smem);
     off = (off + 15) & ~(size_t)15;
     int4* item = reinterpret_cast<int4*>(smem + off);
-    int* ptr = reinterpret_cast<int*>(item + plan.cap.items_at + plan.cap.items_a);
-    uint16_t* idx = reinterpret_cast<uint16_t*>(ptr + plan.cap.pointers);
+    uint16_t* idx = reinterpret_cast<uint16_t*>(item + plan.cap.items_at + plan.cap.items_a);
 
     // ---- each warp's share of both schedules: items, entries, row pointers
     auto items_of = [&](int o, auto&& f) {  // every item of this warp, in order
@@ -259,22 +258,20 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     if (owns)
         for (int o = 0; o < 2; ++o) {
             const Csr<T>& A = o ? da.A : pa.AT;
-            int c = 0, e = 0, r = 0;
+            int c = 0, e = 0;
             items_of(o, [&](const WarpSched& ws, int w) {
-                const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
-                ++c;
-                e += __ldg(A.ptr + r1) - __ldg(A.ptr + r0);
-                r += r1 - r0 + 1;
+                const int r0 = __ldg(ws.row + w);
+                ++c;  // (rows are sorted by decreasing length)
+                e += 32 * staged_count(__ldg(A.ptr + r0 + 1) - __ldg(A.ptr + r0), __ldg(ws.lg + w));
             });
             if (lane == 0) {
                 scnt[o][wi + 1][0] = c;
                 scnt[o][wi + 1][1] = e;
-                scnt[o][wi + 1][2] = r;
             }
         }
     for (int i = threadIdx.x; i < 2 * (pad_at + pad_a); i += kSmallThreads) part_dx[i] = T(0);
     __syncthreads();
-    if (threadIdx.x < 3) {
+    if (threadIdx.x < 2) {
         int run = 0;  // rows of A after those of A~^T, in one sequence
         for (int o = 0; o < 2; ++o) {
             scnt[o][0][threadIdx.x] = run;
@@ -288,16 +285,22 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     if (owns)
         for (int o = 0; o < 2; ++o) {
             const Csr<T>& A = o ? da.A : pa.AT;
-            int k = scnt[o][wi][0], ce = scnt[o][wi][1], cp = scnt[o][wi][2];
+            int k = scnt[o][wi][0], ce = scnt[o][wi][1];
             items_of(o, [&](const WarpSched& ws, int w) {
                 const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
-                const int e0 = __ldg(A.ptr + r0), e1 = __ldg(A.ptr + r1);
-                for (int t = lane; t <= r1 - r0; t += 32) ptr[cp + t] = __ldg(A.ptr + r0 + t) - e0 + ce;
-                for (int q = lane; q < e1 - e0; q += 32) {
-                    idx[ce + q] = (uint16_t)__ldg(A.idx + e0 + q);
-                    val[ce + q] = __ldg(A.val + e0 + q);
+                const int lg = __ldg(ws.lg + w), r = r0 + (lane >> lg);
+                const int cnt = staged_count(__ldg(A.ptr + r0 + 1) - __ldg(A.ptr + r0), lg);
+                int q = 0, e = 0;
+                if (r < r1) {
+                    q = __ldg(A.ptr + r) + (lane & ((1 << lg) - 1));
+                    e = __ldg(A.ptr + r + 1);
                 }
-                if (lane == 0) item[k] = make_int4(r0, r1 - r0, __ldg(ws.lg + w), cp);
+                for (int u = 0; u < cnt; ++u, q += 1 << lg) {
+                    const bool ok = q < e;
+                    idx[ce + 32 * u + lane] = ok ? (uint16_t)__ldg(A.idx + q) : (uint16_t)0;
+                    val[ce + 32 * u + lane] = ok ? __ldg(A.val + q) : T(0);
+                }
+                if (lane == 0) item[k] = make_int4(r0, r1 - r0, lg | cnt << 8, ce);
                 const int i = r0 + lane;
                 if (HELD && lane < r1 - r0) {
                     if (o == 0) {
@@ -317,8 +320,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                         v[(7 + p0) * sa] = da.yavg[p0][i];
                     }
                 }
-                cp += r1 - r0 + 1;
-                ce += e1 - e0;
+                ce += 32 * cnt;
                 ++k;
             });
         }
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     }
     const long long fac_base = pa.ctl->fac_base;
     __syncthreads();
-    const Staged<T> S{ptr, idx, val, item};
+    const Staged<T> S{idx, val};
     // A~^T y of slot q into sg, this warp's items
     auto product_at = [&](int q) {
         int k = it0;
@@ -346,8 +348,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         });
     };
     if (HELD && owns) product_at(p0);
-    cluster_arrive();  // every CTA running and staged before any remote write
-    cluster_wait();
+    cluster_arrive(ctas);  // every CTA running and staged before any remote write
+    cluster_wait(ctas);
 
     int att = 0;
     for (; att < max_attempts; ++att) {
@@ -388,8 +390,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 }
             }
         }
-        cluster_arrive();
-        if (HELD && owns) {  // ||dx||^2 and the average, for barriers to come
+        cluster_arrive(ctas);
+        auto averages_at = [&]() {  // ||dx||^2 and the average
             int k = it0;
             for (int v = first_at; v < plan.virt_at; v += deal_step) {
                 T dx2 = T(0);
@@ -405,9 +407,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 dx2 = lanes_sum(dx2);
                 if (lane == 0) cluster_put(dx_to + v, dx2, ctas);
             }
-        }
-        __syncwarp();
-        cluster_wait();
+        };
+        if (HELD && owns && ctas > 1) averages_at();
+        cluster_wait(ctas);
+        if (HELD && owns && ctas == 1) averages_at();
         if (owns) {  // dual half
             int k = it1;
             DualEpi<T, ClusterBcast<T>> epi{da.rmin,    da.rmax,   da.y[p],    da.axc[p], da.yavg[p], da.yhat,
@@ -446,8 +449,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 }
             }
         }
-        cluster_arrive();
-        if (HELD && owns) {
+        cluster_arrive(ctas);
+        auto averages_a = [&]() {
             int k = it1;
             items_of(1, [&](const WarpSched&, int) {
                 if (lane < item[k].y) {
@@ -458,9 +461,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 }
                 ++k;
             });
-        }
-        __syncwarp();
-        cluster_wait();
+        };
+        if (HELD && owns && ctas > 1) averages_a();
+        cluster_wait(ctas);
+        if (HELD && owns && ctas == 1) averages_a();
         if (owns) {
             if (HELD) product_at(q);
         } else if (wi == kSmallWarps || sizeof(T) == 8) {
@@ -535,8 +539,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
             ++k;
         });
     }
-    cluster_arrive();  // no CTA leaves while another may still write to it
-    cluster_wait();    // (and every CTA has read the control block)
+    cluster_arrive(ctas);  // no CTA leaves while another may still write to it
+    cluster_wait(ctas);    // (and every CTA has read the control block)
     if (rank == 0 && wi == kSmallWarps && lane == 0 && attempts) {
         DevCtl* c = pa.ctl;
         for (int k = 0; k < 3; ++k) c->dots[k] = dots[k];

@@ -121,14 +121,13 @@ static bool cluster_fits(const SmallPlan& plan) {
 
 // Adds a schedule's items to the shares of the CTAs that the cluster kernel
 // deals them to.
-static void small_share(const int* ptr, const std::vector<int>& wr, int virt, int ctas, bool at,
+static void small_share(const int* ptr, const std::vector<int>& wr,
+                        const std::vector<unsigned char>& lg, int virt, int ctas, bool at,
                         std::vector<SmallShare>& share) {
-    const int nw = (int)wr.size() - 1;
-    for (int w = 0; w < nw; ++w) {
+    for (int w = 0; w < (int)lg.size(); ++w) {
         SmallShare& s = share[(w % virt) % ctas];
         ++(at ? s.items_at : s.items_a);
-        s.entries += ptr[wr[w + 1]] - ptr[wr[w]];
-        s.pointers += wr[w + 1] - wr[w] + 1;
+        s.slots += 32 * staged_count(ptr[wr[w] + 1] - ptr[wr[w]], lg[w]);
     }
 }
 
@@ -141,20 +140,20 @@ static bool small_lp(int m, int n, const int* pa, const std::vector<int>& wa, co
                      const std::vector<int>& wat) {
     const int na = (int)wa.size() - 1, nat = (int)wat.size() - 1;
     if (std::max(na, nat) > kSmallMaxItems || std::max(m, n) > 0xffff) return false;
-    std::vector<SmallShare> share(8);
+    long long entries[8] = {}, pointers[8] = {};
     for (int o = 0; o < 2; ++o) {
         const std::vector<int>& wr = o ? wat : wa;
         const int* ptr = o ? pat : pa;
         for (int w = 0; w + 1 < (int)wr.size(); ++w) {
-            SmallShare& s = share[(w % kSmallVirtual) / 16];
-            s.entries += ptr[wr[w + 1]] - ptr[wr[w]];
-            s.pointers += wr[w + 1] - wr[w] + 1;
+            const int r = (w % kSmallVirtual) / 16;
+            entries[r] += ptr[wr[w + 1]] - ptr[wr[w]];
+            pointers[r] += wr[w + 1] - wr[w] + 1;
         }
     }
-    for (const SmallShare& s : share) {
+    for (int r = 0; r < 8; ++r) {
         size_t b = (((size_t)n + 2 * (size_t)m) * 4 + 15) & ~(size_t)15;
-        b = (b + (size_t)s.entries * 4 + 15) & ~(size_t)15;
-        if (b + (size_t)s.entries * 4 + (size_t)s.pointers * 4 + 64 > 200 * 1024) return false;
+        b = (b + (size_t)entries[r] * 4 + 15) & ~(size_t)15;
+        if (b + (size_t)entries[r] * 4 + (size_t)pointers[r] * 4 + 64 > 200 * 1024) return false;
     }
     return true;
 }
@@ -167,7 +166,8 @@ static bool small_lp(int m, int n, const int* pa, const std::vector<int>& wa, co
 // on 8 and 16: 14.8, 15.2.
 template <typename T>
 static SmallPlan small_plan(int m, int n, const int* pa, const std::vector<int>& wa,
-                            const int* pat, const std::vector<int>& wat) {
+                            const std::vector<unsigned char>& la, const int* pat,
+                            const std::vector<int>& wat, const std::vector<unsigned char>& lat) {
     constexpr bool f32 = std::is_same<T, float>::value;
     const int na = (int)wa.size() - 1, nat = (int)wat.size() - 1;
     SmallPlan best;
@@ -179,13 +179,12 @@ static SmallPlan small_plan(int m, int n, const int* pa, const std::vector<int>&
             p.virt_a = f32 ? std::min(kSmallVirtual, na) : na;
             p.virt_at = f32 ? std::min(kSmallVirtual, nat) : nat;
             std::vector<SmallShare> share(ctas);
-            small_share(pa, wa, p.virt_a, ctas, false, share);
-            small_share(pat, wat, p.virt_at, ctas, true, share);
+            small_share(pa, wa, la, p.virt_a, ctas, false, share);
+            small_share(pat, wat, lat, p.virt_at, ctas, true, share);
             for (const SmallShare& s : share) {
                 p.cap.items_at = std::max(p.cap.items_at, s.items_at);
                 p.cap.items_a = std::max(p.cap.items_a, s.items_a);
-                p.cap.entries = std::max(p.cap.entries, s.entries);
-                p.cap.pointers = std::max(p.cap.pointers, s.pointers);
+                p.cap.slots = std::max(p.cap.slots, s.slots);
             }
             p.bytes = small_bytes<T>(m, n, p);
             if (p.bytes > kSmallSmemMax || !cluster_fits<T>(p)) continue;
@@ -358,8 +357,8 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
             cap_ctas_A_ = std::max(cap_ctas_A_, candA_[c].ctas);
         }
         std::vector<int> wa, wat;  // default schedules' items, for the cluster path
-        std::vector<unsigned char> lg;
-        if ((long long)std::max(m, n) <= 32LL * kSmallMaxItems) build_warps(P.data(), m, wa, lg);
+        std::vector<unsigned char> la, lat;
+        if ((long long)std::max(m, n) <= 32LL * kSmallMaxItems) build_warps(P.data(), m, wa, la);
         const std::vector<int> pa_rows = P;
         // FP32 copy of A with every row padded to a multiple of 4 entries
         // (16-byte aligned rows, pads: value 0 and the row's first index) for
@@ -385,10 +384,10 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         // IGAOS_PDHG_CLUSTER=0: never.
         const char* e = std::getenv("IGAOS_PDHG_CLUSTER");
         if (!(e && std::strcmp(e, "0") == 0) && !wa.empty()) {
-            build_warps(P.data(), n, wat, lg);
+            build_warps(P.data(), n, wat, lat);
             if (small_lp(m, n, pa_rows.data(), wa, P.data(), wat)) {
-                small_[0] = small_plan<float>(m, n, pa_rows.data(), wa, P.data(), wat);
-                small_[1] = small_plan<double>(m, n, pa_rows.data(), wa, P.data(), wat);
+                small_[0] = small_plan<float>(m, n, pa_rows.data(), wa, la, P.data(), wat, lat);
+                small_[1] = small_plan<double>(m, n, pa_rows.data(), wa, la, P.data(), wat, lat);
             }
         }
         // the cluster path stages A by its unpadded row pointers: no padded

@@ -101,7 +101,7 @@ template <typename T> struct Candidates;
 // How the attempts of a small LP run in one thread-block cluster (cluster.cuh).
 struct SmallShare {  // what one CTA holds
     int items_at = 0, items_a = 0;
-    long long entries = 0, pointers = 0;
+    long long slots = 0;  // padded entries
 };
 struct SmallPlan {
     int ctas = 0;                 // 0: the grid-wide kernels
