@@ -127,6 +127,17 @@ __device__ __forceinline__ T lanes_sum(T v) {
     return v;
 }
 
+// Two sums at once, each in that order: the first's in lanes 0 to 15, the
+// second's in 16 to 31 (half the additions of two lanes_sum).
+template <typename T>
+__device__ __forceinline__ T lanes_sum2(T v0, T v1) {
+    const bool up = threadIdx.x & 16;
+    T s = up ? v1 : v0;
+    s += __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 16);
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 // The sums of a half's virtual warps lie padded with zeros to small_pad.
 template <typename T>
 __host__ __device__ inline int small_pad(int virt) {
@@ -146,6 +157,17 @@ __host__ __device__ inline size_t small_bytes(int m, int n, const SmallPlan& p) 
     b += (size_t)(p.cap.items_at + p.cap.items_a) * sizeof(int4);              // items
     b += (size_t)p.cap.slots * 2;                                              // indices
     return b + 32;
+}
+
+// (float)(a / b) of the FP64 quotient, ib = 1 / b correctly rounded: the
+// product is within two ulps of it, which decides the float unless they
+// straddle the middle of two.
+__device__ __forceinline__ float float_quotient(double a, double b, double ib) {
+    const double q = __dmul_rn(a, ib);
+    const unsigned low = (unsigned)__double2loint(q) & 0x1fffffffu;
+    const int ex = (__double2hiint(q) >> 20) & 0x7ff;
+    const bool clear = low - 0x0ffffff8u > 16u && ex > 1023 - 126 && ex < 1023 + 127;
+    return clear ? (float)q : (float)div_exact(a, b, ib);
 }
 
 // FP32: the three totals, by one warp: partials of 16 virtual warps, plain
@@ -442,11 +464,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                     }
                 }
                 __syncwarp();
-                const T dy2 = lanes_sum(epi.dy2), cross = lanes_sum(epi.cross);
-                if (lane == 0) {
-                    cluster_put(part_dy + v, dy2, ctas);
-                    cluster_put(part_cr + v, cross, ctas);
-                }
+                const T sums = lanes_sum2(epi.dy2, epi.cross);
+                if ((lane & 15) == 0) cluster_put((lane ? part_cr : part_dy) + v, sums, ctas);
             }
         }
         cluster_arrive(ctas);
@@ -489,7 +508,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                     nv.isigma = __shfl_sync(0xffffffffu, out, 1);
                     nv.tau = out;
                 } else {
-                    nv.tau = (float)div_exact(o.eta, st.omega, st.iomega);
+                    nv.tau = float_quotient(o.eta, st.omega, st.iomega);
                     nv.isigma = 1.0f / (float)sigma;
                 }
                 nv.sigma = (T)sigma;
