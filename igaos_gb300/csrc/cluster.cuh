@@ -120,24 +120,6 @@ __device__ __forceinline__ Acc<T> staged_sums(const int4 d, const Staged<T>& S,
     return reduce_rows<T>(acc, d.z & 0xff);
 }
 
-// Sum over a warp in the order of block_sum_t.
-template <typename T>
-__device__ __forceinline__ T lanes_sum(T v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Two sums at once, each in that order: the first's in lanes 0 to 15, the
-// second's in 16 to 31 (half the additions of two lanes_sum).
-template <typename T>
-__device__ __forceinline__ T lanes_sum2(T v0, T v1) {
-    const bool up = threadIdx.x & 16;
-    T s = up ? v1 : v0;
-    s += __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 16);
-    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
-}
-
 // The sums of a half's virtual warps lie padded with zeros to small_pad.
 template <typename T>
 __host__ __device__ inline int small_pad(int virt) {

@@ -315,18 +315,40 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
     __syncthreads();
 }
 
+// Sum over a warp, in every lane.
+template <typename T>
+__device__ __forceinline__ T lanes_sum(T v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Two sums at once, each in that order: the first's in lanes 0 to 15, the
+// second's in 16 to 31 (half the additions of two lanes_sum).
+template <typename T>
+__device__ __forceinline__ T lanes_sum2(T v0, T v1) {
+    const bool up = threadIdx.x & 16;
+    T s = up ? v1 : v0;
+    s += __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 16);
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 // Same tree in the working precision (FP32 partials of FP32 kernels; the
 // cross-CTA finish is FP64). `sh` needs NW * NV values of type T.
 template <typename T, int NV, int NW = kWarps>
 __device__ __forceinline__ void block_sum_t(T (&v)[NV], T* sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if constexpr (NV == 2) {
+        const T s = lanes_sum2(v[0], v[1]);
+        __syncthreads();
+        if ((lane & 15) == 0) sh[w * 2 + (lane >> 4)] = s;
+    } else {
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-    __syncthreads();
-    if (lane == 0)
+        for (int q = 0; q < NV; ++q) v[q] = lanes_sum(v[q]);
+        __syncthreads();
+        if (lane == 0)
 #pragma unroll
-        for (int q = 0; q < NV; ++q) sh[w * NV + q] = v[q];
+            for (int q = 0; q < NV; ++q) sh[w * NV + q] = v[q];
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll

@@ -525,8 +525,8 @@ void Engine::setup_scaling() {
     k_fill<<<grid_for(m), kThreads, 0, st_>>>(m, 1.0, dr_);
     k_fill<<<grid_for(n), kThreads, 0, st_>>>(n, 1.0, dc_);
     for (int sweep = 0; sweep < 10; ++sweep) {
-        k_ruiz_rows<<<sRA_.ctas, kThreads, 0, st_>>>(sRA_.view(), ap_, ai_, ax_, dc_, dr_);
-        k_ruiz_cols<<<sRAT_.ctas, kThreads, 0, st_>>>(sRAT_.view(), cp_, ci_, acx_, dr_, dc_);
+        launch_following(k_ruiz_rows, sRA_.ctas, st_, sRA_.view(), ap_, ai_, ax_, dc_, dr_, idr_);
+        launch_following(k_ruiz_cols, sRAT_.ctas, st_, sRAT_.view(), cp_, ci_, acx_, dr_, idr_, dc_);
     }
     if (scaling_ == IGAOS_PDHG_SCALING_RUIZ_PC) {
         k_pc_sums<<<sRA_.ctas, kThreads, 0, st_>>>(sRA_.view(), ap_, ai_, ax_, dr_, dc_, 1, tmp_m_);
@@ -570,11 +570,8 @@ template <> Csr<float> Engine::csrAT<float>() const { return Csr<float>{cp_, ci_
 template <typename T>
 void Engine::spmv_dev(bool transpose, const T* x, T* y) {
     ++launches_;
-    if (transpose)
-        k_spmv<T, T><<<sAT_.ctas, kThreads, 0, st_>>>(sAT_.view(), csrAT<T>(), x, y);
-    else
-        k_spmv<T, T><<<sA_.ctas, kThreads, 0, st_>>>(sA_.view(), csrA<T>(), x, y);
-    CU(cudaGetLastError());
+    if (transpose) launch_following(k_spmv<T, T>, sAT_.ctas, st_, sAT_.view(), csrAT<T>(), x, y);
+    else launch_following(k_spmv<T, T>, sA_.ctas, st_, sA_.view(), csrA<T>(), x, y);
 }
 
 // lambda ~ ||A~||_2^2 by 30 power iterations (src/pdhg/pdhg.cu:605-631),
@@ -588,8 +585,8 @@ void Engine::power_iteration() {
     for (int it = 0; it < 30; ++it) {
         spmv_dev<double>(false, v, tm);
         spmv_dev<double>(true, tm, w);
-        k_sumsq<<<red_blocks_, kThreads, 0, st_>>>(NormArgs{w, n, red_part_, scal_, ticket_ + 1}, 1);
-        k_power_normalise<<<grid_for(n), kThreads, 0, st_>>>(n, w, v, scal_, flag_);
+        launch_following(k_sumsq, red_blocks_, st_, NormArgs{w, n, red_part_, scal_, ticket_ + 1}, 1);
+        launch_following(k_power_normalise, grid_for(n), st_, n, w, v, scal_, flag_);
     }
     spmv_dev<double>(false, v, tm);
     k_sumsq<<<red_blocks_, kThreads, 0, st_>>>(NormArgs{tm, m, red_part_, scal_ + 1, ticket_ + 1}, 1);
