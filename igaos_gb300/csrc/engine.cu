@@ -33,12 +33,31 @@ Arena::~Arena() {
     for (void* p : ptrs_) cudaFree(p);
 }
 
+// Buffers are cut from larger allocations: of about what the owner says it will
+// take first, then of an eighth of that. A cudaMalloc and its cudaFree take
+// 4 us together for a few KB, 70 for some MB, and an LP has a hundred buffers.
+// What does not fit in such a block (or would not leave memory for one)
+// gets its own.
 void* Arena::raw(size_t bytes) {
-    void* p = nullptr;
     bytes = (bytes + 255) & ~size_t(255);
-    CU(cudaMalloc(&p, bytes));
-    ptrs_.push_back(p);
     total_ += bytes;
+    if (bytes > left_) {
+        const size_t block = ptrs_.empty() ? expect_ : std::max<size_t>(1 << 20, expect_ / 8);
+        void* p = nullptr;
+        if (block > bytes && cudaMalloc(&p, block) == cudaSuccess) {
+            ptrs_.push_back(p);
+            next_ = static_cast<char*>(p);
+            left_ = block;
+        } else {
+            cudaGetLastError();
+            CU(cudaMalloc(&p, bytes));
+            ptrs_.push_back(p);
+            return p;
+        }
+    }
+    void* p = next_;
+    next_ += bytes;
+    left_ -= bytes;
     return p;
 }
 
@@ -251,8 +270,8 @@ static void permute_csr(int rows, const int* ptr, const int* idx, const double* 
             }
         }
     };
-    const int nt = nnz < (1 << 20) ? 1
-                                   : (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+    const int nt = (int)std::min<long long>(std::max(1u, std::thread::hardware_concurrency()),
+                                            std::min<long long>(16, std::max<long long>(1, nnz >> 16)));
     if (nt == 1) {
         fill(0, rows);
         return;
@@ -268,6 +287,14 @@ static void permute_csr(int rows, const int* ptr, const int* idx, const double* 
         r0 = hi;
     }
     for (auto& th : pool) th.join();
+}
+
+// index of the default schedule among the autotuner's
+static int def_sched() {
+    int def = 0;
+    for (int c = 0; c < kTuneCount; ++c)
+        if (kTuneEntries[c] == kLaneEntries) def = c;
+    return def;
 }
 
 static std::vector<int> inverse(const std::vector<int>& p) {
@@ -331,6 +358,9 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
     ipr_ = inverse(pr_);
     ipc_ = inverse(pc_);
     mark("stream, orderings");
+    // both orientations in FP64 and FP32 with their indices, FP32 padded rows,
+    // and about 45 doubles of vectors per row and column
+    ar_.expect((size_t)nnz * 41 + ((size_t)m + n) * 360 + (1 << 20));
     {
         std::vector<int> P;
         std::unique_ptr<int[]> I;
@@ -350,12 +380,9 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         int sms = 0;
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
         const int resident = std::max(1, sms) * kHotCtasPerSm;
+        cap_ctas_ = resident;
         sRA_ = upload_sched(ar_, P.data(), m, resident, kLaneEntries);
-        for (int c = 0; c < kTuneCount; ++c) {
-            candA_[c] = upload_sched(ar_, P.data(), m, resident, kTuneEntries[c]);
-            if (kTuneEntries[c] == kLaneEntries) sA_ = candA_[c];
-            cap_ctas_A_ = std::max(cap_ctas_A_, candA_[c].ctas);
-        }
+        sA_ = candA_[def_sched()] = sRA_;
         std::vector<int> wa, wat;  // default schedules' items, for the cluster path
         std::vector<unsigned char> la, lat;
         if ((long long)std::max(m, n) <= 32LL * kSmallMaxItems) build_warps(P.data(), m, wa, la);
@@ -372,11 +399,7 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         CU(cudaMemcpy(ci_, I.get(), sizeof(int) * nnz, cudaMemcpyHostToDevice));
         CU(cudaMemcpy(acx_, V.get(), sizeof(double) * nnz, cudaMemcpyHostToDevice));
         sRAT_ = upload_sched(ar_, P.data(), n, resident, kLaneEntries);
-        for (int c = 0; c < kTuneCount; ++c) {
-            candAT_[c] = upload_sched(ar_, P.data(), n, resident, kTuneEntries[c]);
-            if (kTuneEntries[c] == kLaneEntries) sAT_ = candAT_[c];
-            cap_ctas_AT_ = std::max(cap_ctas_AT_, candAT_[c].ctas);
-        }
+        sAT_ = candAT_[def_sched()] = sRAT_;
         // small LPs: the attempts of a chunk in one thread-block cluster with
         // the LP in its shared memory (cluster.cuh): 1,024 FP64 iterations
         // of a 60 x 150 LP take 8.1 ms, 14.7 with the grid-wide kernels;
@@ -452,7 +475,7 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
     fac_ = ar_.alloc<double>(2 * kFac);
     std::memset(h_ctl_, 0, sizeof(DevCtl));
     red_blocks_ = grid_for(std::max(m, n), kThreads, 152 * 4);
-    const int kkt_blocks = std::max(std::max(cap_ctas_A_, cap_ctas_AT_), red_blocks_);
+    const int kkt_blocks = std::max(cap_ctas_, red_blocks_);
     kkt_part_ = ar_.alloc<double>((size_t)2 * kkt_blocks * 8);
     kkt_ax_ = ar_.alloc<double>((size_t)2 * m);
     kkt_aty_ = ar_.alloc<double>((size_t)2 * n);
@@ -619,8 +642,8 @@ void Engine::ensure_work() {
     w.pesx = ar_.alloc<T>(n);
     w.yb = ar_.alloc<T>(m);
     w.pesy = ar_.alloc<T>(m);
-    w.part_p = ar_.alloc<double>(cap_ctas_AT_);
-    w.part_d = ar_.alloc<double>(2 * (size_t)cap_ctas_A_);
+    w.part_p = ar_.alloc<double>(cap_ctas_);
+    w.part_d = ar_.alloc<double>(2 * (size_t)cap_ctas_);
     have = true;
 }
 
@@ -752,6 +775,19 @@ void Engine::launch_attempts(int count, const Vecs& v, bool graphs) {
     CU(cudaGraphLaunch(it->second, st_));
 }
 
+// The autotuner's other schedules, on its first use.
+void Engine::ensure_candidates() {
+    if (candA_[0].row && candA_[kTuneCount - 1].row) return;
+    std::vector<int> pa(m + 1), pat(n + 1);
+    CU(cudaMemcpy(pa.data(), ap_, sizeof(int) * pa.size(), cudaMemcpyDeviceToHost));
+    CU(cudaMemcpy(pat.data(), cp_, sizeof(int) * pat.size(), cudaMemcpyDeviceToHost));
+    for (int c = 0; c < kTuneCount; ++c) {
+        if (c == def_sched()) continue;
+        candA_[c] = upload_sched(ar_, pa.data(), m, cap_ctas_, kTuneEntries[c]);
+        candAT_[c] = upload_sched(ar_, pat.data(), n, cap_ctas_, kTuneEntries[c]);
+    }
+}
+
 void Engine::use_sched(int ia, int iat) {
     ia_ = ia;
     iat_ = iat;
@@ -772,13 +808,12 @@ template <typename T>
 void Engine::tune() {
     const int pi = std::is_same<T, double>::value ? 1 : 0;
     if (choice_[pi][0] >= 0) return;
-    int def = 0;
-    for (int c = 0; c < kTuneCount; ++c)
-        if (kTuneEntries[c] == kLaneEntries) def = c;
+    const int def = def_sched();
     if (small_[pi].ctas) {
         choice_[pi][0] = choice_[pi][1] = def;
         return;
     }
+    ensure_candidates();
     ensure_work<T>();
     Work<T>& w = work<T>();
     for (int s = 0; s < 2; ++s) {
@@ -1546,9 +1581,7 @@ void Engine::solve(const igaos_pdhg_options& o, igaos_pdhg_result& r, double* x,
     // warp schedules: the fixed default, or the autotuner's choice for the
     // attempt kernels' precision (timed once per handle and precision)
     const int pi = o.precision == IGAOS_PDHG_FP64 ? 1 : 0;
-    int def = 0;
-    for (int c = 0; c < kTuneCount; ++c)
-        if (kTuneEntries[c] == kLaneEntries) def = c;
+    const int def = def_sched();
     if (o.schedule == IGAOS_PDHG_SCHEDULE_AUTOTUNE) {
         if (pi) tune<double>();
         else tune<float>();

@@ -36,9 +36,14 @@ class Arena {
     template <typename T>
     T* alloc(size_t n) { return static_cast<T*>(raw(sizeof(T) * (n ? n : 1))); }
     size_t bytes() const { return total_; }
+    // what will be allocated in all, about; before the first allocation
+    void expect(size_t bytes) { expect_ = bytes; }
 
    private:
     std::vector<void*> ptrs_;
+    char* next_ = nullptr;  // free part of the newest block
+    size_t left_ = 0;
+    size_t expect_ = 0;
     size_t total_ = 0;
 };
 
@@ -200,12 +205,13 @@ class Engine {
     // warp schedules of A and A^T for every kTuneEntries value; sA_ / sAT_
     // are one of them (kLaneEntries unless the autotuner chose otherwise)
     Sched candA_[kTuneCount], candAT_[kTuneCount];
-    int cap_ctas_A_ = 0, cap_ctas_AT_ = 0;  // largest launch width of the candidates
+    int cap_ctas_ = 0;                      // largest launch width of any of them
     int ia_ = 2, iat_ = 2;                  // candidates in use as sA_ / sAT_ (8 entries)
     int occ_[2] = {3, 3};                   // FP64 attempts: CTAs per SM of k_dual (A), k_primal (A^T)
     int choice_[2][2] = {{-1, -1}, {-1, -1}};  // autotuned (A, A^T) per FP32 / FP64
     int choice_occ_[2] = {3, 3};            // autotuned FP64 occupancy (A, A^T)
     float tune_us_[2][2][kTuneCount][2] = {};  // per attempt-kernel launch, us (occupancy 3, 4)
+    void ensure_candidates();
     void use_sched(int ia, int iat);
     template <typename T> void tune();
     template <typename T> void attempt_args(const Vecs& v, PrimalArgs<T>& pa, DualArgs<T>& da);
