@@ -424,18 +424,26 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         mark("A^T: permute, upload, sched.");
     }
     // vectors
-    auto vec = [&](const double* h, const std::vector<int>& perm) {
-        std::vector<double> t(perm.size());
-        for (size_t i = 0; i < perm.size(); ++i) t[i] = h[perm[i]];
-        double* d = ar_.alloc<double>(t.size());
-        CU(cudaMemcpy(d, t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice));
+    d_pc_ = ar_.alloc<int>(n);
+    d_pr_ = ar_.alloc<int>(m);
+    CU(cudaMemcpyAsync(d_pc_, pc_.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st_));
+    CU(cudaMemcpyAsync(d_pr_, pr_.data(), sizeof(int) * m, cudaMemcpyHostToDevice, st_));
+    tmp_n_ = ar_.alloc<double>(n);
+    tmp_m_ = ar_.alloc<double>(m);
+    auto vec = [&](const double* h, bool rows) {
+        const int len = rows ? m : n;
+        double* raw = rows ? tmp_m_ : tmp_n_;
+        double* d = ar_.alloc<double>(len);
+        CU(cudaMemcpyAsync(raw, h, sizeof(double) * len, cudaMemcpyHostToDevice, st_));
+        k_from_user<<<grid_for(len), kThreads, 0, st_>>>(len, raw, rows ? d_pr_ : d_pc_, d);
+        CU(cudaGetLastError());
         return d;
     };
-    base_.c = vec(c, pc_);
-    base_.cl = vec(cl, pc_);
-    base_.cu = vec(cu, pc_);
-    base_.rmin = vec(rmin, pr_);
-    base_.rmax = vec(rmax, pr_);
+    base_.c = vec(c, false);
+    base_.cl = vec(cl, false);
+    base_.cu = vec(cu, false);
+    base_.rmin = vec(rmin, true);
+    base_.rmax = vec(rmax, true);
     base_.cmax = 0.0;
     for (int j = 0; j < n; ++j) base_.cmax = std::max(base_.cmax, std::fabs(c[j]));
     base_.lob = ar_.alloc<double>(n);
@@ -484,9 +492,7 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
     ticket_ = ar_.alloc<unsigned int>(4);
     flag_ = ar_.alloc<int>(4);
     CU(cudaMemsetAsync(ticket_, 0, 4 * sizeof(unsigned int), st_));
-    tmp_n_ = ar_.alloc<double>(n);
     tmp_n2_ = ar_.alloc<double>(n);
-    tmp_m_ = ar_.alloc<double>(m);
     tmp_m2_ = ar_.alloc<double>(m);
 
     // matrices streamed with an L2 evict-first policy when the attempt's
@@ -901,6 +907,17 @@ double Engine::elapsed() const {
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0_).count();
 }
 
+// A caller's buffer may have no memory behind its pages yet. The copy engine
+// would fault them in one by one: 36 ms against 20 for a solve that returns 4
+// million values, in every other process; on the host it takes 3 ms, done
+// while the first chunk runs.
+static void touch_pages(double* v, size_t len) {
+    if (!v || !len) return;
+    char* q = reinterpret_cast<char*>(v);  // a write that leaves the byte as it is
+    for (size_t i = 0; i < len * sizeof(double); i += 4096) __atomic_fetch_or(q + i, 0, __ATOMIC_RELAXED);
+    __atomic_fetch_or(reinterpret_cast<char*>(v + len - 1), 0, __ATOMIC_RELAXED);
+}
+
 // Launch attempts until the device raises `stop` (iteration k_stop accepted
 // or NaN). The first batch covers the accepted iterations still needed plus
 // the rejections the history predicts; the rest are topped up in small
@@ -924,6 +941,9 @@ void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out, bool check
         launch_attempts<T>(cnt, v, graphs);
         CU(cudaEventRecord(ev_[3], st_));
         if (check) enqueue_check<T>(v);
+        touch_pages(out.touch_x, n);
+        touch_pages(out.touch_y, m);
+        out.touch_x = out.touch_y = nullptr;
         CU(cudaMemcpyAsync(h_ctl_, ctl_, check ? kMetAt + 2 * sizeof(DevMetrics) : sizeof(DevCtl),
                            cudaMemcpyDeviceToHost, st_));
         CU(cudaStreamSynchronize(st_));
@@ -1283,6 +1303,8 @@ LoopOut Engine::loop(const Vecs& v, const LoopOpts& o) {
     ensure_work<T>();
     Work<T>& w = work<T>();
     LoopOut out;
+    out.touch_x = o.touch_x;
+    out.touch_y = o.touch_y;
     const size_t nb = sizeof(T) * n, mb = sizeof(T) * m;
     CU(cudaMemsetAsync(w.x[0], 0, nb, st_));
     CU(cudaMemsetAsync(w.xavg[0], 0, nb, st_));
@@ -1558,14 +1580,14 @@ void Engine::fetch_scaled(const T* src, int len, double* dst) {
     CU(cudaStreamSynchronize(st_));
 }
 
-// Original-unit x (device numbering) of a scaled iterate, with the FP32
-// at-bound rule of unscale_x.
+// Scaled iterates (x as in k_to_user's op) to the caller's buffers, where given.
 template <typename T>
-void Engine::unscale_cols(const T* xs, const Vecs& v, double* host_out) {
-    k_unscale_cols<T><<<grid_for(n), kThreads, 0, st_>>>(n, xs, VecSel<T>::l(v), VecSel<T>::u(v),
-                                                          dc_, v.cl, v.cu, tmp_n_);
+void Engine::answer(const double* xs, int op, const T* ys, double* x, double* y) {
+    k_to_user<double><<<grid_for(n), kThreads, 0, st_>>>(n, xs, op, dc_, d_pc_, tmp_n2_);
+    k_to_user<T><<<grid_for(m), kThreads, 0, st_>>>(m, ys, 2, dr_, d_pr_, tmp_m2_);
     CU(cudaGetLastError());
-    CU(cudaMemcpyAsync(host_out, tmp_n_, sizeof(double) * n, cudaMemcpyDeviceToHost, st_));
+    if (x) CU(cudaMemcpyAsync(x, tmp_n2_, sizeof(double) * n, cudaMemcpyDeviceToHost, st_));
+    if (y) CU(cudaMemcpyAsync(y, tmp_m2_, sizeof(double) * m, cudaMemcpyDeviceToHost, st_));
     CU(cudaStreamSynchronize(st_));
 }
 
@@ -1627,25 +1649,27 @@ void Engine::solve(const igaos_pdhg_options& o, igaos_pdhg_result& r, double* x,
     lo.eta_init = eta0;
     lo.eta0 = eta0;
     lo.omega_init = omega0;
+    lo.touch_x = x;
+    lo.touch_y = y;
     if (const char* e = std::getenv("IGAOS_PDHG_PERTURB_AT")) lo.perturb_at = std::atoll(e);
     LoopOut out;
-    std::vector<double> hx(n), hy(m);
+    // unscaled (x = dc x~, y = y~/dr) and in the caller's numbering
     if (o.precision == IGAOS_PDHG_FP32) {
         out = loop<float>(base_, lo);
         Work<float>& w = w32_;
         const int p = out.parity;
         const float* fx = out.use_inc ? w.xb : (out.last_is_avg ? w.xavg[p] : w.x[p]);
         const float* fy = out.use_inc ? w.yb : (out.last_is_avg ? w.yavg[p] : w.y[p]);
-        unscale_cols<float>(fx, base_, hx.data());
-        fetch_scaled<float>(fy, m, hy.data());
+        k_unscale_cols<float><<<grid_for(n), kThreads, 0, st_>>>(n, fx, base_.fcl, base_.fcu, dc_,
+                                                                 base_.cl, base_.cu, tmp_n_);
+        answer(tmp_n_, 0, fy, x, y);
     } else {
         out = loop<double>(base_, lo);
         Work<double>& w = w64_;
         const int p = out.parity;
         const double* fx = out.use_inc ? w.xb : (out.last_is_avg ? w.xavg[p] : w.x[p]);
         const double* fy = out.use_inc ? w.yb : (out.last_is_avg ? w.yavg[p] : w.y[p]);
-        unscale_cols<double>(fx, base_, hx.data());
-        fetch_scaled<double>(fy, m, hy.data());
+        answer(fx, 1, fy, x, y);
     }
     const double secs = elapsed();
     CU(cudaEventRecord(ev_[1], st_));
@@ -1685,11 +1709,6 @@ void Engine::solve(const igaos_pdhg_options& o, igaos_pdhg_result& r, double* x,
                               "-inf or > tol)"
                             : "iteration cap reached before tolerance");
     }
-    // unscale (x = dc x~, y = y~/dr) and return to the caller's numbering
-    if (x)
-        for (int j = 0; j < n; ++j) x[pc_[j]] = hx[j];  // already in original units
-    if (y)
-        for (int i = 0; i < m; ++i) y[pr_[i]] = 1.0 * hy[i] / hp_dr_[i];
     emit_repaired(out, r, x, y);
 }
 
@@ -2004,6 +2023,8 @@ void Engine::solve_refine(const igaos_pdhg_options& o, igaos_pdhg_result& r, dou
     lo.eta_init = eta0;
     lo.eta0 = eta0;
     lo.omega_init = omega0;
+    lo.touch_x = x;
+    lo.touch_y = y;
     if (const char* e = std::getenv("IGAOS_PDHG_PERTURB_AT")) lo.perturb_at = std::atoll(e);
     LoopOut out = loop<float>(av_, lo);
     // the answer: incumbent, or anchor + delta of the current / averaged iterate
@@ -2016,9 +2037,7 @@ void Engine::solve_refine(const igaos_pdhg_options& o, igaos_pdhg_result& r, dou
         fx = anc_.xf[out.last_is_avg ? 1 : 0];
         fy = anc_.yf[out.last_is_avg ? 1 : 0];
     }
-    std::vector<double> hx(n), hy(m);
-    CU(cudaMemcpyAsync(hx.data(), fx, sizeof(double) * n, cudaMemcpyDeviceToHost, st_));
-    CU(cudaMemcpyAsync(hy.data(), fy, sizeof(double) * m, cudaMemcpyDeviceToHost, st_));
+    answer(fx, 1, fy, x, y);
     CU(cudaEventRecord(ev_[1], st_));
     CU(cudaEventSynchronize(ev_[1]));
     float ms = 0.f;
@@ -2052,10 +2071,6 @@ void Engine::solve_refine(const igaos_pdhg_options& o, igaos_pdhg_result& r, dou
     } else {
         fill_message(r, "iteration cap reached before tolerance");
     }
-    if (x)
-        for (int j = 0; j < n; ++j) x[pc_[j]] = hx[j] * hp_dc_[j];
-    if (y)
-        for (int i = 0; i < m; ++i) y[pr_[i]] = 1.0 * hy[i] / hp_dr_[i];
     emit_repaired(out, r, x, y);
 }
 }  // namespace igx

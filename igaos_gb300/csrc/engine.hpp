@@ -129,6 +129,7 @@ struct GraphKey {
 };
 
 struct LoopOpts {
+    double *touch_x = nullptr, *touch_y = nullptr;  // the answer's buffers (their pages)
     double tol = 1e-4;
     double deadline = 1e300; // seconds since solve start, checked at each KKT check
     long long maxit = 500000;
@@ -145,6 +146,7 @@ struct LoopOpts {
 };
 
 struct LoopOut {
+    double *touch_x = nullptr, *touch_y = nullptr;  // those of LoopOpts, until touched
     int status = IGAOS_STATUS_ERROR;
     DevMetrics last{};
     bool last_is_avg = false, use_inc = false;
@@ -277,13 +279,14 @@ class Engine {
     template <typename T> void launch_kkt(const Vecs& v, const Candidates<T>& x,
                                           const Candidates<T>& y, int ncand, const DevCtl* ctl);
     template <typename T> void enqueue_check(const Vecs& v);
+    template <typename T> void answer(const double* xs, int op, const T* ys, double* x, double* y);
+    int *d_pc_ = nullptr, *d_pr_ = nullptr;  // pc_, pr_ on the device
     void launch_anchor_full(const DevCtl* ctl, int p);
     template <typename T> void kkt(const Vecs& v, const T* x0, const T* y0, const T* x1,
                                    const T* y1, int ncand);
     template <typename T> void spmv_dev(bool transpose, const T* x, T* y);
     template <typename T> LoopOut loop(const Vecs& v, const LoopOpts& o);
     template <typename T> void fetch_scaled(const T* src, int len, double* dst);
-    template <typename T> void unscale_cols(const T* xs, const Vecs& v, double* host_out);
     // anchored (FP32 + FP64 refinement) iterations
     void emit_repaired(const LoopOut& out, igaos_pdhg_result& r, double* x, double* y);
     // infeasibility certificates from the change between restart points
