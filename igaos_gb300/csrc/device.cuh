@@ -292,29 +292,6 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Block-wide sum of NV values over NW warps (blockDim.x = 32 NW); result valid
-// in thread 0. `sh` needs NW * NV doubles. Fixed reduction tree -> deterministic.
-template <int NV, int NW = kWarps>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] = warp_sum(v[q]);
-    __syncthreads();
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) sh[w * NV + q] = v[q];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double s = 0.0;
-            for (int k = 0; k < NW; ++k) s += sh[k * NV + q];
-            v[q] = s;
-        }
-    }
-    __syncthreads();
-}
-
 // Sum over a warp, in every lane.
 template <typename T>
 __device__ __forceinline__ T lanes_sum(T v) {
@@ -331,34 +308,49 @@ __device__ __forceinline__ T lanes_sum2(T v0, T v1) {
     for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
+// Four sums at once, each in that order, in lanes 0, 8, 16 and 24.
+template <typename T>
+__device__ __forceinline__ T lanes_sum4(T v0, T v1, T v2, T v3) {
+    const bool up = threadIdx.x & 16, up8 = threadIdx.x & 8;
+    T a0 = up ? v2 : v0, a1 = up ? v3 : v1;
+    a0 += __shfl_xor_sync(0xffffffffu, up ? v0 : v2, 16);
+    a1 += __shfl_xor_sync(0xffffffffu, up ? v1 : v3, 16);
+    T s = up8 ? a1 : a0;
+    s += __shfl_xor_sync(0xffffffffu, up8 ? a0 : a1, 8);
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
 
-// Same tree in the working precision (FP32 partials of FP32 kernels; the
-// cross-CTA finish is FP64). `sh` needs NW * NV values of type T.
+// Block-wide sums of NV (1 to 4) values of type T over NW warps (blockDim.x
+// = 32 NW); results valid in thread 0. `sh` needs NW * NV values of type T.
+// Fixed reduction tree -> deterministic: the warps' sums as lanes_sum takes
+// them, then in the order of the warps. An FP64 addition occupies its SMSP's
+// unit for 64 cycles however few lanes it has, so the values share the
+// additions, a lane each.
 template <typename T, int NV, int NW = kWarps>
 __device__ __forceinline__ void block_sum_t(T (&v)[NV], T* sh) {
+    static_assert(NV >= 1 && NV <= 4, "one to four values");
+    constexpr int kApart = NV == 3 ? 8 : 32 / NV;  // lanes between the warp's sums
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if constexpr (NV == 2) {
-        const T s = lanes_sum2(v[0], v[1]);
-        __syncthreads();
-        if ((lane & 15) == 0) sh[w * 2 + (lane >> 4)] = s;
-    } else {
+    T s;
+    if constexpr (NV == 1) s = lanes_sum(v[0]);
+    else if constexpr (NV == 2) s = lanes_sum2(v[0], v[1]);
+    else s = lanes_sum4(v[0], v[1], v[2], NV == 4 ? v[NV - 1] : T(0));
+    __syncthreads();
+    if (lane % kApart == 0 && lane / kApart < NV) sh[w * NV + lane / kApart] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = 0;
+        if (lane < NV)
+            for (int k = 0; k < NW; ++k) s += sh[k * NV + lane];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) v[q] = lanes_sum(v[q]);
-        __syncthreads();
-        if (lane == 0)
-#pragma unroll
-            for (int q = 0; q < NV; ++q) sh[w * NV + q] = v[q];
+        for (int q = 0; q < NV; ++q) v[q] = __shfl_sync(0xffffffffu, s, q);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            T s = 0;
-            for (int k = 0; k < NW; ++k) s += sh[k * NV + q];
-            v[q] = s;
-        }
-    }
-    __syncthreads();
+}
+template <int NV, int NW = kWarps>
+__device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
+    block_sum_t<double, NV, NW>(v, sh);
 }
 
 template <int NV, int NW = kWarps>

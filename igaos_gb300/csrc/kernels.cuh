@@ -818,21 +818,39 @@ __global__ void __launch_bounds__(kThreads) k_kkt_rows(KktArgs<T> a, int m) {
     const double* __restrict__ axv = a.ax[v];
     double pv = 0.0, pa = 0.0, prow = 0.0, ymax = 0.0;
     // comparisons on the integer pipe (dmax, dmin, ...; see device.cuh)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-        const double Ax = axv[i] * a.dr[i];
-        const double lo = a.rmin[i], hi = a.rmax[i];
-        const double vi = dmax(lo - Ax, Ax - hi);
-        pv = dmax(pv, vi);
-        pa = dmax(pa, dabs(dmin(dmax(Ax, lo), hi)));
-        // vi / (1 + sc) <= vi: the FP64 division only when vi beats this
-        // thread's running maximum (with prow = 0 that is vi > 0)
-        if (dlt(prow, vi)) {
-            double sc = dabs(Ax);
-            if (dfinite(lo)) sc = dmax(sc, dabs(lo));
-            if (dfinite(hi)) sc = dmax(sc, dabs(hi));
-            prow = dmax(prow, vi / (1.0 + sc));
+    // (four rows' loads in flight: a small LP has that many per thread)
+    const int step = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < m; i0 += 4 * step) {
+        double av[4], dr[4], lo4[4], hi4[4], idr[4];
+        T y4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * step < m ? i0 + u * step : i0;
+            av[u] = axv[i];
+            dr[u] = a.dr[i];
+            lo4[u] = a.rmin[i];
+            hi4[u] = a.rmax[i];
+            y4[u] = yv[i];
+            idr[u] = a.idr[i];
         }
-        ymax = dmax(ymax, dabs((double)yv[i] * a.idr[i]));
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (i0 + u * step >= m) break;
+            const double Ax = av[u] * dr[u];
+            const double lo = lo4[u], hi = hi4[u];
+            const double vi = dmax(lo - Ax, Ax - hi);
+            pv = dmax(pv, vi);
+            pa = dmax(pa, dabs(dmin(dmax(Ax, lo), hi)));
+            // vi / (1 + sc) <= vi: the FP64 division only when vi beats this
+            // thread's running maximum (with prow = 0 that is vi > 0)
+            if (dlt(prow, vi)) {
+                double sc = dabs(Ax);
+                if (dfinite(lo)) sc = dmax(sc, dabs(lo));
+                if (dfinite(hi)) sc = dmax(sc, dabs(hi));
+                prow = dmax(prow, vi / (1.0 + sc));
+            }
+            ymax = dmax(ymax, dabs((double)y4[u] * idr[u]));
+        }
     }
     double r[4] = {pv, pa, prow, ymax};
     block_dmax<4>(r, smred);
@@ -867,14 +885,28 @@ __global__ void __launch_bounds__(kThreads) k_kkt_cols(KktArgs<T> a, int n, int 
     double dv = 0.0, op = 0.0, od = 0.0, unb = 0.0;
     // comparisons on the integer pipe, at-bound bands precomputed (k_bands);
     // the reduced cost multiplies by 1/dc instead of dividing by dc
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-        const double d = a.c[j] + atyv[j] * a.idc[j];
-        const double x = unscale_x(xv[j], a.slo[j], a.shi[j], a.dc[j], a.cl[j], a.cu[j]);
-        const double cl = a.cl[j], cu = a.cu[j];
+    struct Col {
+        double c, aty, idc, dc, cl, cu, lob, hib;
+        T x, slo, shi;
+    };
+    auto load = [&](int j) {
+        return Col{a.c[j],  atyv[j],  a.idc[j], a.dc[j],  a.cl[j], a.cu[j],
+                   a.lob[j], a.hib[j], xv[j],    a.slo[j], a.shi[j]};
+    };
+    const int step = gridDim.x * blockDim.x;
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    Col ahead{};
+    if (j < n) ahead = load(j);
+    for (; j < n; j += step) {  // the next column's loads in flight
+        const Col v = ahead;
+        if (j + step < n) ahead = load(j + step);
+        const double d = v.c + v.aty * v.idc;
+        const double cl = v.cl, cu = v.cu;
+        const double x = unscale_x(v.x, v.slo, v.shi, v.dc, cl, cu);
         const bool pos = dgt0(d), neg = dlt0(d);
-        const bool excused = (pos && !dlt(a.lob[j], x)) || (neg && !dlt(x, a.hib[j]));
+        const bool excused = (pos && !dlt(v.lob, x)) || (neg && !dlt(x, v.hib));
         if (!excused) dv = dmax(dv, dabs(d));
-        op += a.c[j] * x;
+        op += v.c * x;
         if (!neg) {  // d >= 0
             if (dfinite(cl)) od += d * cl;
             else if (dlt(dz, d)) unb = 1.0;
