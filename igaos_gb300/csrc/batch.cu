@@ -55,13 +55,14 @@ struct BatchDesc {
     long long ap_off, cp_off, nz_off, row_off, col_off;
     long long base_off;  // slice bases (in units of 32 entries): columns'
                          // (slices + 1), then rows'
-    long long out_off;   // kHeldOut: staged entries in global memory
+    long long out_off;   // kHeldOut, kHeldWide: staged entries in global memory
 };
 
-// kHeldOut: everything in global memory. kHeldMatrix: the matrix and the
+// kHeldWide: everything in global memory. kHeldOut: the matrix too (16-bit
+// indices), the gathered vectors in shared memory. kHeldMatrix: the matrix and the
 // gathered vectors in shared memory. kHeldAll: the iterates and the residual
 // data too.
-enum { kHeldOut = 0, kHeldMatrix = 1, kHeldAll = 2 };
+enum { kHeldWide = 0, kHeldOut = 1, kHeldMatrix = 2, kHeldAll = 3 };
 
 __host__ __device__ inline int slices_of(int rows) { return (rows + 31) / 32; }
 // staged values and 16-bit indices, x_bar, both slots of y, A~ x_bar, the
@@ -105,7 +106,7 @@ struct BatchArgs {
     double* cax64;       // original values in CSC order, FP64
     const int *order_c, *order_r;  // columns and rows by decreasing length
     const int* bases;              // first staged entry of each slice of 32 of them
-    float* out_val;                // staged entries of kHeldOut instances
+    float* out_val;                // staged entries of kHeldOut and kHeldWide instances
     int* out_idx;
     float *dr, *dc, *sc, *scl, *scu, *srmin, *srmax, *yh32;
     float *x[2], *xa[2], *xbar, *vt, *g[2], *ab;
@@ -276,11 +277,11 @@ __device__ Inst make_inst(const BatchArgs& a, const BatchDesc& d) {
 // products). Every row's sum keeps the order of its entries.
 template <int MODE>
 struct Held {
-    using Idx = typename std::conditional<MODE == kHeldOut, int, uint16_t>::type;
+    using Idx = typename std::conditional<MODE == kHeldWide, int, uint16_t>::type;
     int m, n;
     const int *cbase, *rbase;
     const uint16_t *cid, *rid;     // row numbers by position, or
-    const int *cid32, *rid32;      // (kHeldOut) these
+    const int *cid32, *rid32;      // (up to kHeldOut) these
     const float *cv, *rv;
     const Idx *ci, *ri;
     float *xbar, *ab, *ys;  // ys: both slots of y
@@ -309,7 +310,7 @@ struct Held {
     __device__ __forceinline__ float* ya(int p) const { return row(3 + p, p ? a->ya[1] : a->ya[0]); }
     __device__ __forceinline__ float* axc(int p) const { return row(5 + p, p ? a->axc[1] : a->axc[0]); }
     __device__ __forceinline__ float* y(int p) const {
-        if constexpr (MODE == kHeldOut) return (p ? a->y[1] : a->y[0]) + r0;
+        if constexpr (MODE == kHeldWide) return (p ? a->y[1] : a->y[0]) + r0;
         else return ys + p * m;
     }
 };
@@ -326,7 +327,7 @@ __device__ __forceinline__ Held<MODE> make_work(const BatchArgs& a, const BatchD
     W.r0 = d.row_off;
     W.cols = W.rows = W.ys = nullptr;
     const int sc = slices_of(n), sr = slices_of(m);
-    if constexpr (MODE == kHeldOut) {
+    if constexpr (MODE <= kHeldOut) {
         W.cbase = a.bases + d.base_off;
         W.rbase = W.cbase + sc + 1;
         W.cid = W.rid = nullptr;
@@ -334,9 +335,14 @@ __device__ __forceinline__ Held<MODE> make_work(const BatchArgs& a, const BatchD
         W.rid32 = a.order_r + d.row_off;
         W.cv = a.out_val + d.out_off;
         W.rv = W.cv + d.pad_c;
-        W.ci = a.out_idx + d.out_off;
+        W.ci = reinterpret_cast<const typename Held<MODE>::Idx*>(a.out_idx + d.out_off);
         W.ri = W.ci + d.pad_c;
-        W.xbar = a.xbar + d.col_off;
+        if constexpr (MODE == kHeldOut) {
+            W.xbar = reinterpret_cast<float*>(smem);
+            W.ys = W.xbar + n;
+        } else {
+            W.xbar = a.xbar + d.col_off;
+        }
         W.ab = a.ab + d.row_off;
     } else {
         float* v = reinterpret_cast<float*>(smem);
@@ -371,7 +377,7 @@ __device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, 
     const int sc = slices_of(I.n), sr = slices_of(I.m);
     const int* order[2] = {a.order_c + d.col_off, a.order_r + d.row_off};
     const int* bases = a.bases + d.base_off;
-    if constexpr (MODE != kHeldOut) {
+    if constexpr (MODE > kHeldOut) {
         for (int s = t; s < sc + sr + 2; s += blockDim.x) const_cast<int*>(W.cbase)[s] = bases[s];
         for (int j = t; j < I.n; j += blockDim.x)
             const_cast<uint16_t*>(W.cid)[j] = (uint16_t)order[0][j];
@@ -403,22 +409,30 @@ __device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, 
 
 // The products of the lane's staged row (slice entries 32 b0 .. 32 b1) with
 // v, compensated FP32, in the order of the entries.
-template <class Idx>
+template <bool OUT, class Idx>
 __device__ __forceinline__ Acc<float> padded_dot(const Idx* idx, const float* val,
                                                  const float* __restrict__ v, int b0, int b1) {
-    using At = typename std::conditional<std::is_same<Idx, int>::value, long long, int>::type;
+    using At = typename std::conditional<OUT, long long, int>::type;
+    constexpr int kAhead = OUT ? 4 : 2;  // loads in flight
     At at = 32 * (At)b0 + (threadIdx.x & 31);
     int left = b1 - b0;
     Acc<float> acc;
 #pragma unroll 1
-    for (; left >= 2; left -= 2, at += 64) {
-        const float a0 = val[at], a1 = val[at + 32];
-        const int j0 = idx[at], j1 = idx[at + 32];
-        const float x0 = v[j0], x1 = v[j1];
-        acc.add(a0, x0);
-        acc.add(a1, x1);
+    for (; left >= kAhead; left -= kAhead, at += 32 * kAhead) {
+        float w[kAhead], x[kAhead];
+        int j[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            w[u] = val[at + 32 * u];
+            j[u] = idx[at + 32 * u];
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) x[u] = v[j[u]];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) acc.add(w[u], x[u]);
     }
-    if (left) acc.add(val[at], v[idx[at]]);
+#pragma unroll 1
+    for (; left; --left, at += 32) acc.add(val[at], v[idx[at]]);
     return acc;
 }
 
@@ -627,9 +641,9 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
     double mx[2][4] = {};  // pv, pa, prow, ymax
     for (int s = wp; works && 32 * s < I.m; s += nw) {
         const int q = 32 * s + lane;
-        const int i = q < I.m ? (MODE == kHeldOut ? W.rid32[q] : (int)W.rid[q]) : I.m;
+        const int i = q < I.m ? (MODE <= kHeldOut ? W.rid32[q] : (int)W.rid[q]) : I.m;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = padded_dot(W.ri, W.rv, xs[v], W.rbase[s], W.rbase[s + 1]);
+            const Acc<float> ad = padded_dot<MODE <= kHeldOut>(W.ri, W.rv, xs[v], W.rbase[s], W.rbase[s + 1]);
             if (i >= I.m) continue;
             const double Ax = (I.axh[i] + ad.result_d()) * (double)I.dr[i];
             const double lo = I.rmin[i], hi = I.rmax[i];
@@ -669,9 +683,9 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
     bool unb[2] = {false, false};
     for (int s = wp; works && 32 * s < I.n; s += nw) {
         const int q = 32 * s + lane;
-        const int j = q < I.n ? (MODE == kHeldOut ? W.cid32[q] : (int)W.cid[q]) : I.n;
+        const int j = q < I.n ? (MODE <= kHeldOut ? W.cid32[q] : (int)W.cid[q]) : I.n;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = padded_dot(W.ci, W.cv, ys[v], W.cbase[s], W.cbase[s + 1]);
+            const Acc<float> ad = padded_dot<MODE <= kHeldOut>(W.ci, W.cv, ys[v], W.cbase[s], W.cbase[s + 1]);
             if (j >= I.n) continue;
             const double dcj = I.dc[j], cj = I.c[j];
             const double aty = I.atyh[j] + ad.result_d();
@@ -826,7 +840,7 @@ __device__ __forceinline__ void lanes_merge(Acc<float> (&v)[NV]) {
 
 // Products of the staged rows: out[id] = row id times v, in the order of its
 // entries (compensated FP32), a warp per slice.
-template <class Idx>
+template <bool OUT, class Idx>
 __device__ __forceinline__ void slice_products(const int* base, const uint16_t* id16,
                                                const int* id32, const Idx* idx, const float* val,
                                                const float* __restrict__ v, float* out,
@@ -835,7 +849,7 @@ __device__ __forceinline__ void slice_products(const int* base, const uint16_t* 
     for (int s = threadIdx.x >> 5; 32 * s < rows; s += warps) {
         const int q = 32 * s + lane;
         const int row = q < rows ? (id16 ? (int)id16[q] : id32[q]) : -1;
-        const Acc<float> acc = padded_dot(idx, val, v, base[s], base[s + 1]);
+        const Acc<float> acc = padded_dot<OUT>(idx, val, v, base[s], base[s + 1]);
         if (row >= 0) out[row] = acc.result();
     }
 }
@@ -875,7 +889,7 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
             lanes_merge(dx2);
             if (lane == 0) sh.acc[wp * 3] = dx2[0];
         }
-        slice_products(W.rbase, W.rid, W.rid32, W.ri, W.rv, W.xbar, W.ab, m);
+        slice_products<MODE <= kHeldOut>(W.rbase, W.rid, W.rid32, W.ri, W.rv, W.xbar, W.ab, m);
         cta_sync();
         {   // dual step; the projection acts on the full value, so the anchor
             // enters its argument
@@ -910,7 +924,7 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
             }
         }
         cta_sync();
-        slice_products(W.cbase, W.cid, W.cid32, W.ci, W.cv, W.y(q), W.g(q), n);
+        slice_products<MODE <= kHeldOut>(W.cbase, W.cid, W.cid32, W.ci, W.cv, W.y(q), W.g(q), n);
         cta_sync();
         if (sh.step.done) return;
         if (!sh.step.check) continue;
@@ -1180,18 +1194,27 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
 // Classes of instances: threads, CTAs per SM the kernel is compiled
 // for, and the shared memory that leaves that many resident. An instance goes
 // to the first class whose threads reach its columns and rows (or are kBT) and
-// whose shared memory holds it; the last class takes the rest.
+// whose shared memory holds it; kTight takes the matrices without their vectors
+// too, and the last class the instances in global memory: apart, because its
+// CTAs leave their SM's memory to L1, which serves them. In one class with
+// instances of 226 KB, 4,096 LPs of 20 to 2,000 rows took 18.5 s, 14.4 before
+// classes; 11.6 now (an iteration of an LP of 1,886 rows 98 us before, now 52).
 struct BatchClass {
     int threads, ctas;  // threads: without the decision warp
     size_t smem;
 };
-constexpr int kClasses = 4;
-constexpr BatchClass kClass[kClasses] = {
-    {128, 6, 36 * 1024}, {256, 4, 55 * 1024}, {512, 2, 112 * 1024}, {512, 1, 226 * 1024}};
+constexpr int kClasses = 5, kTight = 3;
+constexpr BatchClass kClass[kClasses] = {{128, 6, 36 * 1024},
+                                         {256, 4, 55 * 1024},
+                                         {512, 2, 112 * 1024},
+                                         {512, 1, 226 * 1024},
+                                         {512, 1, 110 * 1024}};
 
 size_t held_bytes(const BatchDesc& d, int mode) {
     return kSharedHead +
-           (mode == kHeldOut ? 0 : matrix_bytes(d) + (mode == kHeldAll ? state_bytes(d) : 0));
+           (mode == kHeldWide  ? 0
+            : mode == kHeldOut ? 4 * ((size_t)d.n + 2 * (size_t)d.m)
+                               : matrix_bytes(d) + (mode == kHeldAll ? state_bytes(d) : 0));
 }
 
 // Rows by decreasing length into `order` (counting sort, stable), and the
@@ -1226,11 +1249,14 @@ __global__ void __launch_bounds__(kClass[K].threads + 32, kClass[K].ctas)
         if (qi >= a.count) break;
         const int b = a.order[qi];
         if (a.desc[b].m <= 0 || a.desc[b].n <= 0) continue;
-        const int mode = a.desc[b].mode;
-        if (K < kClasses - 1 || mode == kHeldAll) solve_one<kHeldAll>(a, b);
-        else if constexpr (K == kClasses - 1) {
-            if (mode == kHeldMatrix) solve_one<kHeldMatrix>(a, b);
-            else solve_one<kHeldOut>(a, b);
+        if constexpr (K < kTight) {
+            solve_one<kHeldAll>(a, b);
+        } else if constexpr (K == kTight) {
+            if (a.desc[b].mode == kHeldAll) solve_one<kHeldAll>(a, b);
+            else solve_one<kHeldMatrix>(a, b);
+        } else {
+            if (a.desc[b].mode == kHeldOut) solve_one<kHeldOut>(a, b);
+            else solve_one<kHeldWide>(a, b);
         }
     }
 }
@@ -1332,11 +1358,13 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             const int reach = std::max(d.m, d.n);
             int k = 0;
             d.mode = kHeldAll;
-            while (k < kClasses - 1 && ((reach > kClass[k].threads && kClass[k].threads < kBT) ||
-                                        held_bytes(d, kHeldAll) > kClass[k].smem))
+            while (k < kTight && ((reach > kClass[k].threads && kClass[k].threads < kBT) ||
+                                  held_bytes(d, kHeldAll) > kClass[k].smem))
                 ++k;
             while (held_bytes(d, d.mode) > kClass[k].smem) --d.mode;
-            if (d.mode == kHeldOut) {
+            if (d.mode <= kHeldOut) {
+                k = kClasses - 1;
+                if (held_bytes(d, kHeldOut) > kClass[k].smem || reach > 0xffff) d.mode = kHeldWide;
                 d.out_off = out_off;
                 out_off += d.pad_c + d.pad_r;
             }
@@ -1453,7 +1481,8 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         CU(cudaEventCreate(&fk.e[kClasses]));
         CU(cudaEventCreate(&fk.e[kClasses + 1]));
         CU(cudaEventRecord(fk.e[kClasses], st));
-        void (*const kernels[kClasses])(BatchArgs) = {k_batch<0>, k_batch<1>, k_batch<2>, k_batch<3>};
+        void (*const kernels[kClasses])(BatchArgs) = {k_batch<0>, k_batch<1>, k_batch<2>,
+                                                         k_batch<3>, k_batch<4>};
         bool first = true;
         for (int k = kClasses - 1; k >= 0; --k) {
             if (cls_count[k] == 0) continue;

@@ -50,3 +50,15 @@ def test_classes_against_single_solves(native):
             continue
         assert a["iterations"] == b["iterations"], (lp.m, lp.n)
         assert np.array_equal(a["x"], b["x"]) and np.array_equal(a["y"], b["y"]), (lp.m, lp.n)
+
+
+@pytest.mark.parametrize("m,n", [(40, 29000), (30, 66000)])
+def test_instances_wider_than_the_gathered_vectors_shared_memory(native, m, n):
+    """Beside an instance of the same class whose gathered vectors fit."""
+    from igaos_gb300 import capi
+    lps = [lp_of(m, n, 2e-3, 5), lp_of(130, 420, 0.7, 6)]
+    out = capi.solve_batch(lps, tolerance=1e-6, max_iterations=200000)
+    for lp, r in zip(lps, out):
+        want = capi.solve_lp(lp, tolerance=1e-6, time_limit=60.0, precision="fp64")
+        assert r["status_name"] == want["status_name"] == "near-optimal", (lp.m, lp.n, r, want["message"])
+        assert abs(r["objective"] - want["objective"]) <= 2e-5 * max(1.0, abs(want["objective"])), (lp.m, lp.n)
