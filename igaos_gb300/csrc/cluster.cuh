@@ -5,8 +5,8 @@
 // dependent L2 loads (schedule -> row pointer -> entries -> gathers ->
 // partials) and on the step decision. One cluster of C CTAs (1 to 16) instead
 // runs the whole chunk in one launch, with the LP and its iterates on chip:
-//   * each CTA stages its rows of A~ and A~^T (row pointers, 16-bit indices,
-//     values) and their vectors (both parity slots of the iterates, bounds,
+//   * each CTA stages its rows of A~ and A~^T (16-bit indices and values, lane
+//     by lane) and their vectors (both parity slots of the iterates, bounds,
 //     costs) in shared memory once per launch, and writes the accepted
 //     iterates back at its end;
 //   * every CTA keeps a replica of the gathered vectors (xbar and both parity
@@ -47,11 +47,6 @@ constexpr int kSmallMaxItems = kSmallVirtual * kSmallItems;
 __device__ __forceinline__ int cluster_rank() {
     unsigned r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return (int)r;
-}
-__device__ __forceinline__ int cluster_count() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return (int)r;
 }
 // All threads of every CTA of the cluster, in two halves; release/acquire at
@@ -213,8 +208,9 @@ __device__ __forceinline__ double small_total(const double* v, int pad) {
 // operations of one warp at 60 cycles and more each (its SMSP's unit takes a
 // warp through in 64), so only what the next half waits for stands before a
 // barrier's arrival: the averages and ||dx||^2 are formed behind it. 2,048 FP32
-// iterations of a 2,000 x 5,000 LP: 19.5 -> 14.8 ms (with one deciding CTA, its
-// answer published behind a third barrier, and the vectors in global memory).
+// iterations of a 2,000 x 5,000 LP: 19.5 -> 12.9 ms (with one deciding CTA, its
+// answer published behind a third barrier, the vectors in global memory and
+// entries by row pointers).
 template <typename T, bool HELD>
 __global__ void __launch_bounds__(kSmallThreads, 1)
     k_attempts_cluster(PrimalArgs<T> pa, DualArgs<T> da, int m, int n, int max_attempts,

@@ -177,12 +177,14 @@ static bool small_lp(int m, int n, const int* pa, const std::vector<int>& wa, co
     return true;
 }
 
-// The smallest cluster that holds the LP with at most 8 virtual warps a CTA (two
-// per SMSP); else the largest that holds it, in FP32 one of 8; else, in FP32, one
-// that holds the matrix only. 1,024 iterations of a 300 x 700 LP (22 virtual
-// warps) on 2, 4 and 8 CTAs: FP64 9.4, 7.6, 7.4 ms, FP32 6.4, 5.9, 5.9; of a
-// 60 x 150 LP (5) on 1 and 2: 8.1, 8.6; 2,048 FP32 ones of a 2,000 x 5,000 LP (128)
-// on 8 and 16: 14.8, 15.2.
+// The smallest cluster that holds the LP with at most 8 virtual warps a CTA, in
+// FP64 5 (about one per SMSP, each with an FP64 unit that takes a warp through
+// in 64 cycles) unless one CTA does without releases; else the largest that holds it, in FP32 one of 8; else, in
+// FP32, one that holds the matrix only. 1,024 iterations on 1, 2, 4, 8 and 16
+// CTAs, ms: a 300 x 700 LP (22 virtual warps) FP64 11.3, 8.3, 6.7, 6.4, 6.6, FP32
+// 5.2, 5.3, 4.9, 4.9, 5.1; a 60 x 150 LP (5) from host arrays 6.4, 6.9, 6.8, 6.8,
+// 6.9; 2,048 FP32 ones of a 2,000 x 5,000 LP (128) on 4, 8 and 16: 14.8, 12.5,
+// 13.1; 1,024 FP64 ones of it (157) on 8 and 16: 11.8, 9.8.
 template <typename T>
 static SmallPlan small_plan(int m, int n, const int* pa, const std::vector<int>& wa,
                             const std::vector<unsigned char>& la, const int* pat,
@@ -208,7 +210,8 @@ static SmallPlan small_plan(int m, int n, const int* pa, const std::vector<int>&
             p.bytes = small_bytes<T>(m, n, p);
             if (p.bytes > kSmallSmemMax || !cluster_fits<T>(p)) continue;
             best = p;
-            if (8 * ctas >= std::max(p.virt_at, p.virt_a) || (f32 && ctas >= 8)) break;
+            const int most = f32 || ctas == 1 ? 8 : 5;
+            if (most * ctas >= std::max(p.virt_at, p.virt_a) || (f32 && ctas >= 8)) break;
         }
     return best;
 }
@@ -402,8 +405,8 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         sAT_ = candAT_[def_sched()] = sRAT_;
         // small LPs: the attempts of a chunk in one thread-block cluster with
         // the LP in its shared memory (cluster.cuh): 1,024 FP64 iterations
-        // of a 60 x 150 LP take 8.1 ms, 14.7 with the grid-wide kernels;
-        // of a 2,000 x 5,000 LP 11.0 and 15.5.
+        // of a 60 x 150 LP take 6.4 ms, 14.2 with the grid-wide kernels;
+        // of a 2,000 x 5,000 LP 9.8 and 14.7.
         // IGAOS_PDHG_CLUSTER=0: never.
         const char* e = std::getenv("IGAOS_PDHG_CLUSTER");
         if (!(e && std::strcmp(e, "0") == 0) && !wa.empty()) {
@@ -922,9 +925,9 @@ static void touch_pages(double* v, size_t len) {
 // or NaN). The first batch covers the accepted iterations still needed plus
 // the rejections the history predicts; the rest are topped up in small
 // batches (a stopped launch is a no-op); one cluster's launch covers any number
-// of rejections (it ends at the stop). With `check`, the KKT pass of the two
-// candidates is enqueued behind each batch and its metrics come with the
-// control block, in h_met_.
+// of rejections (it ends at the stop, or after tens of milliseconds). With
+// `check`, the KKT pass of the two candidates is enqueued behind each batch and
+// its metrics come with the control block, in h_met_.
 template <typename T>
 void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out, bool check) {
     for (;;) {
@@ -936,7 +939,7 @@ void Engine::run_until_stop(const Vecs& v, bool graphs, LoopOut& out, bool check
         int cnt = want <= 1 ? 1 : want <= 4 ? 4 : want <= 8 ? 8 : want <= 16 ? 16
                   : want <= 32 ? 32 : want <= 64 ? 64 : want <= 72 ? 72 : want <= 80 ? 80 : 96;
         if (small_[std::is_same<T, double>::value ? 1 : 0].ctas)
-            cnt = (int)std::min<long long>(1 << 30, 32 * std::max(1LL, need));
+            cnt = (int)std::min<long long>(1 << 13, 32 * std::max(1LL, need));
         CU(cudaEventRecord(ev_[2], st_));
         launch_attempts<T>(cnt, v, graphs);
         CU(cudaEventRecord(ev_[3], st_));

@@ -123,7 +123,8 @@ typedef struct igaos_pdhg_options {
      * 8, 16 and 32 entries per lane (8 launches each; FP64 kernels
      * also at 3 and 4 resident CTAs per SM) and the fastest is kept for that
      * handle and precision; the result's entries_a / entries_at report the
-     * choice. The schedule changes the order of each
+     * choice (LPs small enough to run in one thread-block cluster keep the
+     * fixed one). The schedule changes the order of each
      * row's sum, so results match the fixed schedule's to rounding, not bit
      * for bit, and two handles may choose differently. Added in ABI 4. */
     int schedule;
