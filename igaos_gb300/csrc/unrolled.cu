@@ -1147,10 +1147,16 @@ UArgs<T> base_args(const igaos_pdhg_unrolled_layout* L) {
     return a;
 }
 
+// static shared memory of the layer kernels stays below this
+constexpr size_t kStaticSmem = 1024;
+
+// Lets a kernel's launches take any size up to the device's limit. The
+// attribute belongs to the kernel, not to a launch: set to one launch's size, it
+// made another host thread's larger launch fail.
 template <typename K>
-cudaError_t set_smem(K kernel, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+cudaError_t allow_smem(K kernel, const Device& dev) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                dev.optin - (int)kStaticSmem);
 }
 
 int too_large(size_t need, int optin) {
@@ -1160,9 +1166,6 @@ int too_large(size_t need, int optin) {
                   "per CTA, device allows %d", need, optin);
     return igx_set_error(IGAOS_PDHG_ERR_INVALID, buf);
 }
-
-// static shared memory of the layer kernels stays below this
-constexpr size_t kStaticSmem = 1024;
 
 enum Pass { kSteps, kForward, kBackward };
 
@@ -1200,7 +1203,7 @@ int resident_clusters(void (*kernel)(UArgs<T>), Pass pass, const Device& dev, in
     int n = 0;
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = cluster_config(at, C, C, threads, smem, nullptr);
-    if (set_smem(kernel, smem) != cudaSuccess ||
+    if (allow_smem(kernel, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, (const void*)kernel, &cfg) != cudaSuccess) {
         cudaGetLastError();
         n = 0;
@@ -1279,9 +1282,9 @@ Launch plan(void (*kernel)(UArgs<T>), const igaos_pdhg_unrolled_layout* L, Pass 
 // One cluster of C CTAs per instance.
 template <typename T>
 cudaError_t launch(void (*kernel)(UArgs<T>), const Launch& l, int count, const UArgs<T>& a,
-                   cudaStream_t st) {
+                   const Device& dev, cudaStream_t st) {
     if (l.C == 0) return cudaErrorInvalidConfiguration;
-    const cudaError_t e = set_smem(kernel, l.smem);
+    const cudaError_t e = allow_smem(kernel, dev);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg =
@@ -1298,7 +1301,7 @@ int run_steps(const igaos_pdhg_unrolled_layout* L, const void* ax, double omega,
     a.sigma_o = static_cast<T*>(sigma);
     a.omega = (T)omega;
     const Launch l = plan<T>(k_unroll_steps<T>, L, kSteps, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_steps<T>, l, L->count, a, st);
+    const cudaError_t e = launch<T>(k_unroll_steps<T>, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
@@ -1321,7 +1324,7 @@ int run_forward(const igaos_pdhg_unrolled_layout* L, const void* c, const void* 
     a.obj = static_cast<T*>(obj);
     a.ckpt = static_cast<T*>(ckpt);
     const Launch l = plan<T>(k_unroll_fwd<T>, L, kForward, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_fwd<T>, l, L->count, a, st);
+    const cudaError_t e = launch<T>(k_unroll_fwd<T>, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
@@ -1357,7 +1360,7 @@ int run_backward(const igaos_pdhg_unrolled_layout* L, const void* c, const void*
     a.seg = static_cast<T*>(work);
     a.segf = static_cast<unsigned char*>(work) + vb;
     const Launch l = plan<T>(k_unroll_bwd<T>, L, kBackward, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_bwd<T>, l, L->count, a, st);
+    const cudaError_t e = launch<T>(k_unroll_bwd<T>, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
