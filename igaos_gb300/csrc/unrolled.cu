@@ -495,6 +495,7 @@ __device__ __forceinline__ U row_dot(const Share<T>& S, int l, int q, const U* _
         if constexpr (kTwo) acc += odd;
     } else {
         const int p0 = len > 0 ? S.ptr[S.id[q]] : 0;
+        U odd = U(0);
         for (; k < len; k += 4) {
             U a[4], x[4];
 #pragma unroll
@@ -505,8 +506,12 @@ __device__ __forceinline__ U row_dot(const Share<T>& S, int l, int q, const U* _
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (k + u < len) acc = fma(a[u], x[u], acc);
+                if (k + u < len) {
+                    if (kTwo && (u & 1)) odd = fma(a[u], x[u], odd);
+                    else acc = fma(a[u], x[u], acc);
+                }
         }
+        if constexpr (kTwo) acc += odd;
         __syncwarp();
     }
     return acc;
