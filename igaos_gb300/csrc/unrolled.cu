@@ -74,6 +74,7 @@ struct UArgs {
     int ngc, ngr;              // entries of a gathered column and row vector
     int per_cta;               // row entries of a CTA of the largest instance
     int vec_bytes, ent_bytes;  // shared memory of the vectors, and of the staged entries
+    bool lean;                 // backward: see bwd_elems
 };
 
 struct UInst {
@@ -485,12 +486,15 @@ __device__ __forceinline__ U row_dot(const Share<T>& S, int l, int q, const U* _
 #pragma unroll
             for (int u = 0; u < 4; ++u) x[u] = v[j[u]];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < 4; ++u) {
+                // (uniform: an FP64 instruction takes its slot with no lane on)
+                if (sizeof(U) == 8 && k + u >= longest) break;
                 if (k + u < len) {
                     if constexpr (std::is_same<T, U>::value) acc = fma(a[u], x[u], acc);
                     else if (u & 1) odd = fma(u_wide(a[u]), x[u], odd);
                     else acc = fma(u_wide(a[u]), x[u], acc);
                 }
+            }
         }
         if constexpr (kTwo) acc += odd;
     } else {
@@ -548,11 +552,10 @@ __device__ __forceinline__ FwdVec<T> fwd_vec(const UArgs<T>& a, unsigned char* b
 
 // one column's primal step, q its local position; returns the clamp outcome
 template <bool RES, typename T>
-__device__ __forceinline__ int fwd_col(const Plan<T>& P, int l, int q, T* x, const T* c,
-                                       const T* lo, const T* hi, T* xb, const T* y, T tau,
-                                       T kappa, int C, T& xbv) {
-    const T xv = x[q], l0 = lo[q], h0 = hi[q];
-    const T g = row_dot<RES, T, T>(P.col, l, q, y, c[q]);
+__device__ __forceinline__ int fwd_col(const Plan<T>& P, int l, int q, T* x, T c, T l0, T h0, T* xb,
+                                       const T* y, T tau, T kappa, int C, T& xbv) {
+    const T xv = x[q];
+    const T g = row_dot<RES, T, T>(P.col, l, q, y, c);
     const T v = (xv - tau * g) * kappa;
     int f;
     const T xn = clampf(v, l0, h0, f);
@@ -564,10 +567,8 @@ __device__ __forceinline__ int fwd_col(const Plan<T>& P, int l, int q, T* x, con
 
 // one row's dual step from its dual yv; returns the clamp outcome
 template <bool RES, typename T>
-__device__ __forceinline__ int fwd_row(const Plan<T>& P, int l, int q, const T* rl,
-                                       const T* rh, const T* xb, T* y, T yv, T sigma, T isigma,
-                                       int C) {
-    const T l0 = rl[q], h0 = rh[q];
+__device__ __forceinline__ int fwd_row(const Plan<T>& P, int l, int q, T l0, T h0, const T* xb, T* y,
+                                       T yv, T sigma, T isigma, int C) {
     const T z = row_dot<RES, T, T>(P.row, l, q, xb, T(0));
     const T t = fma(sigma, z, yv);
     int f;
@@ -621,13 +622,13 @@ __device__ void fwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
         for (int l = wp; l < P.col.slices; l += nw) {
             const int q = 32 * l + lane;
             T xb;
-            fwd_col<RES>(P, l, q, V.x, V.c, V.lo, V.hi, V.xb, V.y, tau, kappa, C, xb);
+            fwd_col<RES>(P, l, q, V.x, V.c[q], V.lo[q], V.hi[q], V.xb, V.y, tau, kappa, C, xb);
         }
         u_sync(C);
         for (int l = wp; l < P.row.slices; l += nw) {
             const int q = 32 * l + lane;
             const T yv = V.y[P.row.first + q];
-            fwd_row<RES>(P, l, q, V.rl, V.rh, V.xb, V.y, yv, sigma, isigma, C);
+            fwd_row<RES>(P, l, q, V.rl[q], V.rh[q], V.xb, V.y, yv, sigma, isigma, C);
         }
         u_sync(C);
     }
@@ -694,11 +695,13 @@ struct BwdVec {
     T *xb, *x, *y;                       // replay: copy and x (gp's space); copy (ngr)
     T* zh;                               // copy (ngr): reverse steps (y's space)
 };
+// Lean: costs and bounds (c, lo, hi, rl, rh) are read where the caller has them
+// instead, in global memory.
 template <typename T>
-__host__ __device__ inline size_t bwd_elems(int lc, int lr, int C) {
-    return (size_t)32 * ((7 + 2 * C) * (size_t)lc + (6 + C) * (size_t)lr);
+__host__ __device__ inline size_t bwd_elems(int lc, int lr, int C, bool lean) {
+    return (size_t)32 * (((lean ? 4 : 7) + 2 * C) * (size_t)lc + ((lean ? 4 : 6) + C) * (size_t)lr);
 }
-template <typename T>
+template <bool LEAN, typename T>
 __device__ __forceinline__ BwdVec<T> bwd_vec(const UArgs<T>& a, unsigned char* base) {
     const int qc = 32 * a.lc, qr = 32 * a.lr;
     T* p = reinterpret_cast<T*>(base);
@@ -706,16 +709,16 @@ __device__ __forceinline__ BwdVec<T> bwd_vec(const UArgs<T>& a, unsigned char* b
     V.gp = reinterpret_cast<typename Pair<T>::type*>(p);
     V.xb = p;
     V.x = p + a.ngc;
-    V.c = p + 2 * (size_t)a.ngc;
-    V.lo = V.c + qc;
-    V.hi = V.lo + qc;
-    V.xh = V.hi + qc;
+    V.xh = p + 2 * (size_t)a.ngc;
     V.gc = V.xh + qc;
     V.gl = V.gc + qc;
     V.gu = V.gl + qc;
-    V.rl = V.gu + qc;
-    V.rh = V.rl + qr;
-    V.yh = V.rh + qr;
+    V.c = V.gu + qc;
+    V.lo = V.c + (LEAN ? 0 : qc);
+    V.hi = V.lo + (LEAN ? 0 : qc);
+    V.rl = V.hi + (LEAN ? 0 : qc);
+    V.rh = V.rl + (LEAN ? 0 : qr);
+    V.yh = V.rh + (LEAN ? 0 : qr);
     V.th = V.yh + qr;
     V.grl = V.th + qr;
     V.grh = V.grl + qr;
@@ -723,12 +726,12 @@ __device__ __forceinline__ BwdVec<T> bwd_vec(const UArgs<T>& a, unsigned char* b
     return V;
 }
 
-template <bool RES, typename T>
+template <bool RES, bool LEAN, typename T>
 __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>& P, int rank,
                          int C) {
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int m = I.m, n = I.n;
-    const BwdVec<T> V = bwd_vec(a, P.vec);
+    const BwdVec<T> V = bwd_vec<LEAN>(a, P.vec);
     const T tau = a.tau[b], sigma = a.sigma[b];
     const T kappa = T(1) / (T(1) + T(2) * a.ridge * tau);
     const T isigma = u_recip(sigma);
@@ -740,21 +743,26 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
         const int q = 32 * l + lane, j = P.col.id[q];
         V.gl[q] = V.gu[q] = T(0);
         if (j == 0xffff) {
-            V.c[q] = V.lo[q] = V.hi[q] = V.xh[q] = V.gc[q] = T(0);
+            if constexpr (!LEAN) V.c[q] = V.lo[q] = V.hi[q] = T(0);
+            V.xh[q] = V.gc[q] = T(0);
             continue;
         }
         const long long gj = I.c0 + j;
         const T xk = a.xK[gj];
-        V.c[q] = a.c[gj];
-        V.lo[q] = a.cl[gj];
-        V.hi[q] = a.cu[gj];
+        if constexpr (!LEAN) {
+            V.c[q] = a.c[gj];
+            V.lo[q] = a.cl[gj];
+            V.hi[q] = a.cu[gj];
+        }
         V.xh[q] = (a.gx ? a.gx[gj] : T(0)) + go * (a.c[gj] + T(2) * a.ridge * xk);
         V.gc[q] = go * xk;
     }
     for (int l = wp; l < P.row.slices; l += nw) {
         const int q = 32 * l + lane, i = P.row.id[q];
-        V.rl[q] = i == 0xffff ? T(0) : a.rmin[I.r0 + i];
-        V.rh[q] = i == 0xffff ? T(0) : a.rmax[I.r0 + i];
+        if constexpr (!LEAN) {
+            V.rl[q] = i == 0xffff ? T(0) : a.rmin[I.r0 + i];
+            V.rh[q] = i == 0xffff ? T(0) : a.rmax[I.r0 + i];
+        }
         V.yh[q] = i != 0xffff && a.gy ? a.gy[I.r0 + i] : T(0);
         V.grl[q] = V.grh[q] = T(0);
         if constexpr (!RES) {
@@ -768,6 +776,30 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
     T* seg = a.seg + (long long)a.ck * (I.c0 + I.r0);
     unsigned char* segf = a.segf + (long long)a.ck * (I.c0 + I.r0);
     const int nseg = (a.K + a.ck - 1) / a.ck;
+    auto costs = [&](int q, int j, T& c, T& l0, T& h0) {  // of column j at q
+        if constexpr (!LEAN) {
+            c = V.c[q];
+            l0 = V.lo[q];
+            h0 = V.hi[q];
+        } else {
+            c = l0 = h0 = T(0);
+            if (j == 0xffff) return;
+            c = a.c[I.c0 + j];
+            l0 = a.cl[I.c0 + j];
+            h0 = a.cu[I.c0 + j];
+        }
+    };
+    auto bounds = [&](int q, int i, T& l0, T& h0) {  // of row i at q
+        if constexpr (!LEAN) {
+            l0 = V.rl[q];
+            h0 = V.rh[q];
+        } else {
+            l0 = h0 = T(0);
+            if (i == 0xffff) return;
+            l0 = a.rmin[I.r0 + i];
+            h0 = a.rmax[I.r0 + i];
+        }
+    };
     auto pos = [&](int l) { return 32 * u_slice(l, rank, C) + lane; };
     for (int s = nseg - 1; s >= 0; --s) {
         const int k0 = s * a.ck, k1 = min(a.K, k0 + a.ck);
@@ -796,7 +828,9 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
                     fk[at] = (unsigned char)f;
                 }
                 const int q = 32 * l + lane, j = P.col.id[q];
-                f = fwd_col<RES>(P, l, q, V.x, V.c, V.lo, V.hi, V.xb, V.y, tau, kappa, C, xb);
+                T c, l0, h0;
+                costs(q, j, c, l0, h0);
+                f = fwd_col<RES>(P, l, q, V.x, c, l0, h0, V.xb, V.y, tau, kappa, C, xb);
                 at = j != 0xffff ? pos(l) : -1;
             }
             u_sync(C);
@@ -812,7 +846,9 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
                 }
                 const int q = 32 * l + lane, i = P.row.id[q];
                 yv = V.y[P.row.first + q];
-                f = fwd_row<RES>(P, l, q, V.rl, V.rh, V.xb, V.y, yv, sigma, isigma, C);
+                T l0, h0;
+                bounds(q, i, l0, h0);
+                f = fwd_row<RES>(P, l, q, l0, h0, V.xb, V.y, yv, sigma, isigma, C);
                 at = i != 0xffff ? n + pos(l) : -1;
             }
             u_sync(C);
@@ -926,8 +962,10 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
                             }
                         }
 #pragma unroll
-                        for (int u = 0; u < 2; ++u)
+                        for (int u = 0; u < 2; ++u) {
+                            if (sizeof(T) == 8 && e + u >= longest) break;
                             if (e + u < len) gax[at[u]] = entry(v[u], ga[u], g[u]);
+                        }
                     }
                 } else {
                     const int p0 = len > 0 ? P.row.ptr[i] : 0;
@@ -946,9 +984,10 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
         const int q = 32 * l + lane, j = P.col.id[q];
         if (j == 0xffff) continue;
         const long long gj = I.c0 + j;
-        T l0 = V.gl[q], u0 = V.gu[q];
-        if (T(0) < V.lo[q]) l0 += V.xh[q];
-        else if (T(0) > V.hi[q]) u0 += V.xh[q];
+        T l0 = V.gl[q], u0 = V.gu[q], c, lo, hi;
+        costs(q, j, c, lo, hi);
+        if (T(0) < lo) l0 += V.xh[q];
+        else if (T(0) > hi) u0 += V.xh[q];
         a.gc[gj] = V.gc[q];
         a.gcl[gj] = l0;
         a.gcu[gj] = u0;
@@ -976,16 +1015,23 @@ __device__ void bwd_body(const UArgs<T>& a, const UInst& I, int b, const Plan<T>
 // The same bounds; the gradient of A's values, read and written once per
 // entry and step, and the pairs' gathers (64 bits each) are the largest share.
 // As above: 1.69 ms against 2.6.
-template <typename T>
-__global__ void __launch_bounds__(kLT) k_unroll_bwd(UArgs<T> a) {
+// OCC: CTAs of kLT threads per SM that it is compiled for, 1: 128 registers, 2:
+// 64 (in FP64 412 bytes spilled). 200 iterations of 1,024 LPs of 150 x 300
+// (2,250 entries): FP32 5.8 ms with the first, 3.7 with the second, FP64 16.6
+// and 13.2; 304 of 500 x 1,000 (one CTA per SM either way) 3.6 and 3.9, 15.3 and
+// 16.5. plan() takes the second where it lets more CTAs reside.
+template <typename T, int OCC>
+__global__ void __launch_bounds__(kLT, OCC) k_unroll_bwd(UArgs<T> a) {
     extern __shared__ __align__(16) unsigned char u_smem[];
     const int rank = u_rank(), b = u_instance();
     const UInst I = uinst(a, b);
     const int C = u_ctas(a, I);
     if (rank >= C) return;
     const Plan<T> P = stage<T, true, false>(a, I, b, u_smem, rank, C);
-    if (P.resident) bwd_body<true>(a, I, b, P, rank, C);
-    else bwd_body<false>(a, I, b, P, rank, C);
+    if (P.resident && !a.lean) bwd_body<true, false>(a, I, b, P, rank, C);
+    else if (P.resident) bwd_body<true, true>(a, I, b, P, rank, C);
+    else if (!a.lean) bwd_body<false, false>(a, I, b, P, rank, C);
+    else bwd_body<false, true>(a, I, b, P, rank, C);
 }
 
 // ------------------------------------------------------------------ steps
@@ -1119,6 +1165,7 @@ size_t vec_bwd(const igaos_pdhg_unrolled_layout* L) {
 }
 
 constexpr int kMaxDevices = 16;
+constexpr int kClusterPerSm = 2;  // CTAs of a cluster launch per SM at most
 
 struct Device {
     int index, optin, sms;
@@ -1173,9 +1220,17 @@ int too_large(size_t need, int optin) {
 }
 
 enum Pass { kSteps, kForward, kBackward };
+constexpr int kVariants = 2;  // of a pass's kernel, by registers
+
+template <typename T>
+struct Kernels {
+    Pass pass;
+    void (*fn[kVariants])(UArgs<T>);  // the second one may be missing
+};
 
 struct Launch {
-    int C, threads;
+    int C, threads, variant;
+    int per_sm;  // CTAs that one SM holds
     size_t smem;
 };
 
@@ -1194,22 +1249,45 @@ cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* at, unsigned grid, int C,
     return cfg;
 }
 
-// Clusters of C CTAs that are resident at once at `per_sm` CTAs per SM (the
-// GPU's processing clusters hold no whole number of them): a property of the
-// device and the kernel, asked once for each.
+// CTAs of so many warps that a kernel's registers let one SM hold; asked once
+// for each kernel and number of warps.
 template <typename T>
-int resident_clusters(void (*kernel)(UArgs<T>), Pass pass, const Device& dev, int C, int per_sm,
-                      int threads, size_t smem) {
-    if (C == 1) return dev.sms * per_sm;
-    static std::atomic<int> known[kMaxDevices][3][kMaxCluster + 1][5];
+int by_registers(const Kernels<T>& k, int variant, const Device& dev, int warps) {
+    static std::atomic<int> known[kMaxDevices][3][kVariants][kLW + 1];
     std::atomic<int>* slot =
-        dev.index < kMaxDevices ? &known[dev.index][pass][C][std::min(per_sm, 4)] : nullptr;
+        dev.index < kMaxDevices ? &known[dev.index][k.pass][variant][warps] : nullptr;
+    if (slot && slot->load() > 0) return slot->load();
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void*)k.fn[variant], 32 * warps, 0) !=
+        cudaSuccess)
+        cudaGetLastError();
+    n = std::max(1, n);
+    if (slot) slot->store(n);
+    return n;
+}
+
+// Dynamic shared memory that leaves room for per_sm CTAs on an SM.
+size_t smem_at(const Device& dev, int per_sm) {
+    const size_t room = (size_t)dev.optin - kStaticSmem, sm = (size_t)dev.optin + 1024;
+    return std::min(room, sm / per_sm - 1024 - kStaticSmem) & ~(size_t)15;
+}
+
+// Clusters of C CTAs that are resident at once at `per_sm` CTAs per SM (the
+// GPU's processing clusters hold no whole number of them); asked once for each
+// kernel, C, per_sm and number of warps, at the shared memory of smem_at.
+template <typename T>
+int resident_clusters(const Kernels<T>& k, int variant, const Device& dev, int C, int per_sm,
+                      int warps) {
+    if (C == 1) return dev.sms * per_sm;
+    static std::atomic<int> known[kMaxDevices][3][kVariants][kMaxCluster + 1][kClusterPerSm + 1][kLW + 1];
+    std::atomic<int>* slot =
+        dev.index < kMaxDevices ? &known[dev.index][k.pass][variant][C][per_sm][warps] : nullptr;
     if (slot && slot->load() > 0) return slot->load();
     int n = 0;
     cudaLaunchAttribute at[1];
-    cudaLaunchConfig_t cfg = cluster_config(at, C, C, threads, smem, nullptr);
-    if (allow_smem(kernel, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, (const void*)kernel, &cfg) != cudaSuccess) {
+    cudaLaunchConfig_t cfg = cluster_config(at, C, C, 32 * warps, smem_at(dev, per_sm), nullptr);
+    if (allow_smem(k.fn[variant], dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, (const void*)k.fn[variant], &cfg) != cudaSuccess) {
         cudaGetLastError();
         n = 0;
     }
@@ -1226,9 +1304,17 @@ int resident_clusters(void (*kernel)(UArgs<T>), Pass pass, const Device& dev, in
 // them on one CTA each 23.6 ms, on two 34.6; FP64 96 of them 11.3 ms on two or
 // three, 10.4 on five; 96 of up to 1,300 rows (67,000 entries) 8 ms on seven,
 // 32 ms where the largest are read from global memory.
+// One-CTA instances stand on an SM as often as registers, threads and the
+// shared memory they need allow: with at most two, each asking for half of the
+// SM's memory, 200 iterations of 1,024 LPs of 60 x 120 took 1.1 ms forward and
+// 3.1 backward in FP32, now 0.50 and 1.5; 3.4 and 8.0 in FP64, now 1.7 and 5.7.
+// A backward that does not quite fit one CTA leaves costs and bounds in global
+// memory (lean): 1,024 FP64 LPs of 150 x 300 with 7,000 entries 58 ms on two
+// CTAs each, 30 on one.
 template <typename T>
-Launch plan(void (*kernel)(UArgs<T>), const igaos_pdhg_unrolled_layout* L, Pass pass,
-            const Device& dev, UArgs<T>& a) {
+Launch plan(const Kernels<T>& k, const igaos_pdhg_unrolled_layout* L, const Device& dev,
+            UArgs<T>& a) {
+    const Pass pass = k.pass;
     const size_t es = sizeof(T), room = (size_t)dev.optin - kStaticSmem;
     const int sc = (L->max_n + 31) / 32, sr = (L->max_m + 31) / 32;
     const double nnz = (double)L->max_nnz;
@@ -1238,43 +1324,68 @@ Launch plan(void (*kernel)(UArgs<T>), const igaos_pdhg_unrolled_layout* L, Pass 
                                   1.0 + (double)L->total_nnz / std::max(1.0, nnz));
     const double products = (pass == kBackward ? 6.0 : 2.0) * nnz * (wide ? 0.38e-3 : 0.1e-3);
     const double barriers = pass == kBackward ? 4.0 : 2.0;
-    Launch best{0, 0, 0};
+    Launch best{};
     double best_us = 0.0;
     for (int C = 1; C <= kMaxCluster; ++C) {
         if (best.C == 1 && nnz < 4096) break;  // latency-bound on one CTA
+        bool lean = false;
         const int lc = (sc + C - 1) / C, lr = (sr + C - 1) / C;
-        size_t vec = pass == kSteps     ? (size_t)32 * C * (lc + lr) * sizeof(double)
-                     : pass == kForward ? fwd_elems<T>(lc, lr, C) * es
-                                        : bwd_elems<T>(lc, lr, C) * es;
-        vec = (std::max(vec, scratch_bytes(L->max_m, L->max_n)) + 15) & ~(size_t)15;
-        const size_t fixed = vec + meta_bytes(L->max_m, L->max_n, lc, lr);
+        auto vectors = [&]() {
+            const size_t v = pass == kSteps     ? (size_t)32 * C * (lc + lr) * sizeof(double)
+                             : pass == kForward ? fwd_elems<T>(lc, lr, C) * es
+                                                : bwd_elems<T>(lc, lr, C, lean) * es;
+            return (std::max(v, scratch_bytes(L->max_m, L->max_n)) + 15) & ~(size_t)15;
+        };
+        size_t vec = vectors();
+        size_t fixed = vec + meta_bytes(L->max_m, L->max_n, lc, lr);
         if (fixed + 64 > room) continue;
         // entries of the largest share: slices are dealt evenly, by length
         const double pc = sc ? (double)lc / sc : 0.0, pr = sr ? (double)lr / sr : 0.0;
         double need = nnz * (pc * (es + 2) + pr * (es + 2 + (pass == kBackward ? es : 0)));
         if (C > 1) need = 1.02 * need + 1024;
+        if (pass == kBackward && C == 1 && fixed + (size_t)need + 64 > room) {
+            lean = true;
+            const size_t less = vectors();
+            lean = fixed - (vec - less) + (size_t)need + 64 <= room;
+            if (lean) {
+                fixed -= vec - less;
+                vec = less;
+            }
+        }
         const size_t want = fixed + (size_t)need + 64;
         const bool fits = want <= room;
         const int warps = std::min(kLW, std::max(4, std::max(lc, lr)));
         const size_t sm_bytes = (size_t)dev.optin + 1024;
         const int by_smem = fits ? (int)(sm_bytes / (want + kStaticSmem + 1024)) : 1;
-        const int per_sm = std::max(1, std::min({by_smem, 64 / warps, 2}));
-        // all that this residency leaves: shares of uneven rows fit better
-        const size_t smem = std::min(room, sm_bytes / per_sm - 1024 - kStaticSmem) & ~(size_t)15;
-        const int slots = resident_clusters(kernel, pass, dev, C, per_sm, 32 * warps, smem);
+        const int most = std::min(by_smem, C == 1 ? 64 / warps : kClusterPerSm);
+        int variant = 0, per_sm = std::max(1, std::min(most, by_registers(k, 0, dev, warps)));
+        if (k.fn[1] && count * C > (double)per_sm * dev.sms) {
+            const int more = std::min(most, by_registers(k, 1, dev, warps));
+            if (more > per_sm) {
+                variant = 1;
+                per_sm = more;
+            }
+        }
+        // a cluster asks for all that this residency leaves: shares of uneven
+        // rows fit better
+        const size_t smem = C == 1 && fits ? (want + 15) & ~(size_t)15 : smem_at(dev, per_sm);
+        const int slots = resident_clusters(k, variant, dev, C, per_sm, warps);
         if (slots < 1) continue;
         const double rounds = std::ceil(count / slots);
         const double used = std::max(1.0, std::min((double)per_sm, std::ceil(count * C / dev.sms)));
-        const double us = rounds * (used * products * 0.5 * (pc + pr) * (fits ? 1.0 : 8.0) +
+        // (too few warps on an SM leave the FP64 units' latency in the open)
+        const double open = wide ? std::max(1.0, 8.0 / (used * warps)) : 1.0;
+        const double us = rounds * (used * open * products * 0.5 * (pc + pr) * (fits ? 1.0 : 8.0) +
                                     barriers * (wide ? 2.0 : C == 1 ? 0.6 : 1.25));
         if (best.C == 0 || us < 0.95 * best_us) {
-            best = Launch{C, 32 * warps, smem};
+            best = Launch{C, 32 * warps, variant, per_sm, smem};
             best_us = us;
             a.lc = lc;
             a.lr = lr;
             a.ngc = 32 * lc * C;
             a.ngr = 32 * lr * C;
             a.per_cta = std::max(1, (int)((L->max_nnz + C - 1) / C));
+            a.lean = lean;
             a.vec_bytes = (int)vec;
             a.ent_bytes = (int)(smem - fixed);
         }
@@ -1284,11 +1395,19 @@ Launch plan(void (*kernel)(UArgs<T>), const igaos_pdhg_unrolled_layout* L, Pass 
     return best;
 }
 
+template <typename T>
+Kernels<T> kernels(Pass pass) {
+    return pass == kSteps     ? Kernels<T>{pass, {k_unroll_steps<T>, nullptr}}
+           : pass == kForward ? Kernels<T>{pass, {k_unroll_fwd<T>, nullptr}}
+                              : Kernels<T>{pass, {k_unroll_bwd<T, 1>, k_unroll_bwd<T, 2>}};
+}
+
 // One cluster of C CTAs per instance.
 template <typename T>
-cudaError_t launch(void (*kernel)(UArgs<T>), const Launch& l, int count, const UArgs<T>& a,
+cudaError_t launch(const Kernels<T>& k, const Launch& l, int count, const UArgs<T>& a,
                    const Device& dev, cudaStream_t st) {
     if (l.C == 0) return cudaErrorInvalidConfiguration;
+    void (*kernel)(UArgs<T>) = k.fn[l.variant];
     const cudaError_t e = allow_smem(kernel, dev);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute at[1];
@@ -1305,8 +1424,9 @@ int run_steps(const igaos_pdhg_unrolled_layout* L, const void* ax, double omega,
     a.tau_o = static_cast<T*>(tau);
     a.sigma_o = static_cast<T*>(sigma);
     a.omega = (T)omega;
-    const Launch l = plan<T>(k_unroll_steps<T>, L, kSteps, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_steps<T>, l, L->count, a, dev, st);
+    const Kernels<T> k = kernels<T>(kSteps);
+    const Launch l = plan<T>(k, L, dev, a);
+    const cudaError_t e = launch<T>(k, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
@@ -1328,8 +1448,9 @@ int run_forward(const igaos_pdhg_unrolled_layout* L, const void* c, const void* 
     a.y = static_cast<T*>(y);
     a.obj = static_cast<T*>(obj);
     a.ckpt = static_cast<T*>(ckpt);
-    const Launch l = plan<T>(k_unroll_fwd<T>, L, kForward, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_fwd<T>, l, L->count, a, dev, st);
+    const Kernels<T> k = kernels<T>(kForward);
+    const Launch l = plan<T>(k, L, dev, a);
+    const cudaError_t e = launch<T>(k, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
@@ -1364,8 +1485,9 @@ int run_backward(const igaos_pdhg_unrolled_layout* L, const void* c, const void*
     const long long vb = (per * (long long)sizeof(T) + 255) / 256 * 256;
     a.seg = static_cast<T*>(work);
     a.segf = static_cast<unsigned char*>(work) + vb;
-    const Launch l = plan<T>(k_unroll_bwd<T>, L, kBackward, dev, a);
-    const cudaError_t e = launch<T>(k_unroll_bwd<T>, l, L->count, a, dev, st);
+    const Kernels<T> k = kernels<T>(kBackward);
+    const Launch l = plan<T>(k, L, dev, a);
+    const cudaError_t e = launch<T>(k, l, L->count, a, dev, st);
     return e == cudaSuccess ? igx_set_error(IGAOS_PDHG_OK, "") : fail_cuda(e);
 }
 
@@ -1394,6 +1516,31 @@ extern "C" int64_t igaos_pdhg_unrolled_workspace_bytes(const igaos_pdhg_unrolled
     // values, then one clamp-outcome byte per value after a 256-byte boundary
     const int64_t vb = ((per * (int64_t)igx::elem_size(L)) + 255) / 256 * 256;
     return vb + per;
+}
+
+// The launch of a pass (0 steps, 1 forward, 2 backward) over a layout: CTAs per
+// instance, threads, CTAs per SM, dynamic shared memory, the kernel's variant,
+// whether the backward is lean. For tests; not in the public header.
+extern "C" int igx_unrolled_plan(const igaos_pdhg_unrolled_layout* L, int pass, int* out) {
+    using namespace igx;
+    Device dev{};
+    const int rc = prepare(L, &dev);
+    if (rc != IGAOS_PDHG_OK) return rc;
+    if (pass < kSteps || pass > kBackward || !out)
+        return igx_set_error(IGAOS_PDHG_ERR_INVALID, "no such pass");
+    auto fill = [&](auto a) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(a.ax)>>;
+        const Launch l = plan<T>(kernels<T>((Pass)pass), L, dev, a);
+        out[0] = l.C;
+        out[1] = l.threads;
+        out[2] = l.per_sm;
+        out[3] = (int)l.smem;
+        out[4] = l.variant;
+        out[5] = a.lean;
+    };
+    if (L->precision == IGAOS_PDHG_FP64) fill(base_args<double>(L));
+    else fill(base_args<float>(L));
+    return IGAOS_PDHG_OK;
 }
 
 extern "C" int igaos_pdhg_unrolled_steps(const igaos_pdhg_unrolled_layout* L, const void* ax,
