@@ -52,10 +52,13 @@ constexpr unsigned kFull = 0xffffffffu;
 struct BatchDesc {
     int m, n, nnz, mode;  // mode: where the instance is held (kHeld...)
     long long pad_c, pad_r;  // staged entries of the sorted slices, columns and rows
+    int long_c, long_r;      // slices laid in steps
+    int longer_c, longer_r;  // columns and rows of more than kLongRow entries
     long long ap_off, cp_off, nz_off, row_off, col_off;
     long long base_off;  // slice bases (in units of 32 entries): columns'
                          // (slices + 1), then rows'
     long long out_off;   // kHeldOut, kHeldWide: staged entries in global memory
+    long long long_c_at, long_r_at;  // the tables of the slices laid in steps
 };
 
 // kHeldWide: everything in global memory. kHeldOut: the matrix too (16-bit
@@ -65,6 +68,14 @@ struct BatchDesc {
 enum { kHeldWide = 0, kHeldOut = 1, kHeldMatrix = 2, kHeldAll = 3 };
 
 __host__ __device__ inline int slices_of(int rows) { return (rows + 31) / 32; }
+// A slice laid in steps: 32, 16, .. 1 lanes wide, step s as deep as the row of
+// lane step_lane(s) is long, so that half of its lanes or more hold entries all the
+// way. Such slices follow the others (which see them as empty), behind a table
+// {slice, first unit} of them; each has a unit for the depths of its steps, then its
+// entries, step after step.
+constexpr int kSteps = 6;
+constexpr int kLongRow = 64;  // entries of a row that one thread walks at most (each_row)
+__host__ __device__ inline int step_lane(int s) { return 16 >> s; }
 // staged values and 16-bit indices, x_bar, both slots of y, A~ x_bar, the
 // slices' bases and the rows' numbers
 __host__ __device__ inline size_t matrix_bytes(const BatchDesc& d) {
@@ -106,6 +117,7 @@ struct BatchArgs {
     double* cax64;       // original values in CSC order, FP64
     const int *order_c, *order_r;  // columns and rows by decreasing length
     const int* bases;              // first staged entry of each slice of 32 of them
+    const int* longs;              // tables of the slices laid in steps
     float* out_val;                // staged entries of kHeldOut and kHeldWide instances
     int* out_idx;
     float *dr, *dc, *sc, *scl, *scu, *srmin, *srmax, *yh32;
@@ -151,6 +163,7 @@ struct BatchShared {
     double dred[kBW * 8];
     int part[kBT];
     int inst;
+    int longs[2];  // slices laid in steps, columns and rows
     BatchStep step;
 };
 
@@ -274,7 +287,10 @@ __device__ Inst make_inst(const BatchArgs& a, const BatchDesc& d) {
 // slice's rows lie next to each other, padded with (0, entry 0) to its longest
 // row, so a warp reads runs of words and no lane tests a length (a pad adds
 // 0 x, nothing, to a sum; an infinite x ends the LP at its step's dot
-// products). Every row's sum keeps the order of its entries.
+// products). A slice that pads would more than double (a full row among short
+// ones: a budget, a normalisation) is laid in steps instead: as wide
+// as the rows that reach there, rounded up to a power of two. Every row's sum keeps
+// the order of its entries.
 template <int MODE>
 struct Held {
     using Idx = typename std::conditional<MODE == kHeldWide, int, uint16_t>::type;
@@ -391,17 +407,39 @@ __device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, 
         const int* idx = r ? I.ai : I.ci;
         const float* val = r ? I.sax : I.scax;
         const int b0 = bases[r ? sc + 1 + s : s], b1 = bases[r ? sc + 2 + s : s + 1];
-        float* v = const_cast<float*>(r ? W.rv : W.cv) + 32LL * b0 + lane;
-        Idx* ix = const_cast<Idx*>(r ? W.ri : W.ci) + 32LL * b0 + lane;
+        float* v0 = const_cast<float*>(r ? W.rv : W.cv);
+        Idx* ix0 = const_cast<Idx*>(r ? W.ri : W.ci);
+        float* v = v0 + 32LL * b0 + lane;
+        Idx* ix = ix0 + 32LL * b0 + lane;
         int p = 0, e = 0;
         if (q < (r ? I.m : I.n)) {
             const int row = order[r ? 1 : 0][q];
             p = ptr[row];
             e = ptr[row + 1];
         }
-        for (int k = b0; k < b1; ++k, ++p, v += 32, ix += 32) {
+        auto put = [&]() {
             *v = p < e ? val[p] : 0.f;
             *ix = (Idx)(p < e ? idx[p] : 0);
+        };
+        if (b1 > b0 || __all_sync(kFull, p == e)) {
+            for (int k = b0; k < b1; ++k, ++p, v += 32, ix += 32) put();
+            continue;
+        }
+        // in steps: the entry of the slices' table (written here as well), depths, entries
+        const int* table = a.longs + (r ? d.long_r_at : d.long_c_at);
+        const int units = bases[r ? sc + 1 + sr : sc];
+        int at = 0;
+        while (table[2 * at] != s) ++at;
+        if (lane < 2) v0[32LL * units + 2 * at + lane] = __int_as_float(table[2 * at + lane]);
+        const long long first = 32LL * table[2 * at + 1];
+        const int len = e - p;
+        v = v0 + first + 32 + lane;
+        ix = ix0 + first + 32 + lane;
+        for (int st = 0, k = 0; st < kSteps; ++st) {
+            const int w = 32 >> st, to = __shfl_sync(kFull, len, step_lane(st));
+            if (lane == st) v0[first + st] = __int_as_float(to - k);
+            for (; k < to; ++k, ++p, v += w, ix += w)
+                if (lane < w) put();
         }
     }
     __syncthreads();
@@ -436,6 +474,121 @@ __device__ __forceinline__ Acc<float> padded_dot(const Idx* idx, const float* va
     return acc;
 }
 
+// Adds `steps` products (with their errors) to each lane's sum, in order: lane's
+// from the lanes mine, mine + wide, ...
+__device__ __forceinline__ void lane_sums(Acc<float>& acc, float p, float pe, int wide, int mine,
+                                          int steps) {
+    int u = 0;
+#pragma unroll 1
+    for (; u + 8 <= steps; u += 8) {
+        float ps[8], es[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            ps[k] = __shfl_sync(kFull, p, (u + k) * wide + mine);
+            es[k] = __shfl_sync(kFull, pe, (u + k) * wide + mine);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc.add_product(ps[k], es[k]);
+    }
+#pragma unroll 1
+    for (; u < steps; ++u)
+        acc.add_product(__shfl_sync(kFull, p, u * wide + mine), __shfl_sync(kFull, pe, u * wide + mine));
+}
+
+// The same of a slice laid in steps, from its first entry (depths). The lanes
+// take 32 entries at once, loads and products, and the sums then run over them in
+// order, the row's lane getting each product from the lane that formed it.
+template <class Idx>
+__device__ __forceinline__ Acc<float> stepped_dot(const Idx* idx, const float* val,
+                                                  const float* __restrict__ v, long long first) {
+    const int lane = threadIdx.x & 31;
+    long long at = first + 32;
+    Acc<float> acc;
+#pragma unroll 1
+    for (int st = 0; st < kSteps; ++st) {
+        const int wide = 32 >> st, mine = lane & (wide - 1), per = 1 << st;
+        const int depth = __float_as_int(val[first + st]);
+        const long long end = at + (long long)wide * depth;
+        float w = 0.f, x = 0.f;
+        auto load = [&](long long k) {
+            w = x = 0.f;
+            if (k + lane < end) {
+                w = val[k + lane];
+                x = v[idx[k + lane]];
+            }
+        };
+        load(at);
+        const Acc<float> before = acc;
+#pragma unroll 1
+        for (int left = depth; left > 0; left -= per) {
+            const float p = w * x, pe = fmaf(w, x, -p);
+            at += 32;
+            load(at);
+            lane_sums(acc, p, pe, wide, mine, min(left, per));
+        }
+        if (lane >= wide) acc = before;  // (the other lanes' rows have ended)
+        at = end;
+    }
+    return acc;
+}
+
+// Either of them, by slice.
+template <bool OUT, class Idx>
+__device__ __forceinline__ Acc<float> any_dot(const int* base, const Idx* idx, const float* val,
+                                              const float* v, int s, int rows, int longs) {
+    const float* table = val + 32LL * base[slices_of(rows)];
+    for (int i = 0; i < longs; ++i)
+        if (__float_as_int(table[2 * i]) == s)
+            return stepped_dot(idx, val, v, 32LL * __float_as_int(table[2 * i + 1]));
+    return padded_dot<OUT>(idx, val, v, base[s], base[s + 1]);
+}
+
+// Rows of the CSR (columns of the CSC): f by one of the `workers` threads each,
+// those of more than kLongRow entries g by a warp each (they come first in the
+// order by length).
+template <class F, class G>
+__device__ __forceinline__ void each_row(const int* ptr, const int* order, int longer, int rows, int t,
+                                         int workers, F f, G g) {
+    if (longer == 0) {
+        for (int r = t; r < rows; r += workers) f(r);
+        return;
+    }
+    for (int r = t; r < rows; r += workers)
+        if (ptr[r + 1] - ptr[r] <= kLongRow) f(r);
+    if (t >= workers) return;
+    __syncwarp();
+    for (int q = t >> 5; q < longer; q += workers >> 5) g(order[q]);
+}
+// f(p) for every entry p of a row, by a warp
+template <class F>
+__device__ __forceinline__ void warp_entries(const int* ptr, int r, F f) {
+    for (int p = ptr[r] + (threadIdx.x & 31); p < ptr[r + 1]; p += 32) f(p);
+}
+// the sum of a(p) * x(p) over a row by a warp, as one thread takes it: the
+// factors by 32 lanes at once, the chain over them in order in every lane
+template <class A, class X>
+__device__ __forceinline__ double warp_chain(const int* ptr, int r, A a, X x) {
+    double s = 0.0;
+    for (int b = ptr[r], e = ptr[r + 1]; b < e; b += 32) {
+        const int p = min(b + (int)(threadIdx.x & 31), e - 1);
+        const double av = a(p), xv = x(p);
+        for (int u = 0; u < min(32, e - b); ++u)
+            s = fma(__shfl_sync(kFull, av, u), __shfl_sync(kFull, xv, u), s);
+    }
+    return s;
+}
+// row_dot by a warp, in every lane
+__device__ __forceinline__ Acc<float> warp_row_dot(const int* ptr, const int* idx, const float* val,
+                                                   const float* v, int r) {
+    Acc<float> acc;
+    for (int b = ptr[r], e = ptr[r + 1]; b < e; b += 32) {
+        const int p = b + (threadIdx.x & 31);
+        const float w = p < e ? val[p] : 0.f, x = p < e ? v[idx[p]] : 0.f, pr = w * x;
+        lane_sums(acc, pr, fmaf(w, x, -pr), 1, 0, min(32, e - b));
+    }
+    return acc;
+}
+
 // one row of a CSR times v (thread per row, compensated FP32)
 __device__ __forceinline__ Acc<float> row_dot(const int* ptr, const int* idx, const float* val,
                                               const float* v, int r) {
@@ -461,30 +614,54 @@ __device__ __noinline__ void anchor_data(const BatchArgs& a, const BatchDesc* d,
                                          int workers) {
     const Inst I = make_inst(a, *d);
     const Held<MODE> W = make_work<MODE>(a, *d);
-    for (int i = t; i < I.m; i += workers) {
+    auto row = [&](int i, double s) {
         const double dri = I.dr[i];
-        double s = 0.0;
-        for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) {
-            const int j = I.ai[p];
-            s = fma(I.axd[p] * (double)I.dc[j] / dri, I.xh[j], s);
-        }
         I.axh[i] = s;
         W.srmin()[i] = (float)(I.rmin[i] / dri - s);
         W.srmax()[i] = (float)(I.rmax[i] / dri - s);
         W.yh32()[i] = (float)I.yh[i];
-    }
-    for (int j = t; j < I.n; j += workers) {
+    };
+    each_row(I.ap, a.order_r + d->row_off, d->longer_r, I.m, t, workers,
+             [&](int i) {
+                 const double dri = I.dr[i];
+                 double s = 0.0;
+                 for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) {
+                     const int j = I.ai[p];
+                     s = fma(I.axd[p] * (double)I.dc[j] / dri, I.xh[j], s);
+                 }
+                 row(i, s);
+             },
+             [&](int i) {
+                 const double dri = I.dr[i];
+                 const double s = warp_chain(
+                     I.ap, i, [&](int p) { return I.axd[p] * (double)I.dc[I.ai[p]] / dri; },
+                     [&](int p) { return I.xh[I.ai[p]]; });
+                 if ((threadIdx.x & 31) == 0) row(i, s);
+             });
+    auto column = [&](int j, double s) {
         const double dcj = I.dc[j];
-        double s = 0.0;
-        for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) {
-            const int i = I.ci[p];
-            s = fma(I.cax64[p] * dcj / (double)I.dr[i], I.yh[i], s);
-        }
         I.atyh[j] = s;
         W.sc()[j] = (float)(I.c[j] * dcj + s);
         W.scl()[j] = (float)(I.cl[j] / dcj - I.xh[j]);
         W.scu()[j] = (float)(I.cu[j] / dcj - I.xh[j]);
-    }
+    };
+    each_row(I.cp, a.order_c + d->col_off, d->longer_c, I.n, t, workers,
+             [&](int j) {
+                 const double dcj = I.dc[j];
+                 double s = 0.0;
+                 for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) {
+                     const int i = I.ci[p];
+                     s = fma(I.cax64[p] * dcj / (double)I.dr[i], I.yh[i], s);
+                 }
+                 column(j, s);
+             },
+             [&](int j) {
+                 const double dcj = I.dc[j];
+                 const double s = warp_chain(
+                     I.cp, j, [&](int p) { return I.cax64[p] * dcj / (double)I.dr[I.ci[p]]; },
+                     [&](int p) { return I.yh[I.ci[p]]; });
+                 if ((threadIdx.x & 31) == 0) column(j, s);
+             });
     __syncthreads();
 }
 
@@ -494,21 +671,48 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
                                    float& eta0, float& omega0) {
     const Inst I = make_inst(a, *d);
     const int m = I.m, n = I.n;
+    const int *by_row = a.order_r + d->row_off, *by_col = a.order_c + d->col_off;
+    const bool first_lane = (threadIdx.x & 31) == 0;
     // CSC by counting sort; each column's entries ordered by row afterwards
     for (int j = t; j < n; j += workers) I.cnt[j] = 0;
     __syncthreads();
-    for (int i = t; i < m; i += workers)
-        for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) atomicAdd(&I.cnt[I.ai[p]], 1);
+    auto count = [&](int p) { atomicAdd(&I.cnt[I.ai[p]], 1); };
+    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+             [&](int i) {
+                 for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) count(p);
+             },
+             [&](int i) { warp_entries(I.ap, i, count); });
     __syncthreads();
     bscan(I.cnt, I.cp, n, workers);
     for (int j = t; j < n; j += workers) I.cnt[j] = I.cp[j];
     __syncthreads();
-    for (int i = t; i < m; i += workers)
-        for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) {
-            const int q = atomicAdd(&I.cnt[I.ai[p]], 1);
-            I.ci[q] = i;
-            I.cax64[q] = I.axd[p];
-        }
+    auto place = [&](int i, int p) {
+        const int q = atomicAdd(&I.cnt[I.ai[p]], 1);
+        I.ci[q] = i;
+        I.cax64[q] = I.axd[p];
+    };
+    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+             [&](int i) {
+                 for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) place(i, p);
+             },
+             [&](int i) {
+                 // lanes that meet in a column (entries that the row has twice) in order
+                 const int lane = threadIdx.x & 31;
+                 for (int p = I.ap[i] + lane, e = I.ap[i + 1]; p - lane < e; p += 32) {
+                     const unsigned on = __ballot_sync(kFull, p < e);
+                     if (p < e) {
+                         const unsigned peers = __match_any_sync(on, I.ai[p]);
+                         const int first = __ffs(peers) - 1;
+                         int q = 0;
+                         if (lane == first) q = atomicAdd(&I.cnt[I.ai[p]], __popc(peers));
+                         __syncwarp(on);
+                         q = __shfl_sync(on, q, first) + __popc(peers & ((1u << lane) - 1));
+                         I.ci[q] = i;
+                         I.cax64[q] = I.axd[p];
+                     }
+                     __syncwarp();
+                 }
+             });
     __syncthreads();
     for (int j = t; j < n; j += workers) {  // insertion sort by row index
         const int b = I.cp[j], e = I.cp[j + 1];
@@ -531,33 +735,67 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
     for (int j = t; j < n; j += workers) I.dc[j] = 1.f;
     __syncthreads();
     for (int sweep = 0; sweep < 10; ++sweep) {
-        for (int i = t; i < m; i += workers) {
-            float mx = 0.f;
-            for (int p = I.ap[i]; p < I.ap[i + 1]; ++p)
-                mx = fmaxf(mx, fabsf(I.ax[p]) * I.dc[I.ai[p]] / I.dr[i]);
+        auto top = [&](float mx) {  // of a warp
+            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+            return mx;
+        };
+        auto row_max = [&](int i, int p) { return fabsf(I.ax[p]) * I.dc[I.ai[p]] / I.dr[i]; };
+        auto scale_row = [&](int i, float mx) {
             if (mx > 0.f && isfinite(mx)) I.dr[i] *= sqrtf(mx);
-        }
+        };
+        each_row(I.ap, by_row, d->longer_r, m, t, workers,
+                 [&](int i) {
+                     float mx = 0.f;
+                     for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) mx = fmaxf(mx, row_max(i, p));
+                     scale_row(i, mx);
+                 },
+                 [&](int i) {
+                     float mx = 0.f;
+                     warp_entries(I.ap, i, [&](int p) { mx = fmaxf(mx, row_max(i, p)); });
+                     mx = top(mx);
+                     if (first_lane) scale_row(i, mx);
+                 });
         __syncthreads();
-        for (int j = t; j < n; j += workers) {
-            float mx = 0.f;
-            for (int p = I.cp[j]; p < I.cp[j + 1]; ++p)
-                mx = fmaxf(mx, fabsf(I.cax[p]) / I.dr[I.ci[p]] * I.dc[j]);
+        auto col_max = [&](int j, int p) { return fabsf(I.cax[p]) / I.dr[I.ci[p]] * I.dc[j]; };
+        auto scale_col = [&](int j, float mx) {
             if (mx > 0.f && isfinite(mx)) I.dc[j] /= sqrtf(mx);
-        }
+        };
+        each_row(I.cp, by_col, d->longer_c, n, t, workers,
+                 [&](int j) {
+                     float mx = 0.f;
+                     for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) mx = fmaxf(mx, col_max(j, p));
+                     scale_col(j, mx);
+                 },
+                 [&](int j) {
+                     float mx = 0.f;
+                     warp_entries(I.cp, j, [&](int p) { mx = fmaxf(mx, col_max(j, p)); });
+                     mx = top(mx);
+                     if (first_lane) scale_col(j, mx);
+                 });
         __syncthreads();
     }
     for (int i = t; i < m; i += workers) I.rdr[i] = 1.0 / (double)I.dr[i];
     for (int j = t; j < n; j += workers) I.rdc[j] = 1.0 / (double)I.dc[j];
     // scaled FP32 matrix; initial weight from the scaled cost and row bounds
     Acc<float> nq[2];
+    auto scaled = [&](int i, int p) { I.sax[p] = I.ax[p] * I.dc[I.ai[p]] / I.dr[i]; };
+    auto scaled_c = [&](int j, int p) { I.scax[p] = I.cax[p] * I.dc[j] / I.dr[I.ci[p]]; };
+    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+             [&](int i) {
+                 for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) scaled(i, p);
+             },
+             [&](int i) { warp_entries(I.ap, i, [&](int p) { scaled(i, p); }); });
+    each_row(I.cp, by_col, d->longer_c, n, t, workers,
+             [&](int j) {
+                 for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) scaled_c(j, p);
+             },
+             [&](int j) { warp_entries(I.cp, j, [&](int p) { scaled_c(j, p); }); });
     for (int i = t; i < m; i += workers) {
-        for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) I.sax[p] = I.ax[p] * I.dc[I.ai[p]] / I.dr[i];
         const float lo = (float)I.rmin[i] / I.dr[i], hi = (float)I.rmax[i] / I.dr[i];
         const float q = isfinite(hi) ? hi : (isfinite(lo) ? lo : 0.f);
         nq[1].add(q, q);
     }
     for (int j = t; j < n; j += workers) {
-        for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) I.scax[p] = I.cax[p] * I.dc[j] / I.dr[I.ci[p]];
         const float cs = (float)I.c[j] * I.dc[j];
         nq[0].add(cs, cs);
     }
@@ -572,15 +810,24 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
     __syncthreads();
     __shared__ float s_norm;
     for (int it = 0; it < 31; ++it) {
-        for (int i = t; i < m; i += workers) I.mt[i] = row_dot(I.ap, I.ai, I.sax, I.vt, i).result();
+        each_row(I.ap, by_row, d->longer_r, m, t, workers,
+                 [&](int i) { I.mt[i] = row_dot(I.ap, I.ai, I.sax, I.vt, i).result(); },
+                 [&](int i) {
+                     const float s = warp_row_dot(I.ap, I.ai, I.sax, I.vt, i).result();
+                     if (first_lane) I.mt[i] = s;
+                 });
         __syncthreads();
         if (it == 30) break;
+        // (normalised below, past the barrier)
+        each_row(I.cp, by_col, d->longer_c, n, t, workers,
+                 [&](int j) { I.vt[j] = row_dot(I.cp, I.ci, I.scax, I.mt, j).result(); },
+                 [&](int j) {
+                     const float s = warp_row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
+                     if (first_lane) I.vt[j] = s;
+                 });
+        __syncthreads();
         Acc<float> nrm[1];
-        for (int j = t; j < n; j += workers) {
-            const float wv = row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
-            I.vt[j] = wv;  // normalised below, past the barrier
-            nrm[0].add(wv, wv);
-        }
+        for (int j = t; j < n; j += workers) nrm[0].add(I.vt[j], I.vt[j]);
         bmerge<1>(nrm, workers);
         if (t == 0) s_norm = sqrtf((float)nrm[0].result_d());
         __syncthreads();
@@ -643,7 +890,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
         const int q = 32 * s + lane;
         const int i = q < I.m ? (MODE <= kHeldOut ? W.rid32[q] : (int)W.rid[q]) : I.m;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = padded_dot<MODE <= kHeldOut>(W.ri, W.rv, xs[v], W.rbase[s], W.rbase[s + 1]);
+            const Acc<float> ad = any_dot<MODE <= kHeldOut>(W.rbase, W.ri, W.rv, xs[v], s, I.m, sh.longs[1]);
             if (i >= I.m) continue;
             const double Ax = (I.axh[i] + ad.result_d()) * (double)I.dr[i];
             const double lo = I.rmin[i], hi = I.rmax[i];
@@ -685,7 +932,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
         const int q = 32 * s + lane;
         const int j = q < I.n ? (MODE <= kHeldOut ? W.cid32[q] : (int)W.cid[q]) : I.n;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = padded_dot<MODE <= kHeldOut>(W.ci, W.cv, ys[v], W.cbase[s], W.cbase[s + 1]);
+            const Acc<float> ad = any_dot<MODE <= kHeldOut>(W.cbase, W.ci, W.cv, ys[v], s, I.n, sh.longs[0]);
             if (j >= I.n) continue;
             const double dcj = I.dc[j], cj = I.c[j];
             const double aty = I.atyh[j] + ad.result_d();
@@ -840,11 +1087,28 @@ __device__ __forceinline__ void lanes_merge(Acc<float> (&v)[NV]) {
 
 // Products of the staged rows: out[id] = row id times v, in the order of its
 // entries (compensated FP32), a warp per slice.
-template <bool OUT, class Idx>
+// Slices laid in steps by the warps that found them empty (kept out of the other
+// slices' loop).
+template <class Idx>
+__device__ __noinline__ void long_products(const int* base, const uint16_t* id16, const int* id32,
+                                           const Idx* idx, const float* val, const float* v, float* out,
+                                           int rows, int longs) {
+    const int lane = threadIdx.x & 31, warps = (blockDim.x >> 5) - 1, wp = threadIdx.x >> 5;
+    const float* table = val + 32LL * base[slices_of(rows)];
+    for (int i = 0; i < longs; ++i) {
+        const int s = __float_as_int(table[2 * i]);
+        if (s % warps != wp) continue;
+        const int q = 32 * s + lane;
+        const Acc<float> acc = stepped_dot(idx, val, v, 32LL * __float_as_int(table[2 * i + 1]));
+        if (q < rows) out[id16 ? (int)id16[q] : id32[q]] = acc.result();
+    }
+}
+
+template <bool OUT, bool LONG, class Idx>
 __device__ __forceinline__ void slice_products(const int* base, const uint16_t* id16,
                                                const int* id32, const Idx* idx, const float* val,
                                                const float* __restrict__ v, float* out,
-                                               int rows) {
+                                               int rows, int longs) {
     const int lane = threadIdx.x & 31, warps = (blockDim.x >> 5) - 1;
     for (int s = threadIdx.x >> 5; 32 * s < rows; s += warps) {
         const int q = 32 * s + lane;
@@ -852,9 +1116,11 @@ __device__ __forceinline__ void slice_products(const int* base, const uint16_t* 
         const Acc<float> acc = padded_dot<OUT>(idx, val, v, base[s], base[s + 1]);
         if (row >= 0) out[row] = acc.result();
     }
+    if constexpr (LONG) long_products(base, id16, id32, idx, val, v, out, rows, longs);
 }
 
-template <int MODE>
+// LONG: the instance has slices laid in steps.
+template <int MODE, bool LONG>
 __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc* d,
                                             const Held<MODE>& W, int workers, double cmax) {
     BatchShared& sh = b_shared();
@@ -889,7 +1155,8 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
             lanes_merge(dx2);
             if (lane == 0) sh.acc[wp * 3] = dx2[0];
         }
-        slice_products<MODE <= kHeldOut>(W.rbase, W.rid, W.rid32, W.ri, W.rv, W.xbar, W.ab, m);
+        slice_products<MODE <= kHeldOut, LONG>(W.rbase, W.rid, W.rid32, W.ri, W.rv, W.xbar, W.ab, m,
+                                               LONG ? sh.longs[1] : 0);
         cta_sync();
         {   // dual step; the projection acts on the full value, so the anchor
             // enters its argument
@@ -924,7 +1191,8 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
             }
         }
         cta_sync();
-        slice_products<MODE <= kHeldOut>(W.cbase, W.cid, W.cid32, W.ci, W.cv, W.y(q), W.g(q), n);
+        slice_products<MODE <= kHeldOut, LONG>(W.cbase, W.cid, W.cid32, W.ci, W.cv, W.y(q), W.g(q), n,
+                                               LONG ? sh.longs[0] : 0);
         cta_sync();
         if (sh.step.done) return;
         if (!sh.step.check) continue;
@@ -938,6 +1206,13 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
             anchor_data<MODE>(a, d, t, workers);  // ends with a barrier
         }
     }
+}
+
+// (apart, so that its calls cost the other instances' loop no registers)
+template <int MODE>
+__device__ __noinline__ void worker_loop_long(const BatchArgs& a, const BatchDesc* d, int workers,
+                                              double cmax) {
+    worker_loop<MODE, true>(a, d, make_work<MODE>(a, *d), workers, cmax);
 }
 
 // The decision warp's side of the same loop. Its first lane holds the state.
@@ -1137,6 +1412,7 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
         for (int j = t; j < n; j += workers) I.xh[j] = I.pesx[j] = 0.0;
         for (int i = t; i < m; i += workers) I.yh[i] = I.pesy[i] = 0.0;
     }
+    if (threadIdx.x < 2) sh.longs[threadIdx.x] = threadIdx.x ? d.long_r : d.long_c;
     setup(a, dp, t, workers, s_eta0, s_omega0);
     fill_work<MODE>(a, dp, workers);
     anchor_data<MODE>(a, dp, t, workers);
@@ -1172,7 +1448,8 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
             a.out[b] = o;
         }
     } else {
-        worker_loop<MODE>(a, dp, W, workers, s_cmax);
+        if (d.long_c + d.long_r == 0) worker_loop<MODE, false>(a, dp, W, workers, s_cmax);
+        else worker_loop_long<MODE>(a, dp, workers, s_cmax);
         const Inst I = make_inst(a, d);
         // answer: anchor + delta of the chosen candidate, original units
         const int pf = sh.step.parity;
@@ -1217,10 +1494,12 @@ size_t held_bytes(const BatchDesc& d, int mode) {
                                : matrix_bytes(d) + (mode == kHeldAll ? state_bytes(d) : 0));
 }
 
-// Rows by decreasing length into `order` (counting sort, stable), and the
-// first staged entry of each slice of 32 (then the total), in units of 32,
-// onto `bases`; returns the entries.
-long long sort_slices(const std::vector<int>& len, int* order, std::vector<int>& bases) {
+// Rows by decreasing length into `order` (counting sort, stable), the first
+// staged entry of each slice of 32 (then the total), in units of 32, onto `bases`,
+// the slices laid in steps (where pads would take twice as much, if `steps`) onto
+// `longs`; returns the entries.
+long long sort_slices(const std::vector<int>& len, int* order, std::vector<int>& bases,
+                      std::vector<int>& longs, bool steps) {
     const int rows = (int)len.size();
     int longest = 0;
     for (int l : len) longest = std::max(longest, l);
@@ -1229,12 +1508,110 @@ long long sort_slices(const std::vector<int>& len, int* order, std::vector<int>&
     for (int k = 0; k <= longest; ++k) start[k + 1] += start[k];
     for (int r = 0; r < rows; ++r) order[start[longest - len[r]]++] = r;
     int run = 0;
+    const size_t first = longs.size();
+    std::vector<int> units;  // of the slices laid in steps
     for (int q = 0; q < rows; q += 32) {
+        const int in = std::min(32, rows - q), padded = len[order[q]];
         bases.push_back(run);
-        run += len[order[q]];
+        if (steps) {
+            long long entries = 0;
+            for (int st = 0, k = 0; st < kSteps; ++st) {
+                const int lane = step_lane(st), to = lane < in ? len[order[q + lane]] : 0;
+                entries += (long long)(32 >> st) * (to - k);
+                k = to;
+            }
+            const long long u = 1 + (entries + 31) / 32;
+            if (2 * u <= padded) {
+                longs.push_back(q / 32);
+                longs.push_back(0);
+                units.push_back((int)u);
+                continue;
+            }
+        }
+        run += padded;
     }
     bases.push_back(run);
+    run += (int)((longs.size() - first + 31) / 32);  // the table
+    for (size_t i = 0; i < units.size(); ++i) {
+        longs[first + 2 * i + 1] = run;
+        run += units[i];
+    }
     return 32LL * run;
+}
+
+// How a batch is staged and dealt to the classes: each instance's sorted slices,
+// its mode and class.
+struct BatchPlan {
+    std::vector<int> order_c, order_r, bases, longs, cls;
+    long long out_entries = 0;  // staged in global memory
+    size_t smem[kClasses] = {};
+};
+BatchPlan plan_batch(const int* ap, const int* ai, std::vector<BatchDesc>& desc, long long rows,
+                     long long cols) {
+    BatchPlan P;
+    P.order_c.resize(cols);
+    P.order_r.resize(rows);
+    P.cls.resize(desc.size());
+    std::vector<int> len_c, len_r;
+    for (size_t b = 0; b < desc.size(); ++b) {
+        BatchDesc& d = desc[b];
+        len_c.assign(d.n, 0);
+        for (int p = 0; p < d.nnz; ++p) ++len_c[ai[d.nz_off + p]];
+        len_r.resize(d.m);
+        for (int i = 0; i < d.m; ++i) len_r[i] = ap[d.ap_off + i + 1] - ap[d.ap_off + i];
+        auto longer = [](const std::vector<int>& len) {
+            return (int)std::count_if(len.begin(), len.end(), [](int l) { return l > kLongRow; });
+        };
+        d.longer_c = longer(len_c);
+        d.longer_r = longer(len_r);
+        d.base_off = (long long)P.bases.size();
+        d.long_c_at = (long long)P.longs.size();
+        auto stage = [&](bool steps) {
+            P.bases.resize(d.base_off);
+            P.longs.resize(d.long_c_at);
+            d.pad_c = sort_slices(len_c, P.order_c.data() + d.col_off, P.bases, P.longs, steps);
+            d.long_r_at = (long long)P.longs.size();
+            d.pad_r = sort_slices(len_r, P.order_r.data() + d.row_off, P.bases, P.longs, steps);
+            d.long_c = (int)(d.long_r_at - d.long_c_at) / 2;
+            d.long_r = (int)((long long)P.longs.size() - d.long_r_at) / 2;
+        };
+        const int reach = std::max(d.m, d.n);
+        auto deal = [&]() {  // its mode, and the class returned
+            int k = 0;
+            d.mode = kHeldAll;
+            while (k < kTight && ((reach > kClass[k].threads && kClass[k].threads < kBT) ||
+                                  held_bytes(d, kHeldAll) > kClass[k].smem))
+                ++k;
+            while (held_bytes(d, d.mode) > kClass[k].smem) --d.mode;
+            if (d.mode > kHeldOut) return k;
+            k = kClasses - 1;
+            if (held_bytes(d, kHeldOut) > kClass[k].smem || reach > 0xffff) d.mode = kHeldWide;
+            return k;
+        };
+        // Steps only where pads cost a mode, an SM to itself or space and loads in
+        // global memory (a 500 x 1,250 LP of 7,500 nonzeros with one full row: 112
+        // KB, 335 with pads, which no CTA has; its iteration 60 us with pads, 34 in
+        // steps): a short step costs a warp more than its pads. 512 LPs of 20 to 120
+        // rows with one full row: 40 ms padded, at two CTAs per SM, 43 in steps, at
+        // four.
+        stage(true);
+        int k = deal();
+        if (d.long_c + d.long_r > 0) {
+            const int mode = d.mode;
+            stage(false);
+            const int padded = deal();
+            const bool alone = kClass[padded].ctas == 1 && kClass[k].ctas > 1;
+            if (d.mode < mode || d.mode <= kHeldOut || alone) stage(true);
+            k = deal();
+        }
+        if (d.mode <= kHeldOut) {
+            d.out_off = P.out_entries;
+            P.out_entries += d.pad_c + d.pad_r;
+        }
+        P.cls[b] = k;
+        P.smem[k] = std::max(P.smem[k], held_bytes(d, d.mode));
+    }
+    return P;
 }
 
 template <int K>
@@ -1269,6 +1646,36 @@ __global__ void k_to_float(long long n, const double* __restrict__ in, float* __
 
 }  // namespace
 }  // namespace igx
+
+// Class, mode (kHeldWide ..) and staged entries of each instance of a batch. For
+// tests; not in the public header.
+extern "C" void igx_batch_plan(int count, const int* m, const int* n, const int* ap, const int* ai,
+                               int* cls, int* mode, long long* entries) {
+    using namespace igx;
+    std::vector<BatchDesc> desc(count);
+    long long ap_off = 0, nz = 0, rows = 0, cols = 0;
+    for (int b = 0; b < count; ++b) {
+        BatchDesc& d = desc[b];
+        d = BatchDesc{};
+        d.m = m[b];
+        d.n = n[b];
+        d.nnz = ap[ap_off + m[b]];
+        d.ap_off = ap_off;
+        d.nz_off = nz;
+        d.row_off = rows;
+        d.col_off = cols;
+        ap_off += d.m + 1;
+        nz += d.nnz;
+        rows += d.m;
+        cols += d.n;
+    }
+    const BatchPlan plan = plan_batch(ap, ai, desc, rows, cols);
+    for (int b = 0; b < count; ++b) {
+        cls[b] = plan.cls[b];
+        mode[b] = desc[b].mode;
+        entries[b] = desc[b].pad_c + desc[b].pad_r;
+    }
+}
 
 // ---------------------------------------------------------------- C ABI
 extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, const int* ap,
@@ -1336,45 +1743,14 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             return (long long)desc[p1].nnz + desc[p1].m + desc[p1].n >
                    (long long)desc[p2].nnz + desc[p2].m + desc[p2].n;
         });
-        // sorted slices of every instance's columns and rows
-        std::vector<int> order_c(cols), order_r(rows), bases, len;
-        long long out_off = 0;
-        for (int b = 0; b < count; ++b) {
-            BatchDesc& d = desc[b];
-            d.base_off = (long long)bases.size();
-            len.assign(d.n, 0);
-            for (int p = 0; p < d.nnz; ++p) ++len[ai[d.nz_off + p]];
-            d.pad_c = sort_slices(len, order_c.data() + d.col_off, bases);
-            len.resize(d.m);
-            for (int i = 0; i < d.m; ++i) len[i] = ap[d.ap_off + i + 1] - ap[d.ap_off + i];
-            d.pad_r = sort_slices(len, order_r.data() + d.row_off, bases);
-        }
-        // classes, each in that order
-        std::vector<int> cls_of(count), cls_order;
+        // sorted slices and classes, each in that order
+        const BatchPlan plan = plan_batch(ap, ai, desc, rows, cols);
+        std::vector<int> cls_order;
         int cls_count[kClasses] = {}, cls_first[kClasses] = {};
-        size_t cls_smem[kClasses] = {};
-        for (int b = 0; b < count; ++b) {
-            BatchDesc& d = desc[b];
-            const int reach = std::max(d.m, d.n);
-            int k = 0;
-            d.mode = kHeldAll;
-            while (k < kTight && ((reach > kClass[k].threads && kClass[k].threads < kBT) ||
-                                  held_bytes(d, kHeldAll) > kClass[k].smem))
-                ++k;
-            while (held_bytes(d, d.mode) > kClass[k].smem) --d.mode;
-            if (d.mode <= kHeldOut) {
-                k = kClasses - 1;
-                if (held_bytes(d, kHeldOut) > kClass[k].smem || reach > 0xffff) d.mode = kHeldWide;
-                d.out_off = out_off;
-                out_off += d.pad_c + d.pad_r;
-            }
-            cls_of[b] = k;
-            cls_smem[k] = std::max(cls_smem[k], held_bytes(d, d.mode));
-        }
         for (int k = kClasses - 1; k >= 0; --k) {
             cls_first[k] = (int)cls_order.size();
             for (int b : order)
-                if (cls_of[b] == k) cls_order.push_back(b);
+                if (plan.cls[b] == k) cls_order.push_back(b);
             cls_count[k] = (int)cls_order.size() - cls_first[k];
         }
         // constants, the same for every call: 131,072 powers take 5 ms
@@ -1394,7 +1770,7 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             ~StreamGuard() { cudaStreamDestroy(s); }
         } sg{st};
         Arena ar;
-        ar.expect((size_t)nz * 44 + (size_t)out_off * 8 + ((size_t)cols + rows) * 168 +
+        ar.expect((size_t)nz * 44 + (size_t)plan.out_entries * 8 + ((size_t)cols + rows) * 168 +
                   (size_t)count * (sizeof(BatchDesc) + sizeof(BatchOut)) + sizeof(float) * fac.size() +
                   (1 << 18));
         auto up = [&](const auto* h, size_t len) {
@@ -1429,11 +1805,12 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         A.scax = ar.alloc<float>(nz);
         float** colv[] = {&A.dc, &A.sc, &A.scl, &A.scu, &A.x[0], &A.x[1], &A.xa[0], &A.xa[1],
                           &A.xbar, &A.vt, &A.g[0], &A.g[1]};
-        A.order_c = up(order_c.data(), order_c.size());
-        A.order_r = up(order_r.data(), order_r.size());
-        A.bases = up(bases.data(), bases.size());
-        A.out_val = ar.alloc<float>(out_off);
-        A.out_idx = ar.alloc<int>(out_off);
+        A.order_c = up(plan.order_c.data(), plan.order_c.size());
+        A.order_r = up(plan.order_r.data(), plan.order_r.size());
+        A.bases = up(plan.bases.data(), plan.bases.size());
+        A.longs = up(plan.longs.data(), plan.longs.size());
+        A.out_val = ar.alloc<float>(plan.out_entries);
+        A.out_idx = ar.alloc<int>(plan.out_entries);
         for (float** v : colv) *v = ar.alloc<float>(cols);
         float** rowv[] = {&A.dr, &A.srmin, &A.srmax, &A.yh32, &A.y[0], &A.y[1], &A.ya[0],
                           &A.ya[1], &A.axc[0], &A.axc[1], &A.mt, &A.ab};
@@ -1497,13 +1874,13 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             CU(cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kClass[k].smem));
             CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k], threads,
-                                                             cls_smem[k]));
+                                                             plan.smem[k]));
             BatchArgs Ak = A;
             Ak.count = cls_count[k];
             Ak.order = d_order + cls_first[k];
             Ak.queue = queue + k;
             const int grid = std::min(cls_count[k], sms * std::max(1, per_sm));
-            kernels[k]<<<grid, threads, cls_smem[k], sk>>>(Ak);
+            kernels[k]<<<grid, threads, plan.smem[k], sk>>>(Ak);
             CU(cudaGetLastError());
             if (!first) {
                 CU(cudaEventCreateWithFlags(&fk.e[k], cudaEventDisableTiming));

@@ -253,7 +253,10 @@ template <> struct Acc<float> {
     __device__ __forceinline__ Acc() : s(0.f), c(0.f) {}
     __device__ __forceinline__ void add(float a, float x) {
         float p = a * x;
-        float pe = fmaf(a, x, -p);  // exact product error
+        add_product(p, fmaf(a, x, -p));
+    }
+    // a product p with its exact error pe
+    __device__ __forceinline__ void add_product(float p, float pe) {
         float t = s + p;
         float bp = t - s;
         float e = (s - (t - bp)) + (p - bp);  // exact addition error
