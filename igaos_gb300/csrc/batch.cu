@@ -1770,9 +1770,12 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
             ~StreamGuard() { cudaStreamDestroy(s); }
         } sg{st};
         Arena ar;
-        ar.expect((size_t)nz * 44 + (size_t)plan.out_entries * 8 + ((size_t)cols + rows) * 168 +
-                  (size_t)count * (sizeof(BatchDesc) + sizeof(BatchOut)) + sizeof(float) * fac.size() +
-                  (1 << 18));
+        // 40 bytes per entry, 128 per column and 112 per row, the staged entries, the
+        // tables; 50 roundings
+        ar.expect((size_t)nz * 40 + (size_t)cols * 128 + (size_t)rows * 112 +
+                  (size_t)plan.out_entries * 8 + (plan.bases.size() + plan.longs.size()) * sizeof(int) +
+                  (size_t)count * (sizeof(BatchDesc) + sizeof(BatchOut) + 16) +
+                  sizeof(float) * fac.size() + 64 * 256);
         auto up = [&](const auto* h, size_t len) {
             using V = std::remove_const_t<std::remove_pointer_t<decltype(h)>>;
             V* dp = ar.alloc<V>(len);

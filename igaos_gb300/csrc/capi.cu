@@ -385,11 +385,13 @@ int igaos_pdhg_last_error(char* buf, size_t len) {
     return g_code;
 }
 
-int igaos_pdhg_create(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const int* ap,
+// igaos_pdhg_create; next_precision: of the solve that follows at once (-1: none
+// known), whose buffers are then allocated with the problem's.
+static int create_problem(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const int* ap,
                       const int* ai, const double* ax, const int* cp, const int* ci,
                       const double* acx, const double* c, const double* cl, const double* cu,
                       const double* rmin, const double* rmax, double obj_const,
-                      const igaos_pdhg_options* opt) {
+                      const igaos_pdhg_options* opt, int next_precision) {
     if (!out) return fail(IGAOS_PDHG_ERR_INVALID, "out handle pointer is NULL");
     *out = nullptr;
     return guarded([&] {
@@ -430,7 +432,7 @@ int igaos_pdhg_create(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const
                                          R.ai.data(), R.ax.data(), tcp.data(), tci.data(),
                                          tacx.data(), R.c.data(), R.cl.data(), R.cu.data(),
                                          R.rmin.data(), R.rmax.data(), R.obj_const, dev,
-                                         opt->scaling);
+                                         opt->scaling, next_precision);
         } else {
             if (!cp) {
                 transpose_host(m, n, ap, ai, ax, tcp, tci, tacx);
@@ -439,7 +441,8 @@ int igaos_pdhg_create(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const
                 acx = tacx.data();
             }
             p->eng = new igx::Engine(m, n, nnz, ap, ai, ax, cp, ci, acx, c, cl, cu, rmin, rmax,
-                                     obj_const, dev, opt ? opt->scaling : IGAOS_PDHG_SCALING_RUIZ);
+                                     obj_const, dev, opt ? opt->scaling : IGAOS_PDHG_SCALING_RUIZ,
+                                     next_precision);
         }
         if (opt && opt->crossover && m <= igx::kCrossoverMaxRows) {
             p->xo = true;
@@ -456,6 +459,15 @@ int igaos_pdhg_create(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const
         }
         *out = p.release();
     });
+}
+
+int igaos_pdhg_create(igaos_pdhg_problem** out, int m, int n, int64_t nnz, const int* ap,
+                      const int* ai, const double* ax, const int* cp, const int* ci,
+                      const double* acx, const double* c, const double* cl, const double* cu,
+                      const double* rmin, const double* rmax, double obj_const,
+                      const igaos_pdhg_options* opt) {
+    return create_problem(out, m, n, nnz, ap, ai, ax, cp, ci, acx, c, cl, cu, rmin, rmax,
+                          obj_const, opt, -1);
 }
 
 int igaos_pdhg_solve(igaos_pdhg_problem* p, const igaos_pdhg_options* opt,
@@ -511,8 +523,8 @@ int igaos_pdhg_solve_csr(int m, int n, int64_t nnz, const int* ap, const int* ai
                          double* y) {
     if (!res) return fail(IGAOS_PDHG_ERR_INVALID, "result pointer is NULL");
     igaos_pdhg_problem* p = nullptr;
-    int rc = igaos_pdhg_create(&p, m, n, nnz, ap, ai, ax, cp, ci, acx, c, cl, cu, rmin, rmax,
-                               obj_const, opt);
+    int rc = create_problem(&p, m, n, nnz, ap, ai, ax, cp, ci, acx, c, cl, cu, rmin, rmax,
+                            obj_const, opt, opt ? opt->precision : IGAOS_PDHG_FP64);
     if (rc != IGAOS_PDHG_OK) {
         std::memset(res, 0, sizeof(*res));
         res->status = IGAOS_STATUS_ERROR;

@@ -33,16 +33,16 @@ Arena::~Arena() {
     for (void* p : ptrs_) cudaFree(p);
 }
 
-// Buffers are cut from larger allocations: of about what the owner says it will
-// take first, then of an eighth of that. A cudaMalloc and its cudaFree take
-// 4 us together for a few KB, 70 for some MB, and an LP has a hundred buffers.
-// What does not fit in such a block (or would not leave memory for one)
-// gets its own.
+// Buffers are cut from blocks, one for each group that the owner announces by
+// its size. A cudaMalloc and its cudaFree take 4 us together for a few KB, 70 for
+// some MB, and an LP has a hundred buffers. What is not announced, does not fit,
+// or would not leave memory for a block gets its own allocation.
 void* Arena::raw(size_t bytes) {
     bytes = (bytes + 255) & ~size_t(255);
     total_ += bytes;
     if (bytes > left_) {
-        const size_t block = ptrs_.empty() ? expect_ : std::max<size_t>(1 << 20, expect_ / 8);
+        const size_t block = expect_;
+        expect_ = 0;
         void* p = nullptr;
         if (block > bytes && cudaMalloc(&p, block) == cudaSuccess) {
             ptrs_.push_back(p);
@@ -332,7 +332,7 @@ constexpr size_t kMetAt = (sizeof(DevCtl) + 63) & ~(size_t)63;
 Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, const double* ax,
                const int* cp, const int* ci, const double* acx, const double* c,
                const double* cl, const double* cu, const double* rmin, const double* rmax,
-               double obj_const_, int device, int scaling)
+               double obj_const_, int device, int scaling, int next_precision)
     : m(m_), n(n_), nnz(nnz_), obj_const(obj_const_), scaling_(scaling) {
     auto t_setup = std::chrono::steady_clock::now();
     auto t_mark = t_setup;
@@ -361,9 +361,19 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
     ipr_ = inverse(pr_);
     ipc_ = inverse(pc_);
     mark("stream, orderings");
-    // both orientations in FP64 and FP32 with their indices, FP32 padded rows,
-    // and about 45 doubles of vectors per row and column
-    ar_.expect((size_t)nnz * 41 + ((size_t)m + n) * 360 + (1 << 20));
+    // one block: both orientations in FP64 and FP32 with their indices, the FP32
+    // rows padded, schedules, 128 bytes of vectors per column and 92 per row; what the
+    // solve that follows brings in (20,000 x 50,000, 500,000 nonzeros: three more
+    // blocks took 0.5 of 23 ms)
+    {
+        long long pad4 = 0;
+        for (int r = 0; r < m; ++r) pad4 += (ap[r + 1] - ap[r] + 3) & ~3;
+        if (!IGX_PAD4 || pad4 - nnz > nnz / 8) pad4 = 0;
+        const bool f32 = next_precision >= 0 && next_precision != IGAOS_PDHG_FP64;
+        ar_.expect((size_t)nnz * 32 + (size_t)pad4 * 8 + (size_t)n * 138 + (size_t)m * 106 +
+                   (next_precision >= 0 ? work_bytes(f32 ? 4 : 8) + rep_bytes() : 0) +
+                   (f32 && next_precision != IGAOS_PDHG_FP32 ? anchor_bytes() : 0) + (1 << 20));
+    }
     {
         std::vector<int> P;
         std::unique_ptr<int[]> I;
@@ -638,6 +648,7 @@ template <typename T>
 void Engine::ensure_work() {
     bool& have = std::is_same<T, double>::value ? have64_ : have32_;
     if (have) return;
+    ar_.expect(work_bytes(sizeof(T)));
     Work<T>& w = work<T>();
     for (int s = 0; s < 2; ++s) {
         w.x[s] = ar_.alloc<T>(n);
@@ -1096,6 +1107,7 @@ bool Engine::try_repair(const Vecs& v, int p, bool anch, const DevMetrics& ma,
 
 void Engine::ensure_rep() {
     if (have_rep_) return;
+    ar_.expect(rep_bytes());
     rep_.d = ar_.alloc<double>(n);
     rep_.r = ar_.alloc<double>(n);
     rep_.q = ar_.alloc<double>(n);
@@ -1930,6 +1942,7 @@ namespace igx {
 // attainable accuracy is set by FP64, while every attempt streams FP32.
 void Engine::ensure_anchor() {
     if (have_anchor_) return;
+    ar_.expect(anchor_bytes());
     anc_.xh = ar_.alloc<double>(n);
     anc_.yh = ar_.alloc<double>(m);
     for (int s = 0; s < 2; ++s) {

@@ -36,8 +36,8 @@ class Arena {
     template <typename T>
     T* alloc(size_t n) { return static_cast<T*>(raw(sizeof(T) * (n ? n : 1))); }
     size_t bytes() const { return total_; }
-    // what will be allocated in all, about; before the first allocation
-    void expect(size_t bytes) { expect_ = bytes; }
+    // about what the next allocations will take together: one block for them
+    void expect(size_t bytes) { expect_ = bytes > left_ ? bytes : 0; }
 
    private:
     std::vector<void*> ptrs_;
@@ -162,10 +162,12 @@ struct LoopOut {
 
 class Engine {
    public:
+    // next_precision: of the solve that follows at once, if one does
     Engine(int m, int n, long long nnz, const int* ap, const int* ai, const double* ax,
            const int* cp, const int* ci, const double* acx, const double* c,
            const double* cl, const double* cu, const double* rmin, const double* rmax,
-           double obj_const, int device, int scaling = IGAOS_PDHG_SCALING_RUIZ);
+           double obj_const, int device, int scaling = IGAOS_PDHG_SCALING_RUIZ,
+           int next_precision = -1);
     ~Engine();
 
     void solve(const igaos_pdhg_options& o, igaos_pdhg_result& r, double* x, double* y);
@@ -195,6 +197,12 @@ class Engine {
    private:
     int device_ = 0;
     cudaStream_t st_ = nullptr;
+    // sizes of the buffers that come on first use
+    size_t work_bytes(int elem) const {
+        return elem * (7 * (size_t)n + 8 * (size_t)m) + 24 * (size_t)cap_ctas_ + 20 * 256;
+    }
+    size_t anchor_bytes() const { return ((size_t)n + m) * 60 + 24 * 256; }
+    size_t rep_bytes() const { return (size_t)n * 50 + (size_t)m * 49 + 20 * 256; }
     Arena ar_;
     // matrix (scaled in place at setup)
     int *ap_, *ai_, *cp_, *ci_;
