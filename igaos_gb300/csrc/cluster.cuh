@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
                 small_totals(dx_to, part_dy, part_cr, dots);
             }
             if (wi == kSmallWarps) {  // as decide_step
-                const StepOut o = step_rule(st, dots[0], dots[1], dots[2]);
+                const StepOut o = step_rule<sizeof(T) == 8>(st, dots[0], dots[1], dots[2]);
                 const double sigma = __dmul_rn(o.eta, st.omega);
                 CtlView<T> nv = cv;
                 if constexpr (std::is_same<T, double>::value) {

@@ -196,6 +196,10 @@ __device__ __forceinline__ bool dfinite(double a) {
     return (__double_as_longlong(a) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
 }
 __device__ __forceinline__ bool dgt0(double a) { return __double_as_longlong(a) > 0; }
+// a is not the NaN of an operation (a quiet one; dgt0 takes one for a number)
+__device__ __forceinline__ bool number(double a) {
+    return (__double2hiint(a) & 0x7fffffff) <= 0x7ff00000;
+}
 __device__ __forceinline__ bool dlt0(double a) {
     const long long b = __double_as_longlong(a);
     return b < 0 && (b << 1) != 0;  // negative, not -0

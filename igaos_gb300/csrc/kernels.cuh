@@ -303,6 +303,10 @@ struct StepOut {
     double eta, w;  // the next attempt's step size; the averaging weight after an acceptance
     bool accept, sound;
 };
+// OVER: an infinite product beside finite norms gives etabar 0, a rejected step;
+// compensated FP32 sums do not have it (they overflow to NaN), and the four
+// instructions cost 70 ns an attempt.
+template <bool OVER>
 __device__ __forceinline__ StepOut step_rule(const StepState& s, double dx2, double dy2, double cross) {
     const int lane = threadIdx.x & 31;
     const unsigned full = 0xffffffffu;
@@ -311,7 +315,7 @@ __device__ __forceinline__ StepOut step_rule(const StepState& s, double dx2, dou
     };
     const double num = __dadd_rn(__dmul_rn(s.omega, dx2), div_exact(dy2, s.omega, s.iomega));
     const bool sound = dfinite(dx2) && dfinite(dy2) && dfinite(cross);
-    const bool curved = sound && dfinite(num) && dgt0(num) && dgt0(cross);
+    const bool curved = (OVER ? number(cross) : sound) && dfinite(num) && dgt0(num) && dgt0(cross);
     // lane 0: etabar; lane 1: the weight 2 / (hn + 2) after an acceptance
     const double den = lane == 1 ? (double)(s.hn + 1) + 2.0 : (curved ? __dmul_rn(2.0, cross) : 1.0);
     const double quo = __ddiv_rn(lane == 1 ? 2.0 : num, den);
@@ -332,10 +336,11 @@ __device__ __forceinline__ StepOut step_rule(const StepState& s, double dx2, dou
     }
     return StepOut{eta, w_next, accept, sound};
 }
+template <bool OVER>
 __device__ __forceinline__ void decide_step(DevCtl* c, const StepState& s, double dx2, double dy2,
                                             double cross) {
     const int lane = threadIdx.x & 31;
-    const StepOut o = step_rule(s, dx2, dy2, cross);
+    const StepOut o = step_rule<OVER>(s, dx2, dy2, cross);
     const double eta = o.eta;
     const double sigma = __dmul_rn(eta, s.omega);
     // lane 0: tau; lane 1: 1 / sigma
@@ -394,7 +399,7 @@ __device__ __forceinline__ void finish_attempt(const DualArgs<T>& a, int gd, dou
         double d[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) d[q] = __shfl_sync(0xffffffffu, s[q].result_d(), 0);
-        decide_step(a.ctl, st, d[0], d[1], d[2]);
+        decide_step<sizeof(T) == 8>(a.ctl, st, d[0], d[1], d[2]);
     }
 }
 
