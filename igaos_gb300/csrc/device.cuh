@@ -9,8 +9,8 @@
 //
 // The hot SpMV is warp-scheduled over a length-sorted permutation of the LP
 // (see WarpSched below): rows of similar length share a warp, G lanes per
-// row, coalesced streaming of values and indices, x gathered through the
-// read-only path, warp-shuffle reductions. The PDHG step for each row runs
+// row, coalesced streaming of values and indices, x gathered through L1 and
+// L2, warp-shuffle reductions. The PDHG step for each row runs
 // right after its sum, with consecutive lanes on consecutive rows, so
 // A^T y / A xbar never round-trip through HBM.
 #pragma once
@@ -482,10 +482,12 @@ struct PlainEpi {
 // batches of kLaneBatch per lane (all value and index loads of a batch, then
 // its gathers in flight); then the G-lane shuffle reduction, and the sum of
 // the item's i-th row handed to lane i, so consecutive lanes touch
-// consecutive vector entries.
+// consecutive vector entries. x is read by plain loads: under programmatic
+// launches the kernel is alive while its predecessor writes x, and a read-only
+// load (__ldg, or const __restrict__ on a kernel's parameter) promises that
+// nobody does.
 template <typename T>
-__device__ __forceinline__ Acc<T> lane_products(const Csr<T>& A, const T* __restrict__ x, int b,
-                                                int e, int lg) {
+__device__ __forceinline__ Acc<T> lane_products(const Csr<T>& A, const T* x, int b, int e, int lg) {
     const int G = 1 << lg;
     const int gl = (threadIdx.x & 31) & (G - 1);
     Acc<T> acc;
@@ -504,8 +506,7 @@ __device__ __forceinline__ Acc<T> lane_products(const Csr<T>& A, const T* __rest
                     a4 = __ldg(reinterpret_cast<const float4*>(A.val + p));
                     j4 = __ldg(reinterpret_cast<const int4*>(A.idx + p));
                 }
-                const float x0 = __ldg(x + j4.x), x1 = __ldg(x + j4.y), x2 = __ldg(x + j4.z),
-                            x3 = __ldg(x + j4.w);
+                const float x0 = x[j4.x], x1 = x[j4.y], x2 = x[j4.z], x3 = x[j4.w];
                 acc.add(a4.x, x0);
                 acc.add(a4.y, x1);
                 acc.add(a4.z, x2);
@@ -542,7 +543,7 @@ __device__ __forceinline__ Acc<T> lane_products(const Csr<T>& A, const T* __rest
         }
         T xv[kLaneBatch];
 #pragma unroll
-        for (int u = 0; u < kLaneBatch; ++u) xv[u] = __ldg(x + j[u]);
+        for (int u = 0; u < kLaneBatch; ++u) xv[u] = x[j[u]];
 #pragma unroll
         for (int u = 0; u < kLaneBatch; ++u) acc.add(a[u], xv[u]);  // masked: 0 * x[0] adds 0
     }
@@ -558,8 +559,7 @@ __device__ __forceinline__ Acc<T> reduce_rows(Acc<T> acc, int lg) {
 
 // The row sums of the item holding rows [r0, r1).
 template <typename T>
-__device__ __forceinline__ Acc<T> item_sums(const Csr<T>& A, const T* __restrict__ x, int r0,
-                                            int r1, int lg) {
+__device__ __forceinline__ Acc<T> item_sums(const Csr<T>& A, const T* x, int r0, int r1, int lg) {
     const int r = r0 + ((threadIdx.x & 31) >> lg);
     int b = 0, e = 0;
     if (r < r1) {
@@ -574,7 +574,7 @@ __device__ __forceinline__ Acc<T> item_sums(const Csr<T>& A, const T* __restrict
 // the row step (epi.apply) on the 32/G lanes that hold a row.
 template <typename T, class E>
 __device__ __forceinline__ void warp_item(const WarpSched& ws, const Csr<T>& A,
-                                          const T* __restrict__ x, int w, E& epi) {
+                                          const T* x, int w, E& epi) {
     const int lane = threadIdx.x & 31;
     const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
     const int lg = __ldg(ws.lg + w);
@@ -620,8 +620,7 @@ __device__ __forceinline__ FirstItem first_item(const WarpSched& ws, const Csr<T
 // The items of this warp, from its first.
 template <typename T, class E>
 __device__ __forceinline__ void warp_rows_from(const WarpSched& ws, const Csr<T>& A,
-                                               const T* __restrict__ x, E& epi,
-                                               const FirstItem& f) {
+                                               const T* x, E& epi, const FirstItem& f) {
     // software-pipelined: the next item's schedule entries are loaded when
     // this item starts, and its row pointers between this item's products
     // and its reduction, so each item starts with [b, e) in registers
@@ -666,7 +665,7 @@ __device__ __forceinline__ void warp_rows_from(const WarpSched& ws, const Csr<T>
 
 template <typename T, class E>
 __device__ __forceinline__ void warp_rows_all(const WarpSched& ws, const Csr<T>& A,
-                                              const T* __restrict__ x, E& epi) {
+                                              const T* x, E& epi) {
 #if IGX_ITEM_PREFETCH
     warp_rows_from<T>(ws, A, x, epi, first_item<T>(ws, A));
 #else

@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, OCC) k_dual(DualArgs<T> a) {
 // y = A x (Spmv::mv, src/pdhg/pdhg.cu:143-157).
 template <typename T, typename TO>
 __global__ void __launch_bounds__(kThreads, HotCtas<T>::value)
-    k_spmv(WarpSched ws, Csr<T> A, const T* __restrict__ x, TO* __restrict__ y) {
+    k_spmv(WarpSched ws, Csr<T> A, const T* x, TO* y) {
     follow_previous();
     auto f = [&](int r, const Acc<T>& acc) { y[r] = (TO)acc.result_d(); };
     PlainEpi<decltype(f)> epi{f};
@@ -466,9 +466,8 @@ __device__ __forceinline__ double ruiz_max(double mx, double v) {  // both >= 0;
 __global__ void __launch_bounds__(kThreads) k_ruiz_rows(WarpSched ws, const int* __restrict__ ap,
                                                           const int* __restrict__ ai,
                                                           const double* __restrict__ ax,
-                                                          const double* __restrict__ dc,
-                                                          double* __restrict__ dr,
-                                                          double* __restrict__ idr) {
+                                                          const double* dc, double* dr,
+                                                          double* idr) {
     follow_previous();
     const int lane = threadIdx.x & 31;
     for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5); w < ws.nwarps; w += gridDim.x * kWarps) {
@@ -494,9 +493,8 @@ __global__ void __launch_bounds__(kThreads) k_ruiz_rows(WarpSched ws, const int*
 __global__ void __launch_bounds__(kThreads) k_ruiz_cols(WarpSched ws, const int* __restrict__ cp,
                                                           const int* __restrict__ ci,
                                                           const double* __restrict__ acx,
-                                                          const double* __restrict__ dr,
-                                                          const double* __restrict__ idr,
-                                                          double* __restrict__ dc) {
+                                                          const double* dr, const double* idr,
+                                                          double* dc) {
     follow_previous();
     const int lane = threadIdx.x & 31;
     for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5); w < ws.nwarps; w += gridDim.x * kWarps) {
@@ -669,7 +667,7 @@ __global__ void k_sumsq(NormArgs a, int root) {
 
 // Power-iteration normalisation (src/pdhg/pdhg.cu:617-622): v = w / ||w||
 // unless ||w|| < 1e-300, in which case the loop is over (flag latched).
-__global__ void k_power_normalise(int n, const double* __restrict__ w, double* __restrict__ v,
+__global__ void k_power_normalise(int n, const double* w, double* v,
                                   const double* nw, int* done) {
     follow_previous();
     let_next();
