@@ -872,6 +872,14 @@ __device__ __forceinline__ double warp_bmax(double v) {
     return __hiloint2double((int)mh, (int)ml);
 }
 
+// a / b for one divisor b, rb = 1 / b correctly rounded: one remainder step, the
+// correctly rounded quotient (Markstein 1990). The divisors are scale factors and
+// weights, near 1.
+__device__ __forceinline__ double div_by(double a, double b, double rb) {
+    const double q0 = a * rb;
+    return dfinite(q0) ? fma(fma(-b, q0, a), rb, q0) : q0;
+}
+
 // The metrics of the current (0) and averaged (1) iterates; valid in the
 // decision warp's first lane. Two barriers; the candidates share them and the
 // loads of the LP's data.
@@ -903,7 +911,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
                 if (dfinite(hi)) scv = bsel_max(scv, dabs(hi));
                 mx[v][2] = bmax(mx[v][2], vi / (1.0 + scv));
             }
-            mx[v][3] = bmax(mx[v][3], dabs((I.yh[i] + (double)ys[v][i]) * I.rdr[i]));
+            mx[v][3] = bmax(mx[v][3], dabs(div_by(I.yh[i] + (double)ys[v][i], I.dr[i], I.rdr[i])));
         }
     }
     if (works)
@@ -936,7 +944,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
             if (j >= I.n) continue;
             const double dcj = I.dc[j], cj = I.c[j];
             const double aty = I.atyh[j] + ad.result_d();
-            const double d = cj + aty * I.rdc[j];
+            const double d = cj + div_by(aty, dcj, I.rdc[j]);
             const double lo = I.cl[j], hi = I.cu[j];
             const float xv = xs[v][j];
             const double x = xv == W.scl()[j] ? lo : (xv == W.scu()[j] ? hi : (I.xh[j] + (double)xv) * dcj);
@@ -961,7 +969,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
     }
     for (int i = t; i < I.m; i += workers)
         for (int v = 0; v < 2; ++v) {
-            const double yv = (I.yh[i] + (double)ys[v][i]) * I.rdr[i];
+            const double yv = div_by(I.yh[i] + (double)ys[v][i], I.dr[i], I.rdr[i]);
             if (blt(yz[v], yv)) {
                 if (dfinite(I.rmax[i])) od[v] -= yv * I.rmax[i];
                 else unb[v] = true;
@@ -1037,13 +1045,6 @@ __device__ __noinline__ void re_anchor(const BatchArgs& a, const BatchDesc* d, i
         dn[v] = warp_sum(dn[v]);
         if (lane == 0 && wp < workers / 32) sh.dred[2 * wp + v] = dn[v];
     }
-}
-
-// a / b for one divisor b, rb = 1 / b: one remainder step (Markstein 1990;
-// the correctly rounded quotient but for rare cases one ulp off)
-__device__ __forceinline__ double div_by(double a, double b, double rb) {
-    const double q0 = a * rb;
-    return dfinite(q0) ? fma(fma(-b, q0, a), rb, q0) : a / b;
 }
 
 // ---- one LP --------------------------------------------------------------

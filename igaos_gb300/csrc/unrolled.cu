@@ -167,9 +167,11 @@ __device__ __forceinline__ T clampf(T v, T lo, T hi, int& f) {
     return v;
 }
 // t / s for one divisor s many times, is = u_recip(s). FP64: the product with
-// the correctly rounded reciprocal and one remainder step (Markstein 1990;
-// the correctly rounded quotient but for rare cases one ulp off), three
-// operations on the FP64 pipe instead of the division's. Operands far from 1
+// the correctly rounded reciprocal and one remainder step, the correctly rounded
+// quotient (Markstein 1990) in three operations on the FP64 pipe instead of the
+// division's. (Where t / s is so close to the middle of two doubles that the step's
+// own error could decide, the product is half an ulp off, and the error s / 2^54 of
+// what a quotient's distance from a middle is at least.) Operands far from 1
 // by hundreds of binades, where a step could leave the normal range, divide.
 __device__ __forceinline__ bool u_tame(double v) {
     const int ex = (__double2hiint(v) >> 20) & 0x7ff;
