@@ -795,9 +795,10 @@ void Engine::launch_attempts(int count, const Vecs& v, bool graphs) {
     CU(cudaGraphLaunch(it->second, st_));
 }
 
-// The autotuner's other schedules, on its first use.
+// The autotuner's other schedules, on its first use (all of them or, where an
+// allocation fails, none).
 void Engine::ensure_candidates() {
-    if (candA_[0].row && candA_[kTuneCount - 1].row) return;
+    if (have_cand_) return;
     std::vector<int> pa(m + 1), pat(n + 1);
     CU(cudaMemcpy(pa.data(), ap_, sizeof(int) * pa.size(), cudaMemcpyDeviceToHost));
     CU(cudaMemcpy(pat.data(), cp_, sizeof(int) * pat.size(), cudaMemcpyDeviceToHost));
@@ -806,6 +807,7 @@ void Engine::ensure_candidates() {
         candA_[c] = upload_sched(ar_, pa.data(), m, cap_ctas_, kTuneEntries[c]);
         candAT_[c] = upload_sched(ar_, pat.data(), n, cap_ctas_, kTuneEntries[c]);
     }
+    have_cand_ = true;
 }
 
 void Engine::use_sched(int ia, int iat) {

@@ -221,6 +221,7 @@ class Engine {
     int choice_[2][2] = {{-1, -1}, {-1, -1}};  // autotuned (A, A^T) per FP32 / FP64
     int choice_occ_[2] = {3, 3};            // autotuned FP64 occupancy (A, A^T)
     float tune_us_[2][2][kTuneCount][2] = {};  // per attempt-kernel launch, us (occupancy 3, 4)
+    bool have_cand_ = false;
     void ensure_candidates();
     void use_sched(int ia, int iat);
     template <typename T> void tune();
