@@ -25,8 +25,8 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 // Resident CTAs per SM the hot kernels are compiled for; launch widths use
 // the same figure. Measured on the 200k x 500k LP (FP32 attempt): 6 CTAs
-// (<= 40 registers, no spills) 59 us, 7 or 8 CTAs (forced to 32-36
-// registers, with spills) 70 us.
+// (<= 40 registers; 32 bytes spilled in k_dual's decision, by its last CTA) 59 us,
+// 7 or 8 CTAs (forced to 32-36 registers, with spills in the loops) 70 us.
 #ifndef IGX_HOT_CTAS
 #define IGX_HOT_CTAS 6
 #endif
@@ -557,45 +557,6 @@ __device__ __forceinline__ Acc<T> reduce_rows(Acc<T> acc, int lg) {
     return acc.shfl_from(0xffffffffu, ((threadIdx.x & 31) << lg) & 31);
 }
 
-// The row sums of the item holding rows [r0, r1).
-template <typename T>
-__device__ __forceinline__ Acc<T> item_sums(const Csr<T>& A, const T* x, int r0, int r1, int lg) {
-    const int r = r0 + ((threadIdx.x & 31) >> lg);
-    int b = 0, e = 0;
-    if (r < r1) {
-        b = __ldg(A.ptr + r);
-        e = __ldg(A.ptr + r + 1);
-    }
-    return reduce_rows<T>(lane_products<T>(A, x, b, e, lg), lg);
-}
-
-// One warp item with its row steps in place: the epilogue's vector entries
-// for the lane's row are loaded first (epi.load), then the row sums, then
-// the row step (epi.apply) on the 32/G lanes that hold a row.
-template <typename T, class E>
-__device__ __forceinline__ void warp_item(const WarpSched& ws, const Csr<T>& A,
-                                          const T* x, int w, E& epi) {
-    const int lane = threadIdx.x & 31;
-    const int r0 = __ldg(ws.row + w), r1 = __ldg(ws.row + w + 1);
-    const int lg = __ldg(ws.lg + w);
-    const int er = r0 + lane;
-    const bool has_epi = lane < (32 >> lg) && er < r1;
-    typename E::Pre pre{};
-    if (has_epi) pre = epi.load(er);
-    const Acc<T> mine = item_sums<T>(A, x, r0, r1, lg);
-    if (has_epi) epi.apply(er, mine, pre);
-}
-
-// All warp items of the schedule, grid-stride over the launched warps
-// (CTAs are sized to stay resident, so per-CTA costs are paid once).
-// IGX_ITEM_PREFETCH=0 compiles the plain loop (one dependent load chain
-// per item: schedule -> row pointers -> entries -> gathers). Pipelined,
-// FP32 attempts took 70.0 -> 67.9 us on the multicommodity LP and
-// 56.6 -> 55.1 us on the 200k x 500k LP, FP64 89.3 -> 87.7 us on the latter.
-#ifndef IGX_ITEM_PREFETCH
-#define IGX_ITEM_PREFETCH 1
-#endif
-
 // A warp's first item: rows [r0, r1), 2^lg lanes per row, the lane's row's
 // entries [b, e); r1 = 0 where the schedule has none for it.
 struct FirstItem {
@@ -617,7 +578,14 @@ __device__ __forceinline__ FirstItem first_item(const WarpSched& ws, const Csr<T
     return f;
 }
 
-// The items of this warp, from its first.
+// The items of this warp, from its first, each with its row steps in place: the
+// epilogue's vector entries for the lane's row are loaded first (epi.load), then
+// the row sums, then the row step (epi.apply) on the 32/G lanes that hold a row.
+// Grid-stride over the launched warps (CTAs are sized to stay resident, so per-CTA
+// costs are paid once). Against the plain loop (one dependent load chain per item:
+// schedule -> row pointers -> entries -> gathers) FP32 attempts took 70.0 -> 67.9
+// us on the multicommodity LP and 56.6 -> 55.1 us on the 200k x 500k LP, FP64 89.3
+// -> 87.7 us on the latter.
 template <typename T, class E>
 __device__ __forceinline__ void warp_rows_from(const WarpSched& ws, const Csr<T>& A,
                                                const T* x, E& epi, const FirstItem& f) {
@@ -666,13 +634,7 @@ __device__ __forceinline__ void warp_rows_from(const WarpSched& ws, const Csr<T>
 template <typename T, class E>
 __device__ __forceinline__ void warp_rows_all(const WarpSched& ws, const Csr<T>& A,
                                               const T* x, E& epi) {
-#if IGX_ITEM_PREFETCH
     warp_rows_from<T>(ws, A, x, epi, first_item<T>(ws, A));
-#else
-    const int stride = gridDim.x * kWarps;
-    for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5); w < ws.nwarps; w += stride)
-        warp_item<T>(ws, A, x, w, epi);
-#endif
 }
 
 }  // namespace igx

@@ -121,10 +121,15 @@ static cudaLaunchConfig_t cluster_config(cudaLaunchAttribute* at, const SmallPla
     cfg.numAttrs = 1;
     return cfg;
 }
+// (FP64 iterates are always held in shared memory)
+template <typename T>
+static auto attempts_kernel(const SmallPlan& plan) {
+    if constexpr (std::is_same<T, double>::value) return k_attempts_cluster<T, true>;
+    else return plan.held ? k_attempts_cluster<T, true> : k_attempts_cluster<T, false>;
+}
 template <typename T>
 static bool cluster_fits(const SmallPlan& plan) {
-    const void* fn = plan.held ? (const void*)k_attempts_cluster<T, true>
-                               : (const void*)k_attempts_cluster<T, false>;
+    const void* fn = (const void*)attempts_kernel<T>(plan);
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = cluster_config(at, plan, nullptr);
     int clusters = 0;
@@ -763,9 +768,7 @@ void Engine::launch_attempts(int count, const Vecs& v, bool graphs) {
         ++launches_;
         cudaLaunchAttribute at[1];
         const cudaLaunchConfig_t cfg = cluster_config(at, plan, st_);
-        CU(cudaLaunchKernelEx(&cfg,
-                              plan.held ? k_attempts_cluster<T, true> : k_attempts_cluster<T, false>,
-                              pa, da, m, n, count, plan));
+        CU(cudaLaunchKernelEx(&cfg, attempts_kernel<T>(plan), pa, da, m, n, count, plan));
         return;
     }
     launches_ += 2LL * count;
