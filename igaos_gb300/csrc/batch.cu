@@ -383,7 +383,7 @@ __device__ __forceinline__ Held<MODE> make_work(const BatchArgs& a, const BatchD
 }
 
 // Fills the staged matrix (by the worker warps, a slice at a time).
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, int workers) {
     const BatchDesc d = *dp;
     const Inst I = make_inst(a, d);
@@ -421,7 +421,7 @@ __device__ __noinline__ void fill_work(const BatchArgs& a, const BatchDesc* dp, 
             *v = p < e ? val[p] : 0.f;
             *ix = (Idx)(p < e ? idx[p] : 0);
         };
-        if (b1 > b0 || __all_sync(kFull, p == e)) {
+        if (!LONG || b1 > b0 || __all_sync(kFull, p == e)) {
             for (int k = b0; k < b1; ++k, ++p, v += 32, ix += 32) put();
             continue;
         }
@@ -533,23 +533,25 @@ __device__ __forceinline__ Acc<float> stepped_dot(const Idx* idx, const float* v
 }
 
 // Either of them, by slice.
-template <bool OUT, class Idx>
+template <bool OUT, bool LONG, class Idx>
 __device__ __forceinline__ Acc<float> any_dot(const int* base, const Idx* idx, const float* val,
                                               const float* v, int s, int rows, int longs) {
-    const float* table = val + 32LL * base[slices_of(rows)];
-    for (int i = 0; i < longs; ++i)
-        if (__float_as_int(table[2 * i]) == s)
-            return stepped_dot(idx, val, v, 32LL * __float_as_int(table[2 * i + 1]));
+    if constexpr (LONG) {
+        const float* table = val + 32LL * base[slices_of(rows)];
+        for (int i = 0; i < longs; ++i)
+            if (__float_as_int(table[2 * i]) == s)
+                return stepped_dot(idx, val, v, 32LL * __float_as_int(table[2 * i + 1]));
+    }
     return padded_dot<OUT>(idx, val, v, base[s], base[s + 1]);
 }
 
 // Rows of the CSR (columns of the CSC): f by one of the `workers` threads each,
 // those of more than kLongRow entries g by a warp each (they come first in the
 // order by length).
-template <class F, class G>
+template <bool LONG, class F, class G>
 __device__ __forceinline__ void each_row(const int* ptr, const int* order, int longer, int rows, int t,
                                          int workers, F f, G g) {
-    if (longer == 0) {
+    if constexpr (!LONG) {
         for (int r = t; r < rows; r += workers) f(r);
         return;
     }
@@ -609,19 +611,18 @@ __device__ __forceinline__ double full_x(const Inst& I, const Held<MODE>& W, int
 // Residual data of the LP seen from the anchor (xh, yh), FP64 -> FP32:
 // sc = c~ + A~^T yh, [scl, scu] = box~ - xh, [srmin, srmax] = rows~ - A~ xh,
 // with A~_ij = a_ij dc_j / dr_i formed in FP64 from the FP64 values.
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __noinline__ void anchor_data(const BatchArgs& a, const BatchDesc* d, int t,
                                          int workers) {
     const Inst I = make_inst(a, *d);
     const Held<MODE> W = make_work<MODE>(a, *d);
-    auto row = [&](int i, double s) {
-        const double dri = I.dr[i];
+    auto row = [&](int i, double dri, double s) {
         I.axh[i] = s;
         W.srmin()[i] = (float)(I.rmin[i] / dri - s);
         W.srmax()[i] = (float)(I.rmax[i] / dri - s);
         W.yh32()[i] = (float)I.yh[i];
     };
-    each_row(I.ap, a.order_r + d->row_off, d->longer_r, I.m, t, workers,
+    each_row<LONG>(I.ap, a.order_r + d->row_off, d->longer_r, I.m, t, workers,
              [&](int i) {
                  const double dri = I.dr[i];
                  double s = 0.0;
@@ -629,23 +630,22 @@ __device__ __noinline__ void anchor_data(const BatchArgs& a, const BatchDesc* d,
                      const int j = I.ai[p];
                      s = fma(I.axd[p] * (double)I.dc[j] / dri, I.xh[j], s);
                  }
-                 row(i, s);
+                 row(i, dri, s);
              },
              [&](int i) {
                  const double dri = I.dr[i];
                  const double s = warp_chain(
                      I.ap, i, [&](int p) { return I.axd[p] * (double)I.dc[I.ai[p]] / dri; },
                      [&](int p) { return I.xh[I.ai[p]]; });
-                 if ((threadIdx.x & 31) == 0) row(i, s);
+                 if ((threadIdx.x & 31) == 0) row(i, dri, s);
              });
-    auto column = [&](int j, double s) {
-        const double dcj = I.dc[j];
+    auto column = [&](int j, double dcj, double s) {
         I.atyh[j] = s;
         W.sc()[j] = (float)(I.c[j] * dcj + s);
         W.scl()[j] = (float)(I.cl[j] / dcj - I.xh[j]);
         W.scu()[j] = (float)(I.cu[j] / dcj - I.xh[j]);
     };
-    each_row(I.cp, a.order_c + d->col_off, d->longer_c, I.n, t, workers,
+    each_row<LONG>(I.cp, a.order_c + d->col_off, d->longer_c, I.n, t, workers,
              [&](int j) {
                  const double dcj = I.dc[j];
                  double s = 0.0;
@@ -653,20 +653,21 @@ __device__ __noinline__ void anchor_data(const BatchArgs& a, const BatchDesc* d,
                      const int i = I.ci[p];
                      s = fma(I.cax64[p] * dcj / (double)I.dr[i], I.yh[i], s);
                  }
-                 column(j, s);
+                 column(j, dcj, s);
              },
              [&](int j) {
                  const double dcj = I.dc[j];
                  const double s = warp_chain(
                      I.cp, j, [&](int p) { return I.cax64[p] * dcj / (double)I.dr[I.ci[p]]; },
                      [&](int p) { return I.yh[I.ci[p]]; });
-                 if ((threadIdx.x & 31) == 0) column(j, s);
+                 if ((threadIdx.x & 31) == 0) column(j, dcj, s);
              });
     __syncthreads();
 }
 
 // ---- setup: CSC, Ruiz, scaled data, power iteration ----------------------
 // (t: this thread among the workers, beyond every size for the decision warp)
+template <bool LONG>
 __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t, int workers,
                                    float& eta0, float& omega0) {
     const Inst I = make_inst(a, *d);
@@ -677,7 +678,7 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
     for (int j = t; j < n; j += workers) I.cnt[j] = 0;
     __syncthreads();
     auto count = [&](int p) { atomicAdd(&I.cnt[I.ai[p]], 1); };
-    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+    each_row<LONG>(I.ap, by_row, d->longer_r, m, t, workers,
              [&](int i) {
                  for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) count(p);
              },
@@ -691,7 +692,7 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
         I.ci[q] = i;
         I.cax64[q] = I.axd[p];
     };
-    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+    each_row<LONG>(I.ap, by_row, d->longer_r, m, t, workers,
              [&](int i) {
                  for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) place(i, p);
              },
@@ -743,7 +744,7 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
         auto scale_row = [&](int i, float mx) {
             if (mx > 0.f && isfinite(mx)) I.dr[i] *= sqrtf(mx);
         };
-        each_row(I.ap, by_row, d->longer_r, m, t, workers,
+        each_row<LONG>(I.ap, by_row, d->longer_r, m, t, workers,
                  [&](int i) {
                      float mx = 0.f;
                      for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) mx = fmaxf(mx, row_max(i, p));
@@ -760,7 +761,7 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
         auto scale_col = [&](int j, float mx) {
             if (mx > 0.f && isfinite(mx)) I.dc[j] /= sqrtf(mx);
         };
-        each_row(I.cp, by_col, d->longer_c, n, t, workers,
+        each_row<LONG>(I.cp, by_col, d->longer_c, n, t, workers,
                  [&](int j) {
                      float mx = 0.f;
                      for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) mx = fmaxf(mx, col_max(j, p));
@@ -780,12 +781,12 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
     Acc<float> nq[2];
     auto scaled = [&](int i, int p) { I.sax[p] = I.ax[p] * I.dc[I.ai[p]] / I.dr[i]; };
     auto scaled_c = [&](int j, int p) { I.scax[p] = I.cax[p] * I.dc[j] / I.dr[I.ci[p]]; };
-    each_row(I.ap, by_row, d->longer_r, m, t, workers,
+    each_row<LONG>(I.ap, by_row, d->longer_r, m, t, workers,
              [&](int i) {
                  for (int p = I.ap[i]; p < I.ap[i + 1]; ++p) scaled(i, p);
              },
              [&](int i) { warp_entries(I.ap, i, [&](int p) { scaled(i, p); }); });
-    each_row(I.cp, by_col, d->longer_c, n, t, workers,
+    each_row<LONG>(I.cp, by_col, d->longer_c, n, t, workers,
              [&](int j) {
                  for (int p = I.cp[j]; p < I.cp[j + 1]; ++p) scaled_c(j, p);
              },
@@ -810,7 +811,7 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
     __syncthreads();
     __shared__ float s_norm;
     for (int it = 0; it < 31; ++it) {
-        each_row(I.ap, by_row, d->longer_r, m, t, workers,
+        each_row<LONG>(I.ap, by_row, d->longer_r, m, t, workers,
                  [&](int i) { I.mt[i] = row_dot(I.ap, I.ai, I.sax, I.vt, i).result(); },
                  [&](int i) {
                      const float s = warp_row_dot(I.ap, I.ai, I.sax, I.vt, i).result();
@@ -819,15 +820,23 @@ __device__ __noinline__ void setup(const BatchArgs& a, const BatchDesc* d, int t
         __syncthreads();
         if (it == 30) break;
         // (normalised below, past the barrier)
-        each_row(I.cp, by_col, d->longer_c, n, t, workers,
-                 [&](int j) { I.vt[j] = row_dot(I.cp, I.ci, I.scax, I.mt, j).result(); },
-                 [&](int j) {
-                     const float s = warp_row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
-                     if (first_lane) I.vt[j] = s;
-                 });
-        __syncthreads();
         Acc<float> nrm[1];
-        for (int j = t; j < n; j += workers) nrm[0].add(I.vt[j], I.vt[j]);
+        if constexpr (!LONG) {
+            for (int j = t; j < n; j += workers) {
+                const float wv = row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
+                I.vt[j] = wv;
+                nrm[0].add(wv, wv);
+            }
+        } else {
+            each_row<LONG>(I.cp, by_col, d->longer_c, n, t, workers,
+                     [&](int j) { I.vt[j] = row_dot(I.cp, I.ci, I.scax, I.mt, j).result(); },
+                     [&](int j) {
+                         const float s = warp_row_dot(I.cp, I.ci, I.scax, I.mt, j).result();
+                         if (first_lane) I.vt[j] = s;
+                     });
+            __syncthreads();
+            for (int j = t; j < n; j += workers) nrm[0].add(I.vt[j], I.vt[j]);
+        }
         bmerge<1>(nrm, workers);
         if (t == 0) s_norm = sqrtf((float)nrm[0].result_d());
         __syncthreads();
@@ -883,7 +892,7 @@ __device__ __forceinline__ double div_by(double a, double b, double rb) {
 // The metrics of the current (0) and averaged (1) iterates; valid in the
 // decision warp's first lane. Two barriers; the candidates share them and the
 // loads of the LP's data.
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int pc, int t,
                                      int workers, double cmax, BMetrics* out) {
     BatchShared& sh = b_shared();
@@ -898,7 +907,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
         const int q = 32 * s + lane;
         const int i = q < I.m ? (MODE <= kHeldOut ? W.rid32[q] : (int)W.rid[q]) : I.m;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = any_dot<MODE <= kHeldOut>(W.rbase, W.ri, W.rv, xs[v], s, I.m, sh.longs[1]);
+            const Acc<float> ad = any_dot<MODE <= kHeldOut, LONG>(W.rbase, W.ri, W.rv, xs[v], s, I.m, sh.longs[1]);
             if (i >= I.m) continue;
             const double Ax = (I.axh[i] + ad.result_d()) * (double)I.dr[i];
             const double lo = I.rmin[i], hi = I.rmax[i];
@@ -940,7 +949,7 @@ __device__ __noinline__ void metrics(const BatchArgs& a, const BatchDesc* d, int
         const int q = 32 * s + lane;
         const int j = q < I.n ? (MODE <= kHeldOut ? W.cid32[q] : (int)W.cid[q]) : I.n;
         for (int v = 0; v < 2; ++v) {
-            const Acc<float> ad = any_dot<MODE <= kHeldOut>(W.cbase, W.ci, W.cv, ys[v], s, I.n, sh.longs[0]);
+            const Acc<float> ad = any_dot<MODE <= kHeldOut, LONG>(W.cbase, W.ci, W.cv, ys[v], s, I.n, sh.longs[0]);
             if (j >= I.n) continue;
             const double dcj = I.dc[j], cj = I.c[j];
             const double aty = I.atyh[j] + ad.result_d();
@@ -1198,26 +1207,19 @@ __device__ __forceinline__ void worker_loop(const BatchArgs& a, const BatchDesc*
         if (sh.step.done) return;
         if (!sh.step.check) continue;
         const int pc = sh.step.parity;
-        metrics<MODE>(a, d, pc, t, workers, cmax, nullptr);
+        metrics<MODE, LONG>(a, d, pc, t, workers, cmax, nullptr);
         cta_sync();
         if (sh.step.done) return;
         if (sh.step.restart) {
             re_anchor<MODE>(a, d, pc, sh.step.use_avg, t, workers);
             cta_sync();
-            anchor_data<MODE>(a, d, t, workers);  // ends with a barrier
+            anchor_data<MODE, LONG>(a, d, t, workers);  // ends with a barrier
         }
     }
 }
 
-// (apart, so that its calls cost the other instances' loop no registers)
-template <int MODE>
-__device__ __noinline__ void worker_loop_long(const BatchArgs& a, const BatchDesc* d, int workers,
-                                              double cmax) {
-    worker_loop<MODE, true>(a, d, make_work<MODE>(a, *d), workers, cmax);
-}
-
 // The decision warp's side of the same loop. Its first lane holds the state.
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __forceinline__ void decision_loop(const BatchArgs& a, const BatchDesc* d, int workers,
                                               double cmax, double eta, double omega, BatchOut& o) {
     BatchShared& sh = b_shared();
@@ -1308,7 +1310,7 @@ __device__ __forceinline__ void decision_loop(const BatchArgs& a, const BatchDes
         if (sh.step.done) break;
         if (!sh.step.check) continue;
         const int pc = sh.step.parity;
-        metrics<MODE>(a, d, pc, 1 << 30, workers, cmax, c.now);
+        metrics<MODE, LONG>(a, d, pc, 1 << 30, workers, cmax, c.now);
         if (lane == 0) {
             const BMetrics &mc = c.now[0], &ma = c.now[1];
             const long long kd = k - 1;  // index of the iteration just accepted
@@ -1394,7 +1396,7 @@ __device__ __forceinline__ void decision_loop(const BatchArgs& a, const BatchDes
     o.restarts = c.restarts;
 }
 
-template <int MODE>
+template <int MODE, bool LONG>
 __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
     const long long t_begin = global_ns();
     BatchShared& sh = b_shared();
@@ -1414,9 +1416,9 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
         for (int i = t; i < m; i += workers) I.yh[i] = I.pesy[i] = 0.0;
     }
     if (threadIdx.x < 2) sh.longs[threadIdx.x] = threadIdx.x ? d.long_r : d.long_c;
-    setup(a, dp, t, workers, s_eta0, s_omega0);
-    fill_work<MODE>(a, dp, workers);
-    anchor_data<MODE>(a, dp, t, workers);
+    setup<LONG>(a, dp, t, workers, s_eta0, s_omega0);
+    fill_work<MODE, LONG>(a, dp, workers);
+    anchor_data<MODE, LONG>(a, dp, t, workers);
     {
         double cm = 0.0;
         for (int j = t; j < n; j += workers) cm = bmax(cm, fabs(a.c[d.col_off + j]));
@@ -1443,14 +1445,13 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
     __syncthreads();
     if (decider) {
         BatchOut o;
-        decision_loop<MODE>(a, dp, workers, s_cmax, eta, omega, o);
+        decision_loop<MODE, LONG>(a, dp, workers, s_cmax, eta, omega, o);
         if (lane == 0) {
             o.ns = global_ns() - t_begin;
             a.out[b] = o;
         }
     } else {
-        if (d.long_c + d.long_r == 0) worker_loop<MODE, false>(a, dp, W, workers, s_cmax);
-        else worker_loop_long<MODE>(a, dp, workers, s_cmax);
+        worker_loop<MODE, LONG>(a, dp, W, workers, s_cmax);
         const Inst I = make_inst(a, d);
         // answer: anchor + delta of the chosen candidate, original units
         const int pf = sh.step.parity;
@@ -1477,12 +1478,16 @@ __device__ __forceinline__ void solve_one(const BatchArgs& a, int b) {
 // CTAs leave their SM's memory to L1, which serves them. In one class with
 // instances of 226 KB, 4,096 LPs of 20 to 2,000 rows took 18.5 s, 14.4 before
 // classes; 11.6 now (an iteration of an LP of 1,886 rows 98 us before, now 52).
+// Instances with long rows (LONG: slices laid in steps, rows that a warp takes in the
+// setup) have the same classes again, as kernels of their own: in one kernel with the
+// others, their code cost the others' loops registers (150 LPs of 30 to 400 rows 182
+// -> 190 ms).
 struct BatchClass {
     int threads, ctas;  // threads: without the decision warp
     size_t smem;
 };
-constexpr int kClasses = 5, kTight = 3;
-constexpr BatchClass kClass[kClasses] = {{128, 6, 36 * 1024},
+constexpr int kShapes = 5, kTight = 3, kClasses = 2 * kShapes;
+constexpr BatchClass kClass[kShapes] = {{128, 6, 36 * 1024},
                                          {256, 4, 55 * 1024},
                                          {512, 2, 112 * 1024},
                                          {512, 1, 226 * 1024},
@@ -1585,7 +1590,7 @@ BatchPlan plan_batch(const int* ap, const int* ai, std::vector<BatchDesc>& desc,
                 ++k;
             while (held_bytes(d, d.mode) > kClass[k].smem) --d.mode;
             if (d.mode > kHeldOut) return k;
-            k = kClasses - 1;
+            k = kShapes - 1;
             if (held_bytes(d, kHeldOut) > kClass[k].smem || reach > 0xffff) d.mode = kHeldWide;
             return k;
         };
@@ -1609,6 +1614,7 @@ BatchPlan plan_batch(const int* ap, const int* ai, std::vector<BatchDesc>& desc,
             d.out_off = P.out_entries;
             P.out_entries += d.pad_c + d.pad_r;
         }
+        if (d.longer_c + d.longer_r + d.long_c + d.long_r > 0) k += kShapes;
         P.cls[b] = k;
         P.smem[k] = std::max(P.smem[k], held_bytes(d, d.mode));
     }
@@ -1616,7 +1622,7 @@ BatchPlan plan_batch(const int* ap, const int* ai, std::vector<BatchDesc>& desc,
 }
 
 template <int K>
-__global__ void __launch_bounds__(kClass[K].threads + 32, kClass[K].ctas)
+__global__ void __launch_bounds__(kClass[K % kShapes].threads + 32, kClass[K % kShapes].ctas)
     k_batch(const __grid_constant__ BatchArgs a) {
     BatchShared& sh = b_shared();
     for (;;) {
@@ -1627,14 +1633,16 @@ __global__ void __launch_bounds__(kClass[K].threads + 32, kClass[K].ctas)
         if (qi >= a.count) break;
         const int b = a.order[qi];
         if (a.desc[b].m <= 0 || a.desc[b].n <= 0) continue;
-        if constexpr (K < kTight) {
-            solve_one<kHeldAll>(a, b);
-        } else if constexpr (K == kTight) {
-            if (a.desc[b].mode == kHeldAll) solve_one<kHeldAll>(a, b);
-            else solve_one<kHeldMatrix>(a, b);
+        constexpr int S = K % kShapes;
+        constexpr bool LONG = K >= kShapes;
+        if constexpr (S < kTight) {
+            solve_one<kHeldAll, LONG>(a, b);
+        } else if constexpr (S == kTight) {
+            if (a.desc[b].mode == kHeldAll) solve_one<kHeldAll, LONG>(a, b);
+            else solve_one<kHeldMatrix, LONG>(a, b);
         } else {
-            if (a.desc[b].mode == kHeldOut) solve_one<kHeldOut>(a, b);
-            else solve_one<kHeldWide>(a, b);
+            if (a.desc[b].mode == kHeldOut) solve_one<kHeldOut, LONG>(a, b);
+            else solve_one<kHeldWide, LONG>(a, b);
         }
     }
 }
@@ -1862,10 +1870,12 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
         CU(cudaEventCreate(&fk.e[kClasses]));
         CU(cudaEventCreate(&fk.e[kClasses + 1]));
         CU(cudaEventRecord(fk.e[kClasses], st));
-        void (*const kernels[kClasses])(BatchArgs) = {k_batch<0>, k_batch<1>, k_batch<2>,
-                                                         k_batch<3>, k_batch<4>};
+        void (*const kernels[kClasses])(BatchArgs) = {
+            k_batch<0>, k_batch<1>, k_batch<2>, k_batch<3>, k_batch<4>,
+            k_batch<5>, k_batch<6>, k_batch<7>, k_batch<8>, k_batch<9>};
         bool first = true;
-        for (int k = kClasses - 1; k >= 0; --k) {
+        for (int i = 0; i < kClasses; ++i) {
+            const int k = kShapes - 1 - i / 2 + (i % 2 ? 0 : kShapes);
             if (cls_count[k] == 0) continue;
             cudaStream_t sk = st;
             if (!first) {
@@ -1873,10 +1883,11 @@ extern "C" int igaos_pdhg_solve_batch(int count, const int* m, const int* n, con
                 sk = fk.s[k];
                 CU(cudaStreamWaitEvent(sk, fk.e[kClasses], 0));
             }
-            const int threads = kClass[k].threads + 32;
+            const BatchClass& shape = kClass[k % kShapes];
+            const int threads = shape.threads + 32;
             int per_sm = 0;
             CU(cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kClass[k].smem));
+                                    (int)shape.smem));
             CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernels[k], threads,
                                                              plan.smem[k]));
             BatchArgs Ak = A;
