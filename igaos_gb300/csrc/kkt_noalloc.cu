@@ -19,8 +19,8 @@
 namespace igx {
 namespace {
 
-constexpr int kNaMaxCtas = 16384;
-constexpr int kNaMaxDim = 256 * kNaMaxCtas;  // m, n <= 4,194,304
+constexpr int kNaMaxCtas = 1024;  // resident ones take rows and columns in strides
+constexpr int kNaMaxDim = 1 << 22;  // a limit of the interface, not of the scratch
 
 struct NaScratch {
     double part[kNaMaxCtas * 8];  // per-CTA partials of the current pass
@@ -29,7 +29,7 @@ struct NaScratch {
     unsigned int ticket[2];       // last-CTA counters (must start at zero)
 };
 
-// 1 MiB + a few bytes of device memory, per device that loads the library.
+// 64 KiB + a few bytes of device memory, per device that loads the library.
 static __device__ __align__(256) NaScratch g_na_scratch;
 
 constexpr int kMaxDevices = 64;
@@ -92,7 +92,7 @@ struct NaRow {
 // first, G lanes per row from the longest row of the pass at about eight
 // entries per lane. In file order with one G per warp, columns of mixed length
 // (a Zipf tail among short ones) issued more of them: 128 us against 86 us for
-// 500,000 columns of 5 M entries.
+// 500,000 columns of 5 M entries (80 us with the block sums as they are now).
 __device__ __forceinline__ NaRow na_row_sums(const int* __restrict__ ptr,
                                              const int* __restrict__ idx,
                                              const double* __restrict__ val,
@@ -139,7 +139,7 @@ __device__ __forceinline__ NaRow na_row_sums(const int* __restrict__ ptr,
 // and the FP64 pipe (53 % busy here, 70 % in the column pass). A warp used to
 // take a row with all its lanes and 32 rows in series, one dependent load
 // chain after another: on a 200,000 x 500,000 LP of 5 M entries 569 us, and
-// 691 us for the column pass; now 61 and 86 us, and a call 1,286 -> 127 us.
+// 691 us for the column pass; now 57 and 80 us, and a call 1,286 -> 122 us.
 __global__ void __launch_bounds__(kThreads, 4) na_rows(int m, int n, int per_warp,
                                                     const int* __restrict__ ap,
                                                     const int* __restrict__ ai,
@@ -350,8 +350,8 @@ extern "C" int igaos_pdhg_evaluate_noalloc(int m, int n, const int* ap, const in
     if (m <= 0 || n <= 0) return igx_set_error(IGAOS_PDHG_ERR_INVALID, "m and n must be positive");
     if (m > kNaMaxDim || n > kNaMaxDim)
         return igx_set_error(IGAOS_PDHG_ERR_INVALID,
-                             "m or n above 4,194,304: beyond the fixed scratch of the "
-                             "allocation-free evaluation (use igaos_pdhg_evaluate)");
+                             "m or n above 4,194,304, the limit of the allocation-free "
+                             "evaluation (use igaos_pdhg_evaluate)");
     if (!ap || !ai || !ax || !cp || !ci || !acx || !c || !cl || !cu || !rmin || !rmax || !x ||
         !y || !out6)
         return igx_set_error(IGAOS_PDHG_ERR_INVALID, "NULL device pointer");

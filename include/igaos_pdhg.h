@@ -433,9 +433,9 @@ int igaos_pdhg_solve_batch(int count, const int* m, const int* n,
  * receives {pinf, dinf, gap, op, od, prow} as evaluate() defines them
  * (src/pdhg/pdhg.cu:173-254). Work is enqueued on `stream` (a cudaStream_t,
  * NULL = default stream); the caller synchronises before reading out6.
- * Scratch is a fixed 1 MiB array in device memory that every GPU loading the
- * library holds until exit; m and n are limited to 4,194,304 (larger sizes
- * return IGAOS_PDHG_ERR_INVALID). The first call on a device looks up that
+ * Scratch is a fixed 64 KiB array in device memory that every GPU loading the
+ * library holds until exit; m and n are limited to 4,194,304, by this interface
+ * (larger sizes return IGAOS_PDHG_ERR_INVALID). The first call on a device looks up that
  * array's device address (no allocation); make that first call before any
  * stream capture. All calls share the array: calls that overlap on the GPU
  * (other streams, other threads) race and must be serialised by the caller.
