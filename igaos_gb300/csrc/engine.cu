@@ -420,7 +420,7 @@ Engine::Engine(int m_, int n_, long long nnz_, const int* ap, const int* ai, con
         sAT_ = candAT_[def_sched()] = sRAT_;
         // small LPs: the attempts of a chunk in one thread-block cluster with
         // the LP in its shared memory (cluster.cuh): 1,024 FP64 iterations
-        // of a 60 x 150 LP take 6.4 ms, 14.2 with the grid-wide kernels;
+        // of a 60 x 150 LP take 6.5 ms, 14.2 with the grid-wide kernels;
         // of a 2,000 x 5,000 LP 9.8 and 14.7.
         // IGAOS_PDHG_CLUSTER=0: never.
         const char* e = std::getenv("IGAOS_PDHG_CLUSTER");

@@ -91,7 +91,7 @@ def test_register_budgets_agree(native, dtype):
 def test_lean_backward(native, dtype, density):
     """LPs just past what one CTA holds with their costs and bounds: bit for bit
     as beside a larger one, whose launch spreads them over a cluster, and in FP64
-    against the dense checker."""
+    against the dense oracle."""
     lp = bernoulli(150, density, 4)
     many, beside = [lp] * 400, [lp] * 3 + [bernoulli(700, 0.03, 5)]
     assert plan(many, dtype, 2)["ctas"] == plan(many, dtype, 2)["lean"] == 1, lp.nnz
